@@ -71,6 +71,10 @@ int fg_attention_generic(const void *q, int ldq, void *out, int ldo, int dtype, 
                          const int *row_seq, const int *block_table, int table_width, const void *k_pool,
                          const void *v_pool, int M, int H, int KV, int hd, int page_size, float scale, int window,
                          cudaStream_t stream);
+/* prefill in float32 on the FMA units: head sizes 64 and 128, pages of 64 (arguments as fg_attention_prefill) */
+int fg_attention_prefill_f32(const void *q, int ldq, void *out, int ldo, const int *cu_rows, const int *seq_start,
+                             const int *block_table, int table_width, const void *k_pool, const void *v_pool, int n_seq,
+                             int max_new, int H, int KV, int hd, int page_size, float scale, int window, cudaStream_t stream);
 /* the same with values of head size hdv and, with a window, the sequence's first keep_first keys visible as well */
 /* softcap > 0: scores capped by softcap * tanh(score / softcap); sinks: a float per query head that joins the softmax's denominator;
    latent: the cache holds a latent (v_pool, hdv numbers, also the value) and a rotated key part (k_pool, hd numbers) a position,

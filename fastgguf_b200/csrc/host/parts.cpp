@@ -303,6 +303,20 @@ static Tensor attention(Runtime &rt, const Tensor &q, const Batch &b, const Laye
         return out;
     }
     if (q.dtype != io.cache_dtype) fail(FG_E_INTERNAL, "attention: q and the cache must share a dtype");
+    // Float32 with 64 and more (token, head of a group) rows a sequence: tiles of 128 rows that share the keys they read.  Fewer
+    // rows leave most of a tile idle, and a block a row keeps more of the GPU busy.
+    if (!rt.plain_kernels && q.dtype == FG_F32 && a.v_head_dim == hd && (hd == 64 || hd == 128) && io.page_size == 64 &&
+        !(a.window > 0 && a.keep_first > 0) && b.max_new * (H / KV) >= 64) {
+        count_launch();
+        ProfileScope scope("fg_attention_prefill_f32");
+        int code = FG_KERNEL("core", fg_attention_prefill_f32)(q.data, (int)q.ld, out.data, (int)out.ld, b.cu_rows, b.seq_start, table, b.table_width,
+                                                               io.k_pool, io.v_pool, b.n_seq, b.max_new, H, KV, hd, io.page_size, a.scale, a.window,
+                                                               rt.stream);
+        if (code != KERNEL_BAD_SIZE) {
+            check_kernel(code, "fg_attention_prefill_f32");
+            return out;
+        }
+    }
     if (hd > 256 || a.v_head_dim > 256)
         fail(FG_E_KERNEL, format("attention: head size %d / %d exceeds 256, the largest the any-size kernel takes", hd, a.v_head_dim));
     FG_LAUNCH("core", fg_attention_generic_kept, q.data, (int)q.ld, out.data, (int)out.ld, q.dtype, b.positions, b.row_seq, table,

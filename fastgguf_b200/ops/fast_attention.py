@@ -94,6 +94,18 @@ def attention_prefill(q, cu_rows, seq_start, block_table, k_pool, v_pool, n_seq,
     return out
 
 
+def attention_prefill_f32(q, cu_rows, seq_start, block_table, k_pool, v_pool, n_seq, max_new, n_heads, n_kv_heads,
+                          head_dim, scale, window=0, out=None):
+    """The same contract as ``attention_prefill`` in float32 on the FMA units (head sizes 64 and 128)."""
+    if out is None:
+        out = torch.empty((q.shape[0], n_heads * head_dim), dtype=torch.float32, device=q.device)
+    check(lib("core").fg_attention_prefill_f32(ptr(q), q.stride(0), ptr(out), out.stride(0), ptr(cu_rows), ptr(seq_start),
+                                               ptr(block_table), block_table.shape[1], ptr(k_pool), ptr(v_pool), n_seq,
+                                               max_new, n_heads, n_kv_heads, head_dim, k_pool.shape[2], float(scale),
+                                               int(window), stream()), "attention_prefill_f32")
+    return out
+
+
 def attention_prefill_tc(q, cu_rows, seq_start, block_table, k_pool, v_pool, n_seq, max_new, n_heads, n_kv_heads,
                          head_dim, scale, window=0, out=None):
     """The same contract as ``attention_prefill`` on the tcgen05 tensor cores (128-row tiles, K/V by TMA,

@@ -91,6 +91,8 @@ _SIGNATURES = {
                             c_int, c_int, c_int, c_void_p],
         "fg_attention_generic": [c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int,
                                  c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p],
+        "fg_attention_prefill_f32": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
+                                     c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p],
         "fg_sample": [c_void_p, c_int, c_int, c_int, c_float, c_int, c_float, c_float, c_int, c_void_p,
                       c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p],
         "fg_argmax": [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p],

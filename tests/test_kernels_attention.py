@@ -95,6 +95,43 @@ def test_attention_generic(H, KV, hd, window, dtype, tol):
     assert _err(got, plain(case, H, KV, hd, scale, window)) < tol
 
 
+@pytest.mark.parametrize("H,KV,hd,window", [(8, 2, 64, 0), (3, 1, 128, 0), (24, 8, 128, 0), (20, 1, 64, 0), (4, 4, 64, 100), (4, 2, 64, 64),
+                                            (8, 2, 64, 65), (6, 2, 128, 128), (4, 2, 64, -48), (3, 1, 128, -200)])
+def test_attention_prefill_f32(H, KV, hd, window):
+    """The tiled float32 kernel against float64, and - chunked masks too - against the any-size kernel.  A value that is no number in
+    rows of the last page that no sequence has reached, or at a later token's place, reaches no other row."""
+    from fastgguf_b200 import ops
+    from fastgguf_b200.ops import fast_attention
+    new = [200, 1, 67, 5, 130]
+    case = make_case([0, 300, 60, 0, 700], new, H, KV, hd, torch.float32, 13)
+    scale = 1.0 / math.sqrt(hd)
+
+    def both():
+        got = fast_attention.attention_prefill_f32(case["q"], case["cu_rows"], case["seq_start"], case["table"], case["k_pool"],
+                                                   case["v_pool"], len(new), max(new), H, KV, hd, scale, window)
+        return got, ops.attention_generic(case["q"], case["positions"], case["row_seq"], case["table"], case["k_pool"], case["v_pool"],
+                                          H, KV, hd, scale, window)
+
+    got, any_size = both()
+    assert _err(got, any_size.double().cpu()) < 5e-6
+    if window >= 0:
+        want = plain(case, H, KV, hd, scale, window)
+        assert _err(got, want) < 5e-6
+        assert (got.double().cpu() - want).norm() <= 1.2 * (any_size.double().cpu() - want).norm()
+    # the first sequence's key 150 and everything behind each sequence's end are no numbers
+    page, off = int(case["table"][0, 150 // PAGE]), 150 % PAGE
+    case["v_pool"][page, :, off] = float("nan")
+    for s, (before, n) in enumerate(zip(case["lens_before"], new)):
+        end = before + n
+        if end % PAGE:
+            last = int(case["table"][s, end // PAGE])
+            case["v_pool"][last, :, end % PAGE:] = float("inf")
+            case["k_pool"][last, :, end % PAGE:] = float("nan")
+    bad, bad_any = both()
+    assert torch.equal(bad.isnan(), bad_any.isnan())
+    assert torch.equal(bad[:150], got[:150]) and torch.equal(bad[200:], got[200:])
+
+
 @pytest.mark.parametrize("n_splits", [None, 1, 2, 3, 8, 16])
 @pytest.mark.parametrize("H,KV,hd,window", [(8, 2, 64, 0), (3, 1, 128, 0), (24, 8, 128, 0), (20, 1, 64, 0),
                                             (4, 4, 64, 100), (4, 2, 64, 64), (4, 2, 64, 128), (8, 2, 64, 65),
