@@ -271,6 +271,10 @@ int fg_gemm_tc_grouped(const void *X, int ldx, int rows, const void *W, int ldw,
                        const void *tiles, int n_tiles, cudaStream_t stream);
 int fg_gemm_tc_grouped_ext(const void *X, int ldx, int rows, const void *W, int ldw, int stack_rows, void *out, int ldc, int epi /* 1 or 4 */, int N,
                            int K, const void *tiles, int n_tiles, cudaStream_t stream);
+/* float32 operands and result: C (+)= A W^T with every operand as the sum of three bfloat16 planes made in scratch memory; 0 bytes: refused */
+long long fg_gemm_f32_tc_workspace_bytes(int M, int N, int K);
+int fg_gemm_f32_tc(const float *A, int lda, const float *W, int ldw, float *C, int ldc, int accumulate, int M, int N, int K,
+                   void *ws, long long ws_bytes, cudaStream_t stream);
 int fg_gemm_tc_error(void);
 /* tests only: shorten the bounded waits and make the decode kernel's pipeline stall, see gemm_tc.cu */
 int fg_gemm_tc_test_hook(long long wait_limit_cycles, int skip_copy);

@@ -1,0 +1,393 @@
+// float32 contraction on the tensor cores without giving up float32: C[m, n] (+)= sum_k A[m, k] * W[n, k] with float32 operands
+// and results, for more rows than the weight-streaming kernel takes (part of gemm_tc.cu's translation unit, whose helpers it uses).
+//
+// A float32 number is the sum of three bfloat16 numbers: hi = bf16(a), mid = bf16(a - hi), lo = a - hi - mid, 8 bits of mantissa each
+// and the differences exact.  A product of two such sums is nine products of bfloat16 numbers, each exact in float32; the six largest
+// (hi hi, hi mid, mid hi, mid mid, hi lo, lo hi) are computed, the other three are below 2^-24 of the product.
+//
+// What is left is the order of additions.  The tensor cores' accumulator is float32, but its sums are cut off, not rounded, and over
+// a long reduction the cuts all go one way.  So an accumulator in tensor memory only ever holds ONE K-block of 64: the six products in
+// rising order of size, hi hi last (four instructions whose cuts count); then the epilogue warps take it out and add it, correctly rounded, to
+// the sums they keep in registers.  The chain of additions of an output is K / 64 long instead of K.
+//
+//   f32_split_kernel        operand -> three bfloat16 planes in scratch memory
+//   gemm_f32_pair_kernel    the persistent pair-of-CTAs kernel of gemm_tc.cu with six planes a stage, two accumulators that
+//                           alternate from K-block to K-block, and eight warps that add them up
+//   gemm_f32_finish_kernel  adds the parts of a contraction that is split along K (few output tiles), in split order
+//
+// Distance from float64 (2-norm, normal operands, 600 rows): 1.1e-7 at K = 2,048 and 1.5e-7 at 8,192, where the chain of fused multiply-adds
+// has 8.1e-7 and 1.6e-6.  Times with the planes' making, against gemm_tile128_kernel (us): 2,048 rows x 16,384 x 2,048: 554 against
+// 3,175 (248 TFLOP/s; a sixth of the bfloat16 burst rate is 270); 2,048 x 2,048 x 8,192: 306 against 1,747; 600 x 2,048 x 8,192: 143
+// against 1,249; 24 x 2,048 x 2,048: 38 against 210.
+//
+// Numbers that the split does not carry (infinities, NaN, magnitudes whose first plane or whose partial sums overflow) leave a sum
+// that is no finite number; such an output is computed again by the plain chain of fused multiply-adds over the float32 operands.
+#pragma once
+
+#define F32_EPI_WARPS 8
+#define F32_THREADS (64 + 32 * F32_EPI_WARPS)
+#define F32_STAGING 4096                   // per epilogue warp: a 32 x 32 float32 tile
+
+struct F32Args {
+    float *out;                            // [M, ldc], or the parts [splits][M][N]
+    const float *A, *W;                    // the float32 operands, for outputs that are computed again
+    int M, N, K, ldc, lda, ldw;
+    int splits, kb_per_split;
+    int a_rows, w_rows;                    // rows between the planes of the operands
+    int accumulate, vec_ok;
+};
+
+__device__ __noinline__ float f32_plain_dot(const float *a, const float *w, int K) {
+    float s = 0.f;
+    for (int k = 0; k < K; k++) s = fmaf(a[k], w[k], s);
+    return s;
+}
+__device__ __forceinline__ bool f32_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
+
+// planes[p][row][k], p = 0 (hi), 1 (mid), 2 (lo).  Bound by memory: 4 bytes in, 6 out.  A thread takes eight numbers.
+__global__ void __launch_bounds__(256)
+f32_split_kernel(const float *__restrict__ x, int ld, bf16 *__restrict__ planes, int rows, int K) {
+    const int per_row = K / 8;
+    const long long n = (long long)rows * per_row;
+    const size_t plane = (size_t)rows * K;
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
+        const int r = (int)(i / per_row), c = (int)(i % per_row) * 8;
+        const float4 u[2] = {__ldcs((const float4 *)(x + (size_t)r * ld + c)), __ldcs((const float4 *)(x + (size_t)r * ld + c + 4))};
+        const float v[8] = {u[0].x, u[0].y, u[0].z, u[0].w, u[1].x, u[1].y, u[1].z, u[1].w};
+        uint32_t w[3][4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            float a = v[2 * j], b = v[2 * j + 1];
+#pragma unroll
+            for (int p = 0; p < 3; p++) {
+                const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
+                w[p][j] = *(const uint32_t *)&t;
+                a -= __low2float(t);
+                b -= __high2float(t);
+            }
+        }
+#pragma unroll
+        for (int p = 0; p < 3; p++) *(uint4 *)(planes + p * plane + (size_t)r * K + c) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+    }
+}
+
+// Stages: three 16 KB planes of token rows and three of half the weight rows: 96 KB at 256 columns, 72 KB at 128; two fit
+// beside the staging tiles.  A K-block is 24 instructions of 256 x BN x 16: 3,072 cycles at 256 columns, for 96 KB of operands - less than half
+// of what the bfloat16 kernel asks of the L2-to-SM path.
+template <int BN>
+__global__ void __launch_bounds__(F32_THREADS, 1)
+gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmQ, F32Args a, int n_pt, int n_tiles) {
+    constexpr int STAGES = 2;
+    constexpr int P_BYTES = BM * BK * 2, Q_BYTES = (BN / 2) * BK * 2;      // one plane of this CTA's share
+    constexpr int STAGE_BYTES = 3 * (P_BYTES + Q_BYTES);
+    constexpr int TMEM_COLS = 2 * BN;
+    constexpr int NC = BN / 2;                                             // columns an epilogue warp adds up
+
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    __shared__ __align__(8) uint64_t bars[2 * STAGES + 4];
+    __shared__ uint32_t tmem_base_s;
+
+    const int warp = warp_index(), lane = threadIdx.x & 31;
+    const int rank = (int)(blockIdx.x & 1);            // 0: the pair's leader (issues the MMAs), 1: its peer
+    const int pair = (int)(blockIdx.x >> 1), n_pairs = (int)(gridDim.x >> 1);
+    const int nkb = (a.K + BK - 1) / BK;
+    const int per_split = n_tiles / a.splits;          // the tile index counts the split, slowest
+    const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[STAGES]);
+    const uint32_t tfull0 = smem_u32(&bars[2 * STAGES]), tempty0 = smem_u32(&bars[2 * STAGES + 2]);
+    const uint32_t smem0 = smem_u32(smem);
+    const uint32_t lead_full0 = mapa_u32(full0, 0), lead_tempty0 = mapa_u32(tempty0, 0);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; s++) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
+        for (int i = 0; i < 2; i++) { mbar_init(tfull0 + 8 * i, 1); mbar_init(tempty0 + 8 * i, 2 * F32_EPI_WARPS); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
+                     ::"r"(smem_u32(&tmem_base_s)), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();                                    // the partner's barriers exist before anything arrives on them
+    tc_fence_after();
+    const uint32_t tmem_base = tmem_base_s;
+
+    if (warp == 0) {
+        // ------------------------------------------------------------ TMA producer (both CTAs)
+        int s = 0, ph = 0;
+        bool ok = true;
+        for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
+            const int t2 = tile % per_split, kb0 = tile / per_split * a.kb_per_split, kb1 = min(nkb, kb0 + a.kb_per_split);
+            const int p0 = (t2 % n_pt) * (2 * BM) + rank * BM, q0 = (t2 / n_pt) * BN + rank * (BN / 2);
+            for (int kb = kb0; kb < kb1; kb++) {
+                ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, ph ^ 1));
+                if (!ok) { raise_error(1); break; }
+                if (elect_one()) {
+                    const uint32_t dst = smem0 + s * STAGE_BYTES, bar = lead_full0 + 8 * s;
+                    if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * STAGE_BYTES);     // both CTAs' copies of the stage
+#pragma unroll
+                    for (int p = 0; p < 3; p++) {
+                        // (a box that runs past its plane reads the next plane's rows: outputs of rows past M and N are not stored)
+                        tma_load_2d_pair(dst + p * P_BYTES, &tmP, kb * BK, p * a.a_rows + p0, bar);
+                        tma_load_2d_pair(dst + 3 * P_BYTES + p * Q_BYTES, &tmQ, kb * BK, p * a.w_rows + q0, bar);
+                    }
+                }
+                __syncwarp();
+                if (++s == STAGES) { s = 0; ph ^= 1; }
+            }
+        }
+    } else if (warp == 1) {
+        // ------------------------------------------------------------ MMA issuer (the leader only)
+        if (rank == 0) {
+            const uint32_t idesc = make_idesc(2 * BM, BN);
+            const uint64_t pdesc0 = make_smem_desc(smem0), qdesc0 = make_smem_desc(smem0 + 3 * P_BYTES);
+            int s = 0, ph = 0, i = 0;                  // i: K-blocks so far, over all tiles
+            bool ok = true;
+            for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
+                const int kb0 = tile / per_split * a.kb_per_split, kb1 = min(nkb, kb0 + a.kb_per_split);
+                for (int kb = kb0; kb < kb1; kb++, i++) {
+                    const int acc = i & 1;
+                    ok = __all_sync(0xffffffffu, mbar_wait(tempty0 + 8 * acc, ((i >> 1) & 1) ^ 1));
+                    if (!ok) { raise_error(4); break; }
+                    ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, ph));
+                    if (!ok) { raise_error(2); break; }
+                    tc_fence_after();
+                    const uint64_t soff = (uint64_t)(s * (STAGE_BYTES >> 4));
+                    const uint64_t pdesc = pdesc0 + soff, qdesc = qdesc0 + soff;
+                    if (elect_one()) {
+                        // planes of the two factors, the smallest products first
+                        constexpr int PA[6] = {0, 2, 1, 0, 1, 0}, PB[6] = {2, 0, 1, 1, 0, 0};
+#pragma unroll
+                        for (int pr = 0; pr < 6; pr++)
+#pragma unroll
+                            for (int k = 0; k < BK / UMMA_K; k++) {
+                                const uint64_t koff = (uint64_t)((k * UMMA_K * 2) >> 4);
+                                tc_mma_bf16_pair(tmem_base + acc * BN, pdesc + (uint64_t)((PA[pr] * P_BYTES) >> 4) + koff,
+                                                 qdesc + (uint64_t)((PB[pr] * Q_BYTES) >> 4) + koff, idesc, (pr | k) != 0);
+                            }
+                        tc_commit_pair(empty0 + 8 * s);              // frees the stage in both CTAs
+                        tc_commit_pair(tfull0 + 8 * acc);            // the K-block's sums are complete
+                    }
+                    __syncwarp();
+                    if (++s == STAGES) { s = 0; ph ^= 1; }
+                }
+            }
+        }
+    } else {
+        // ------------------------------------------------------------ sums and epilogue (warps 2.., both CTAs): this CTA's 128 rows
+        const int lg = warp & 3, half = (warp - 2) >> 2;
+        float *T = (float *)(smem + STAGES * STAGE_BYTES) + (warp - 2) * (F32_STAGING / 4);
+        int i = 0;
+        bool ok = true;
+        for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
+            const int t2 = tile % per_split, z = tile / per_split, kb0 = z * a.kb_per_split, kb1 = min(nkb, kb0 + a.kb_per_split);
+            const int m_base = (t2 % n_pt) * (2 * BM) + rank * BM + lg * 32, n_base = (t2 / n_pt) * BN + half * NC;
+            float sum[NC];
+#pragma unroll
+            for (int j = 0; j < NC; j++) sum[j] = 0.f;
+            for (int kb = kb0; kb < kb1; kb++, i++) {
+                const int acc = i & 1;
+                ok = __all_sync(0xffffffffu, mbar_wait(tfull0 + 8 * acc, (i >> 1) & 1));
+                if (!ok) { raise_error(3); break; }
+                tc_fence_after();
+                const uint32_t trow = tmem_base + ((uint32_t)(lg * 32) << 16) + acc * BN + half * NC;
+#pragma unroll
+                for (int c = 0; c < NC / 16; c++) {                // 16 at a time: 128 sums and the kernel's 168 registers a thread
+                    float v[16];
+                    tc_ld16(trow + c * 16, v);
+#pragma unroll
+                    for (int j = 0; j < 16; j++) sum[c * 16 + j] += v[j];
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(lead_tempty0 + 8 * acc);
+            }
+            if (!ok) break;
+            // 32 columns at a time through a tile in shared memory, so that a warp stores whole 128-byte lines
+            const bool part = a.splits > 1;
+            float *out = part ? a.out + (size_t)z * a.M * a.N : a.out;
+            const int ldc = part ? a.N : a.ldc;
+#pragma unroll
+            for (int c = 0; c < NC / 32; c++) {
+#pragma unroll
+                for (int ch = 0; ch < 8; ch++)
+                    *(float4 *)(T + lane * 32 + ((ch ^ (lane & 7)) << 2)) =
+                        make_float4(sum[c * 32 + 4 * ch], sum[c * 32 + 4 * ch + 1], sum[c * 32 + 4 * ch + 2], sum[c * 32 + 4 * ch + 3]);
+                __syncwarp();
+                const int ch = lane & 7, n = n_base + c * 32 + ch * 4;
+#pragma unroll 2
+                for (int pass = 0; pass < 8; pass++) {
+                    const int row = pass * 4 + (lane >> 3), m = m_base + row;
+                    if (m >= a.M || n >= a.N) continue;
+                    float4 t = *(const float4 *)(T + row * 32 + ((ch ^ (row & 7)) << 2));
+                    float *dst = out + (size_t)m * ldc + n;
+                    if (!part && !(f32_finite(t.x) && f32_finite(t.y) && f32_finite(t.z) && f32_finite(t.w))) {
+                        const float *ar = a.A + (size_t)m * a.lda, *wr = a.W + (size_t)n * a.ldw;
+                        if (!f32_finite(t.x)) t.x = f32_plain_dot(ar, wr, a.K);
+                        if (!f32_finite(t.y) && n + 1 < a.N) t.y = f32_plain_dot(ar, wr + (size_t)a.ldw, a.K);
+                        if (!f32_finite(t.z) && n + 2 < a.N) t.z = f32_plain_dot(ar, wr + 2 * (size_t)a.ldw, a.K);
+                        if (!f32_finite(t.w) && n + 3 < a.N) t.w = f32_plain_dot(ar, wr + 3 * (size_t)a.ldw, a.K);
+                    }
+                    if (a.vec_ok && n + 3 < a.N) {
+                        if (a.accumulate && !part) {
+                            const float4 r = __ldcg((const float4 *)dst);
+                            t.x += r.x; t.y += r.y; t.z += r.z; t.w += r.w;
+                        }
+                        *(float4 *)dst = t;
+                    } else {
+                        const float tv[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+                        for (int j = 0; j < 4; j++)
+                            if (n + j < a.N) dst[j] = tv[j] + (a.accumulate && !part ? dst[j] : 0.f);
+                    }
+                }
+                __syncwarp();
+            }
+        }
+    }
+    // see gemm_tc_prefill_pair_kernel: neither CTA leaves while the other may still touch its memory or its barriers
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+    }
+}
+
+// out[m, n] (+)= the sum of the parts [splits][M][N], in split order; four columns a thread (N % 4 == 0 where splits are taken)
+__global__ void __launch_bounds__(256)
+gemm_f32_finish_kernel(F32Args a, const float *__restrict__ parts) {
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x, per_row = a.N / 4;
+    if (i >= a.M * per_row) return;
+    const int m = (int)(i / per_row), n = (int)(i % per_row) * 4;
+    float *dst = a.out + (size_t)m * a.ldc + n;
+    float t[4] = {0.f, 0.f, 0.f, 0.f}, res[4] = {0.f, 0.f, 0.f, 0.f};
+    if (a.accumulate) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) res[j] = dst[j];
+    }
+    const float *p = parts + (size_t)m * a.N + n;
+#pragma unroll 4
+    for (int z = 0; z < a.splits; z++) {
+        const float4 v = __ldcs((const float4 *)(p + (size_t)z * a.M * a.N));
+        t[0] += v.x; t[1] += v.y; t[2] += v.z; t[3] += v.w;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        if (!f32_finite(t[j])) t[j] = f32_plain_dot(a.A + (size_t)m * a.lda, a.W + (size_t)(n + j) * a.ldw, a.K);
+        dst[j] = t[j] + res[j];
+    }
+}
+
+// ---------------------------------------------------------------------------- host side
+#define F32_PLANE_LIMIT ((size_t)256 << 20)            // bytes of planes of one operand at a time: scratch memory stays bounded
+
+struct F32Plan { int bn, splits, kb_per_split, a_rows, w_rows; size_t a_bytes, w_bytes, part_bytes; };
+
+// How the contraction is cut: rows of the operands whose planes are made at a time, tile width, splits along K.  The times
+// are those of a K-block (microseconds), of the start and end of a tile, and of the pass that adds the parts.
+static F32Plan f32_plan(int M, int N, int K) {
+    F32Plan best{};
+    const int nkb = (K + BK - 1) / BK, pairs = sm_count() / 2;
+    const size_t row_bytes = (size_t)K * 6;
+    auto rows_at_a_time = [&](int rows) {
+        const size_t most = F32_PLANE_LIMIT / row_bytes / 256 * 256;
+        return (size_t)rows <= most ? rows : (int)(most < 256 ? 256 : most);
+    };
+    const int am = rows_at_a_time(M), wn = rows_at_a_time(N);
+    double best_us = 1e30;
+    for (int bn = 128; bn <= 256; bn += 128)
+        for (int s = 1; s <= 16; s++) {
+            const int per = (nkb + s - 1) / s;
+            if (s > 1 && (per < 4 || (s - 1) * per >= nkb || N % 4)) continue;
+            const long long tiles = (long long)((am + 255) / 256) * ((wn + bn - 1) / bn) * s;
+            const double rounds = (double)((tiles + pairs - 1) / pairs);
+            const double us = rounds * (per * (bn == 256 ? 1.75 : 0.95) + 4.0) + (s > 1 ? 4.0 + (s + 2.0) * am * wn * 4.0 / 4e6 : 0.0);
+            if (us < best_us) { best_us = us; best.bn = bn; best.splits = s; best.kb_per_split = per; }
+        }
+    auto up = [](size_t b) { return (b + 1023) / 1024 * 1024; };
+    best.a_rows = am; best.w_rows = wn;
+    best.a_bytes = up(am * row_bytes); best.w_bytes = up(wn * row_bytes);
+    best.part_bytes = best.splits > 1 ? up((size_t)best.splits * am * wn * 4) : 0;
+    return best;
+}
+
+// Scratch memory fg_gemm_f32_tc needs; 0: sizes it does not take.  Rows up to 16 belong to the weight-streaming kernel.  Short
+// reductions and narrow outputs (K < 512, N < 256) stay with the plain kernels: one or two rounds of their tiles take about
+// what the three launches here do.  From 17 rows on the planes won at every size measured (K 2,048 and 8,192, N 2,048 to 16,384, 24 to
+// 2,048 rows: 2.7 to 13 times).
+extern "C" long long fg_gemm_f32_tc_workspace_bytes(int M, int N, int K) {
+    if (M <= 16 || N < 256 || K < 512 || K % 8) return 0;
+    const F32Plan p = f32_plan(M, N, K);
+    return (long long)(p.a_bytes + p.w_bytes + p.part_bytes);
+}
+
+template <int BN>
+static int launch_f32_pair(const CUtensorMap &tmP, const CUtensorMap &tmQ, const F32Args &a, cudaStream_t stream) {
+    constexpr int smem = 2 * 3 * (BM + BN / 2) * BK * 2 + 1024 + F32_EPI_WARPS * F32_STAGING;
+    static FgPerDevice configured;
+    if (fg_needs_setup(configured)) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_f32_pair_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return (int)e;
+    }
+    const int n_pt = (a.M + 2 * BM - 1) / (2 * BM), n_tiles = n_pt * ((a.N + BN - 1) / BN) * a.splits, pairs = sm_count() / 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * (n_tiles < pairs ? n_tiles : pairs), 1, 1); cfg.blockDim = dim3(F32_THREADS);
+    cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    return (int)cudaLaunchKernelEx(&cfg, gemm_f32_pair_kernel<BN>, tmP, tmQ, a, n_pt, n_tiles);
+}
+
+static int launch_f32_split(const float *x, int ld, bf16 *planes, int rows, int K, cudaStream_t stream) {
+    const long long blocks = ((long long)rows * (K / 8) + 255) / 256, most = 8LL * sm_count();
+    return fg_launch_in_order(f32_split_kernel, dim3((unsigned)(blocks < most ? blocks : most)), dim3(256), 0, stream, x, ld, planes, rows, K);
+}
+
+// C[m, n] (+)= sum_k A[m, k] W[n, k], everything float32.  Needs fg_gemm_f32_tc_workspace_bytes of 1024-byte aligned scratch
+// memory; FG_ERR_BAD_SIZE for what it does not take (the plain kernels do).  Kernels are launched in plain stream order.
+extern "C" int fg_gemm_f32_tc(const float *A, int lda, const float *W, int ldw, float *C, int ldc, int accumulate, int M, int N, int K,
+                              void *ws, long long ws_bytes, cudaStream_t stream) {
+    if (M <= 0 || N <= 0) return 0;
+    const long long need = fg_gemm_f32_tc_workspace_bytes(M, N, K);
+    if (need == 0 || ws == nullptr || ws_bytes < need || lda % 4 || ldw % 4 || (((uintptr_t)A | (uintptr_t)W) & 15) || ((uintptr_t)ws & 255))
+        return FG_ERR_BAD_SIZE;
+    const F32Plan p = f32_plan(M, N, K);
+    bf16 *ap = (bf16 *)ws, *wp = (bf16 *)((char *)ws + p.a_bytes);
+    float *parts = (float *)((char *)ws + p.a_bytes + p.w_bytes);
+    for (int m0 = 0; m0 < M; m0 += p.a_rows) {
+        const int mr = M - m0 < p.a_rows ? M - m0 : p.a_rows;
+        int e = launch_f32_split(A + (size_t)m0 * lda, lda, ap, mr, K, stream);
+        if (e) return e;
+        for (int n0 = 0; n0 < N; n0 += p.w_rows) {
+            const int nr = N - n0 < p.w_rows ? N - n0 : p.w_rows;
+            if (n0 > 0 || m0 == 0 || p.w_rows < N) {                        // (the planes of W are kept where all of them fit)
+                e = launch_f32_split(W + (size_t)n0 * ldw, ldw, wp, nr, K, stream);
+                if (e) return e;
+            }
+            CUtensorMap tmP, tmQ;
+            e = make_map(&tmP, ap, 3 * mr, K, K, BM);
+            if (e) return e;
+            e = make_map(&tmQ, wp, 3 * nr, K, K, p.bn / 2);
+            if (e) return e;
+            float *out = C + (size_t)m0 * ldc + n0;
+            const bool split = p.splits > 1;
+            F32Args a{split ? parts : out, A + (size_t)m0 * lda, W + (size_t)n0 * ldw, mr, nr, K, ldc, lda, ldw, p.splits, p.kb_per_split, mr, nr,
+                      accumulate, split ? nr % 4 == 0 : ((uintptr_t)out % 16 == 0 && ldc % 4 == 0)};
+            e = p.bn == 256 ? launch_f32_pair<256>(tmP, tmQ, a, stream) : launch_f32_pair<128>(tmP, tmQ, a, stream);
+            if (e) return e;
+            if (split) {
+                a.out = out;
+                const long long n4 = (long long)mr * (nr / 4);
+                e = fg_launch_in_order(gemm_f32_finish_kernel, dim3((unsigned)((n4 + 255) / 256)), dim3(256), 0, stream, a, (const float *)parts);
+                if (e) return e;
+            }
+        }
+    }
+    return 0;
+}

@@ -1539,6 +1539,8 @@ extern "C" int fg_gemm_tc_grouped(const void *X, int ldx, int rows, const void *
     return fg_gemm_tc_grouped_ext(X, ldx, rows, W, ldw, stack_rows, out, ldc, EPI_F32, N, K, tiles, n_tiles, stream);
 }
 
+#include "gemm_f32_tc.cuh"
+
 // For the test of the bounded waits: wait_limit_cycles > 0 sets how long a wait may last (0 restores the default of
 // about a second; values below half a millisecond act as half a millisecond), and skip_copy != 0 makes the decode
 // kernel's producer leave the first stage of every launch incomplete, so that its waits run out: the kernel then

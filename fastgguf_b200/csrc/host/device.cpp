@@ -188,6 +188,22 @@ fg_dev_tensor Tensor::view() const {
 Arena::~Arena() {
     for (auto &l : lanes_)
         for (auto &b : l.blocks) cudaFree(b.p);
+    if (scratch_) cudaFree(scratch_);
+}
+
+void *Arena::scratch(size_t bytes) {
+    if (bytes <= scratch_bytes_) return scratch_;
+    if (frozen_) return nullptr;                       // (the warm-up run before a recording has sized it)
+    size_t size = bytes > 2 * scratch_bytes_ ? bytes : 2 * scratch_bytes_, free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b + scratch_bytes_ < size + ((size_t)1 << 30)) {
+        cudaGetLastError();
+        return nullptr;                                // a gigabyte stays free for what has no other path
+    }
+    if (scratch_) cudaFree(scratch_);                  // waits for the device
+    scratch_bytes_ = 0;
+    if (cudaMalloc(&scratch_, size) != cudaSuccess) { cudaGetLastError(); scratch_ = nullptr; return nullptr; }
+    scratch_bytes_ = size;
+    return scratch_;
 }
 
 void Arena::reset() {
@@ -239,6 +255,13 @@ void *Arena::alloc(size_t bytes) {
         size_t size = bytes > block_bytes_ ? bytes : block_bytes_;
         void *p = nullptr;
         cudaError_t e = cudaMalloc(&p, size);
+        if (e != cudaSuccess && scratch_) {
+            cudaGetLastError();
+            cudaFree(scratch_);                        // waits for the device
+            scratch_ = nullptr;
+            scratch_bytes_ = 0;
+            e = cudaMalloc(&p, size);
+        }
         if (e != cudaSuccess) {
             cudaGetLastError();
             fail(FG_E_DEVICE, format("out of device memory: the activations of this step need another %zu MiB (%s)",
@@ -264,7 +287,7 @@ size_t Arena::bytes_reserved() const {
     size_t n = 0;
     for (auto &l : lanes_)
         for (auto &b : l.blocks) n += b.size;
-    return n;
+    return n + scratch_bytes_;
 }
 
 DeviceBuffer::DeviceBuffer(size_t bytes, const char *what) : bytes_(bytes) {

@@ -79,6 +79,9 @@ public:
     ~Arena();
     Arena(const Arena &) = delete;
     void *alloc(size_t bytes);
+    // Memory that one launch uses and nothing reads afterwards: the same block for every caller, grown as needed.  Null where the
+    // device has no room to spare for it: the caller then takes a path that needs none, and an `alloc` that fails gives it back.
+    void *scratch(size_t bytes);
     Tensor matrix(int64_t rows, int64_t cols, int dtype);
     void reset();                       // a new step: every lane starts over
     void begin_layer(int i);            // allocations now go to the lane of layer i, which starts over
@@ -96,6 +99,8 @@ private:
     int cur_ = 0;
     size_t block_bytes_;
     bool frozen_ = false;
+    void *scratch_ = nullptr;
+    size_t scratch_bytes_ = 0;
 };
 
 // Device memory that lives as long as its owner.

@@ -213,3 +213,54 @@ def test_gemm_tc_prefill_split_along_k(M, N, K):
         bound = ((xw.double().abs() * inv[:, None]) @ w.double().abs().T).max().item()
         assert (got_n.double() - want_n).abs().max().item() <= 4e-6 * bound
     assert fast_gemm.pipeline_error() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(17, 256, 512), (64, 300, 520), (129, 1000, 2048), (257, 512, 8192), (300, 257, 1000), (700, 3072, 2048),
+                                   (513, 2048, 4096), (32, 90000, 512), (90000, 256, 512)])     # the last two: planes made in two portions
+def test_gemm_f32_on_planes(M, N, K):
+    """float32 by three bfloat16 planes: no further from float64 than the plain chain of fused multiply-adds is."""
+    from fastgguf_b200 import ops
+    from fastgguf_b200.ops import fast_gemm
+    a, w = _operands(M, N, K, torch.float32, 5)
+    wide = torch.cat([a, torch.full((M, 4), 7.0, device="cuda")], 1)[:, :K]             # rows further apart than they are long
+    want = a.double() @ w.double().T
+    got = fast_gemm.gemm_f32(wide, w)
+    plain = ops.gemm_generic(a, w, out_dtype=torch.float32)
+    _check(got, a, w, want, False)
+    assert (got.double() - want).norm() <= (plain.double() - want).norm()
+    res = torch.randn(M, N, device="cuda")
+    acc = res.clone()
+    fast_gemm.gemm_f32(a, w, out=acc, accumulate=True)
+    assert torch.equal(acc, got + res)                     # one rounding more, of the same sum
+    into = torch.full((M, N + 3), 9.0, device="cuda")      # rows of the output that no vector store may touch
+    fast_gemm.gemm_f32(a, w, out=into[:, 1:N + 1])
+    assert torch.equal(into[:, 1:N + 1], got) and (into[:, 0] == 9).all() and (into[:, N + 1:] == 9).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(40, 260, 512), (300, 2048, 2048)])
+def test_gemm_f32_on_planes_keeps_what_the_split_does_not_carry(M, N, K):
+    """Infinities, NaN, magnitudes above bfloat16's largest and sums that overflow on the way give what the plain kernel gives."""
+    from fastgguf_b200 import ops
+    from fastgguf_b200.ops import fast_gemm
+    a, w = _operands(M, N, K, torch.float32, 6)
+    a[3, 7] = float("inf")
+    a[5, 9] = float("nan")
+    a[8, 11] = 3.4e38
+    w[8] *= 1e-3
+    a[20, 0], a[20, 300], w[:, 300] = 3e38, 3e38, -w[:, 0]
+    w[17, 2] = float("-inf")
+    got, plain = fast_gemm.gemm_f32(a, w), ops.gemm_generic(a, w, out_dtype=torch.float32)
+    assert torch.equal(got.isnan(), plain.isnan()) and torch.equal(got.isinf(), plain.isinf())
+    ok = plain.isfinite()
+    assert torch.equal(got.sign()[~plain.isnan()], plain.sign()[~plain.isnan()]) or ok.any()
+    scale = a.double().nan_to_num(0, 0, 0).abs() @ w.double().nan_to_num(0, 0, 0).abs().T
+    assert ((got - plain).double().abs()[ok] <= 4e-6 * scale[ok]).all()
+
+
+def test_gemm_f32_on_planes_refuses_other_sizes():
+    from fastgguf_b200.ops import fast_gemm
+    for M, N, K in ((16, 512, 1024), (64, 128, 1024), (64, 512, 256), (64, 512, 1028)):
+        a, w = _operands(M, N, K, torch.float32, 7)
+        assert fast_gemm.gemm_f32(a, w) is None
+    a, w = _operands(64, 512, 1025, torch.float32, 7)
+    assert fast_gemm.gemm_f32(a[:, 1:], w[:, 1:]) is None  # rows that start off a 16-byte boundary
