@@ -44,6 +44,8 @@ attention_generic_kernel(const T *__restrict__ q, int ldq, void *__restrict__ ou
     float *qs = smem;                 // [qd]
     float *sc = smem + qd;            // [CHUNK]
     __shared__ float scratch[32];
+    pdl_launch_dependents_small_step(gridDim.x);
+    pdl_wait();
     int m = blockIdx.x, h = blockIdx.y;
     int kvh = h / (H / KV);
     const int VH = KV / v_share, vh = kvh / v_share;    // value heads in the pool, and this one
@@ -174,7 +176,8 @@ extern "C" int fg_attention_generic_ext(const void *q, int ldq, void *out, int l
     dim3 grid(M, H);
     size_t smem = (size_t)((latent ? hd + hdv : hd) + CHUNK + ATT_WARPS * hdv) * sizeof(float);
     if (smem > 48 * 1024) return FG_ERR_BAD_SIZE;
-#define ATT_LAUNCH(T, DPL) attention_generic_kernel<T, DPL><<<grid, ATT_THREADS, smem, stream>>>((const T *)q, ldq, out, ldo, \
+    int e = 0;
+#define ATT_LAUNCH(T, DPL) e = fg_launch(attention_generic_kernel<T, DPL>, grid, dim3(ATT_THREADS), smem, stream, (const T *)q, ldq, out, ldo, \
         positions, row_seq, block_table, table_width, (const T *)k_pool, (const T *)v_pool, H, KV, hd, hdv, page_size, scale, window, \
         window > 0 ? keep_first : 0, softcap, sinks, latent, v_share, out_f32)
 #define ATT_BY_SIZE(T) do { if (hdv <= 64) ATT_LAUNCH(T, 2); else if (hdv <= 128) ATT_LAUNCH(T, 4); else if (hdv <= 256) ATT_LAUNCH(T, 8); \
@@ -184,7 +187,7 @@ extern "C" int fg_attention_generic_ext(const void *q, int ldq, void *out, int l
     else return FG_ERR_BAD_DTYPE;
 #undef ATT_BY_SIZE
 #undef ATT_LAUNCH
-    return FG_LAUNCH_CHECK();
+    return e;
 }
 
 extern "C" int fg_attention_generic_kept(const void *q, int ldq, void *out, int ldo, int dtype,

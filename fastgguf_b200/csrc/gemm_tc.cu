@@ -1207,6 +1207,20 @@ static int make_map(CUtensorMap *map, const void *base, int rows, int K, int ld,
     return r == CUDA_SUCCESS ? 0 : FG_ERR_TENSORMAP;
 }
 
+// a [rows, K] float32 matrix, boxes of box_rows x 128, rows one after another in shared memory
+static int make_map_f32(CUtensorMap *map, const void *base, int rows, int K, int ld, int box_rows) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return FG_ERR_TENSORMAP;
+    cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
+    cuuint32_t box[2] = {128, (cuuint32_t)box_rows};
+    cuuint32_t estr[2] = {1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void *)base, dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : FG_ERR_TENSORMAP;
+}
+
 static int sm_count();
 template <int BN>
 static int launch_decode(const CUtensorMap &tmW, const CUtensorMap &tmX, GemmArgs a, dim3 grid, cudaStream_t stream) {
@@ -1540,6 +1554,7 @@ extern "C" int fg_gemm_tc_grouped(const void *X, int ldx, int rows, const void *
 }
 
 #include "gemm_f32_tc.cuh"
+#include "gemm_f32_stream.cuh"
 
 // For the test of the bounded waits: wait_limit_cycles > 0 sets how long a wait may last (0 restores the default of
 // about a second; values below half a millisecond act as half a millisecond), and skip_copy != 0 makes the decode

@@ -176,6 +176,16 @@ Tensor Linear::forward(Runtime &rt, const Tensor &a_in, const DeferredNorm *defe
     }
     if (deferred) a = deferred->materialize(rt);
     if (!rt.plain_kernels && a.dtype == FG_F32 && W.dtype == FG_F32 && out.dtype == FG_F32) {
+        if (M <= 16 && N >= 512 && K >= 512) {
+            count_launch();
+            ProfileScope scope("fg_gemm_f32_stream", profile_on() ? format("%lld x %lld, %lld rows%s", (long long)N, (long long)K, (long long)M, accumulate ? ", residual add" : "").c_str() : nullptr);
+            int code = FG_KERNEL("tc", fg_gemm_f32_stream)(a.ptr<float>(), (int)a.ld, W.ptr<float>(), (int)W.ld, out.ptr<float>(), (int)out.ld,
+                                                           accumulate ? 1 : 0, (int)M, (int)N, (int)K, rt.stream);
+            if (code != KERNEL_BAD_SIZE) {
+                check_kernel(code, "fg_gemm_f32_stream");
+                return out;
+            }
+        }
         // float32 operands as sums of three bfloat16 planes on the tensor cores (more than 16 rows, see gemm_f32_tc.cuh)
         const long long ws_bytes = M > 16 && N >= 256 && K >= 512 ? FG_KERNEL("tc", fg_gemm_f32_tc_workspace_bytes)((int)M, (int)N, (int)K) : 0;
         void *ws = ws_bytes > 0 ? rt.arena->scratch((size_t)ws_bytes) : nullptr;

@@ -29,6 +29,7 @@ register_signatures("tc", {
                       c_void_p, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p],
     "fg_gemm_tc_workspace_bytes": [c_int, c_int, c_int, c_int],
     "fg_gemm_tc_error": [],
+    "fg_gemm_f32_stream": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
     "fg_gemm_f32_tc_workspace_bytes": [c_int, c_int, c_int],
     "fg_gemm_f32_tc": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_longlong, c_void_p],
     "fg_gemm_tc_max_ss_tiles": [c_int],
@@ -184,4 +185,20 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = Non
     if code == _BAD_SIZE:
         return None
     check(code, "gemm_f32_tc")
+    return out
+
+
+def gemm_f32_stream(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, accumulate: bool = False) -> Optional[torch.Tensor]:
+    """a [M <= 16, K] times w [N, K] transposed, everything float32, weights streamed through shared memory.  None for
+    sizes or alignments the kernel does not take (the caller then uses ``ops.gemm_generic``)."""
+    if a.dtype != torch.float32 or w.dtype != torch.float32 or a.stride(1) != 1 or w.stride(1) != 1:
+        return None
+    M, K = a.shape
+    N = w.shape[0]
+    if out is None:
+        out = torch.empty((M, N), dtype=torch.float32, device=a.device)
+    code = lib("tc").fg_gemm_f32_stream(ptr(a), a.stride(0), ptr(w), w.stride(0), ptr(out), out.stride(0), int(accumulate), M, N, K, stream())
+    if code == _BAD_SIZE:
+        return None
+    check(code, "gemm_f32_stream")
     return out

@@ -264,3 +264,38 @@ def test_gemm_f32_on_planes_refuses_other_sizes():
         assert fast_gemm.gemm_f32(a, w) is None
     a, w = _operands(64, 512, 1025, torch.float32, 7)
     assert fast_gemm.gemm_f32(a[:, 1:], w[:, 1:]) is None  # rows that start off a 16-byte boundary
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 5, 8, 9, 16])
+@pytest.mark.parametrize("N,K", [(512, 512), (1000, 2048), (2048, 8192), (16384, 520), (20011, 1000), (9473, 644)])
+def test_gemm_f32_stream(M, N, K):
+    """Against float64 and, where a tile is tall enough for its order of additions, bit for bit what gemv_rows_kernel gives."""
+    from fastgguf_b200 import ops
+    from fastgguf_b200.ops import fast_gemm
+    a, w = _operands(M, N, K, torch.float32, 8)
+    got = fast_gemm.gemm_f32_stream(a, w)
+    _check(got, a, w, a.double() @ w.double().T, False)
+    if N == 20011 or N == 16384:
+        assert torch.equal(got, ops.gemm_generic(a, w, out_dtype=torch.float32))
+    # a row's result does not depend on the other rows of the step
+    assert torch.equal(fast_gemm.gemm_f32_stream(a[M - 1:].contiguous(), w)[0], got[M - 1])
+    wide = torch.full((M, K + 8), 7.0, device="cuda")
+    wide[:, 4:K + 4] = a
+    into = torch.full((M, N + 3), 9.0, device="cuda")
+    res = torch.randn(M, N, device="cuda")
+    into[:, 1:N + 1] = res
+    fast_gemm.gemm_f32_stream(wide[:, 4:K + 4], w, out=into[:, 1:N + 1], accumulate=True)
+    assert torch.equal(into[:, 1:N + 1], got + res) and (into[:, 0] == 9).all() and (into[:, N + 1:] == 9).all()
+    special = a.clone()
+    special[0, 3], special[M - 1, 5] = float("inf"), float("nan")
+    x, y = fast_gemm.gemm_f32_stream(special, w), ops.gemm_generic(special, w, out_dtype=torch.float32)
+    assert torch.equal(x.isnan(), y.isnan()) and torch.equal(x.isinf(), y.isinf())
+
+
+def test_gemm_f32_stream_refuses_other_sizes():
+    from fastgguf_b200.ops import fast_gemm
+    for M, N, K in ((17, 1024, 1024), (4, 500, 1024), (4, 1024, 508), (4, 1024, 1026)):
+        a, w = _operands(M, N, K, torch.float32, 7)
+        assert fast_gemm.gemm_f32_stream(a, w) is None
+    a, w = _operands(4, 1024, 1025, torch.float32, 7)
+    assert fast_gemm.gemm_f32_stream(a[:, 1:], w[:, 1:]) is None
