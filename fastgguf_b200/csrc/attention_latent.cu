@@ -423,7 +423,8 @@ latent_expand_kernel(const float *__restrict__ q, int ldq, const float *__restri
 template <typename T>
 __global__ void gate_slice_kernel(const T *__restrict__ x, int ldx, int stride, const float *__restrict__ gate, int ldg, T *__restrict__ out,
                                   int ldo, int H, int DV) {
-    pdl_wait();             // (stands between two tensor-memory kernels: its successor is released when it ends, not here)
+    pdl_launch_dependents_small_step(gridDim.x);
+    pdl_wait();
     const int m = blockIdx.x;
     for (int e = threadIdx.x; e < H * DV; e += blockDim.x) {
         const int h = e / DV, d = e - h * DV;
@@ -454,7 +455,7 @@ static int launch_latent(const void *q, int ldq, void *out, int ldo, const int *
                          ldq, (T *)out, ldo, positions, row_seq, block_table, table_width, (const T *)k_pool, (const T *)v_pool, H, R, DR, page_size,
                          scale, sinks, n_splits, part);
     if (code || n_splits == 1) return code;
-    return fg_launch(latent_merge_kernel<T>, dim3(H, M), dim3(128), 0, stream, (const float *)part, (T *)out, ldo, H, R, n_splits);
+    return fg_launch(latent_merge_kernel<T>, dim3(H, M), dim3(R <= 128 ? 128 : R <= 256 ? 256 : 512), 0, stream, (const float *)part, (T *)out, ldo, H, R, n_splits);
 }
 
 // q: [M, H * (R + DR)], out: [M, H * R], both of the cache's dtype.
@@ -512,7 +513,7 @@ extern "C" int fg_latent_decode_mma(const void *q, int ldq, void *out, int ldo, 
     }
 #undef LM_RUN
     if (code || n_splits == 1) return code;
-    return fg_launch(latent_merge_kernel<bf16>, dim3(H, M), dim3(128), 0, stream, (const float *)part, (bf16 *)out, ldo, H, R, n_splits);
+    return fg_launch(latent_merge_kernel<bf16>, dim3(H, M), dim3(R <= 128 ? 128 : R <= 256 ? 256 : 512), 0, stream, (const float *)part, (bf16 *)out, ldo, H, R, n_splits);
 }
 
 extern "C" int fg_seq_page_table(const int *cu_rows, int n_seq, int width, int page_size, int *table, cudaStream_t stream) {

@@ -529,8 +529,7 @@ extern "C" int fg_differential_combine(const float *maps, int ld, void *out, int
 template <typename T>
 __global__ void head_gate_kernel(T *__restrict__ x, int ldx, const float *__restrict__ gate, int ldg, int H, int DV, int pad, int vec) {
     extern __shared__ float head_gate_sig[];        // the row's H gates
-    // (no early release of the successor: this kernel stands between two tensor-memory contractions, and the second must not
-    // start beside the first while this one sits resident and waiting; the successor starts when this kernel has finished)
+    pdl_launch_dependents_small_step(gridDim.x);
     pdl_wait();
     const int m = blockIdx.x;
     T *row = x + (size_t)m * ldx;

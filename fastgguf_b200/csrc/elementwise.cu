@@ -321,8 +321,69 @@ extern "C" int fg_kv_append(const void *qkv, int dtype, int ld, int k_off, const
 // the row instead of three kernels.  Statistics and the sum are 32-bit; one block a row, fixed reduction order.
 // Without w_next, out (when given) receives the updated x[m] itself: the input of a sublayer that reads the stream as it is.
 // add_row ([E] or null) joins every row of x in the same sum.
-// VEC: rows are read and written four elements at a time (E % 4 == 0, 16-byte aligned rows)
-template <typename TO, bool VEC>
+// Two kernels: with rows that 16-byte accesses can walk (E % 4 == 0, aligned), a row lives in the block's registers, PER vectors of four a
+// thread: everything is asked for at once, the norm weights before the wait on the preceding kernel, and nothing is read twice.
+// The other walks the row element by element.  (The register form stands for a walk in three passes by 128 threads,
+// where each pass waited for its loads: 8 rows of 2,048 took 6.6 us, now 3.7.)
+// Vectors of four a thread holds, for a row of E numbers (at most 512 threads, E up to 16,384): with few rows (a decode step) latency counts, and a row is spread over many
+// threads; with many, memory bounds the kernel, and small blocks keep more rows in flight (4,925 rows of 2,048, norm_add_norm: 25.4 us in three passes, 29.8 at one vector a thread, 22.8 at four).
+static int row_vectors(int M, int E) {
+    if (M > 64) return E <= 4096 ? 4 : 8;
+    return E <= 2048 ? 1 : E <= 4096 ? 2 : E <= 8192 ? 4 : 8;
+}
+template <typename TO, int PER>
+__global__ void __launch_bounds__(512) norm_add_norm_regs_kernel(const float *__restrict__ t, const float *__restrict__ w_post, const float *__restrict__ add_row,
+                                          float *__restrict__ x, const float *__restrict__ w_next, TO *__restrict__ out, int E, float eps_post,
+                                          float eps_next) {
+    __shared__ float scratch[32];
+    pdl_launch_dependents_small_step(gridDim.x);
+    const int n4 = E / 4;
+    const size_t base = (size_t)blockIdx.x * E;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 g[PER], gn[PER], a[PER], v[PER];
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const int i = threadIdx.x + j * blockDim.x;
+        g[j] = i < n4 ? __ldg((const float4 *)w_post + i) : zero;
+        gn[j] = i < n4 && w_next ? __ldg((const float4 *)w_next + i) : zero;
+    }
+    pdl_wait();
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const int i = threadIdx.x + j * blockDim.x;
+        a[j] = i < n4 ? ((const float4 *)(t + base))[i] : zero;
+        v[j] = i < n4 ? ((const float4 *)(x + base))[i] : zero;
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < PER; j++) { ss += a[j].x * a[j].x; ss += a[j].y * a[j].y; ss += a[j].z * a[j].z; ss += a[j].w * a[j].w; }
+    ss = block_sum(ss, scratch);
+    const float inv = 1.0f / sqrtf(ss / (float)E + eps_post);
+    float ss2 = 0.f;
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const int i = threadIdx.x + j * blockDim.x;
+        v[j].x += a[j].x * inv * g[j].x; v[j].y += a[j].y * inv * g[j].y; v[j].z += a[j].z * inv * g[j].z; v[j].w += a[j].w * inv * g[j].w;
+        if (add_row && i < n4) {
+            const float4 r = ((const float4 *)add_row)[i];
+            v[j].x += r.x; v[j].y += r.y; v[j].z += r.z; v[j].w += r.w;
+        }
+        ss2 += v[j].x * v[j].x; ss2 += v[j].y * v[j].y; ss2 += v[j].z * v[j].z; ss2 += v[j].w * v[j].w;
+        if (i >= n4) continue;
+        ((float4 *)(x + base))[i] = v[j];
+        if (!w_next && out) store4<TO>(out + base + 4 * i, v[j].x, v[j].y, v[j].z, v[j].w);
+    }
+    if (!w_next) return;
+    ss2 = block_sum(ss2, scratch);
+    const float inv2 = 1.0f / sqrtf(ss2 / (float)E + eps_next);
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const int i = threadIdx.x + j * blockDim.x;
+        if (i < n4) store4<TO>(out + base + 4 * i, v[j].x * inv2 * gn[j].x, v[j].y * inv2 * gn[j].y, v[j].z * inv2 * gn[j].z, v[j].w * inv2 * gn[j].w);
+    }
+}
+
+template <typename TO>
 __global__ void norm_add_norm_kernel(const float *__restrict__ t, const float *__restrict__ w_post, const float *__restrict__ add_row, float *__restrict__ x,
                                      const float *__restrict__ w_next, TO *__restrict__ out, int E, float eps_post,
                                      float eps_next) {
@@ -332,47 +393,21 @@ __global__ void norm_add_norm_kernel(const float *__restrict__ t, const float *_
     pdl_wait();
     const size_t base = (size_t)blockIdx.x * E;
     float ss = 0.f;
-    if (VEC) {
-        const float4 *t4 = (const float4 *)(t + base);
-        for (int i = threadIdx.x; i < E / 4; i += blockDim.x) { float4 v = t4[i]; ss += v.x * v.x; ss += v.y * v.y; ss += v.z * v.z; ss += v.w * v.w; }
-    } else {
-        for (int i = threadIdx.x; i < E; i += blockDim.x) { float v = t[base + i]; ss += v * v; }
-    }
+    for (int i = threadIdx.x; i < E; i += blockDim.x) { float v = t[base + i]; ss += v * v; }
     ss = block_sum(ss, scratch);
     const float inv = 1.0f / sqrtf(ss / (float)E + eps_post);
     float ss2 = 0.f;
-    if (VEC) {
-        const float4 *t4 = (const float4 *)(t + base), *w4 = (const float4 *)w_post;
-        float4 *x4 = (float4 *)(x + base), *r4 = (float4 *)row;
-        for (int i = threadIdx.x; i < E / 4; i += blockDim.x) {
-            float4 a = t4[i], g = w4[i], v = x4[i];
-            v.x += a.x * inv * g.x; v.y += a.y * inv * g.y; v.z += a.z * inv * g.z; v.w += a.w * inv * g.w;
-            if (add_row) { const float4 b = ((const float4 *)add_row)[i]; v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w; }
-            x4[i] = v;
-            if (w_next) { r4[i] = v; ss2 += v.x * v.x; ss2 += v.y * v.y; ss2 += v.z * v.z; ss2 += v.w * v.w; }
-            else if (out) store4<TO>(out + base + 4 * i, v.x, v.y, v.z, v.w);
-        }
-    } else {
-        for (int i = threadIdx.x; i < E; i += blockDim.x) {
-            float v = x[base + i] + t[base + i] * inv * w_post[i];
-            if (add_row) v += add_row[i];
-            x[base + i] = v;
-            if (w_next) { row[i] = v; ss2 += v * v; }
-            else if (out) out[base + i] = from_f32<TO>(v);
-        }
+    for (int i = threadIdx.x; i < E; i += blockDim.x) {
+        float v = x[base + i] + t[base + i] * inv * w_post[i];
+        if (add_row) v += add_row[i];
+        x[base + i] = v;
+        if (w_next) { row[i] = v; ss2 += v * v; }
+        else if (out) out[base + i] = from_f32<TO>(v);
     }
     if (!w_next) return;
     ss2 = block_sum(ss2, scratch);
     const float inv2 = 1.0f / sqrtf(ss2 / (float)E + eps_next);
-    if (VEC) {
-        const float4 *r4 = (const float4 *)row, *w4 = (const float4 *)w_next;
-        for (int i = threadIdx.x; i < E / 4; i += blockDim.x) {
-            float4 v = r4[i], g = w4[i];
-            store4<TO>(out + base + 4 * i, v.x * inv2 * g.x, v.y * inv2 * g.y, v.z * inv2 * g.z, v.w * inv2 * g.w);
-        }
-    } else {
-        for (int i = threadIdx.x; i < E; i += blockDim.x) out[base + i] = from_f32<TO>(row[i] * inv2 * w_next[i]);
-    }
+    for (int i = threadIdx.x; i < E; i += blockDim.x) out[base + i] = from_f32<TO>(row[i] * inv2 * w_next[i]);
 }
 
 extern "C" int fg_norm_add_norm_row(const float *t, const float *w_post, const float *add_row, float *x, const float *w_next, void *out, int out_dtype,
@@ -381,15 +416,22 @@ extern "C" int fg_norm_add_norm_row(const float *t, const float *w_post, const f
     size_t smem = w_next ? (size_t)E * sizeof(float) : 0;
     if (smem > 48 * 1024) return FG_ERR_BAD_SIZE;
     const bool vec = E % 4 == 0 && ((((uintptr_t)t) | ((uintptr_t)w_post) | ((uintptr_t)x) | ((uintptr_t)w_next) | ((uintptr_t)out) | ((uintptr_t)add_row)) & 15) == 0;
-    int per = vec ? E / 4 : E;
-    int threads = per >= 1024 ? 256 : (per >= 256 ? 128 : 64);
     const bool wide = out_dtype == FG_F32 || (!w_next && !out);
     if (!wide && out_dtype != FG_BF16) return FG_ERR_BAD_DTYPE;
-#define NAN_LAUNCH(TO, VEC) fg_launch(norm_add_norm_kernel<TO, VEC>, dim3(M), dim3(threads), smem, stream, t, w_post, add_row, x, w_next, (TO *)out, E, \
-                                      eps_post, eps_next)
-    if (wide) return vec ? NAN_LAUNCH(float, true) : NAN_LAUNCH(float, false);
-    return vec ? NAN_LAUNCH(bf16, true) : NAN_LAUNCH(bf16, false);
-#undef NAN_LAUNCH
+#define NAN_REGS(TO, PER) fg_launch(norm_add_norm_regs_kernel<TO, PER>, dim3(M), dim3(threads), 0, stream, t, w_post, add_row, x, w_next, (TO *)out, E, eps_post, eps_next)
+#define NAN_RUN(TO)                                                                                                                        \
+    do {                                                                                                                                   \
+        if (vec && E <= 4096 * 4) {                                                                                                        \
+            const int per = row_vectors(M, E), threads = ((E / 4 + per - 1) / per + 31) / 32 * 32;                                         \
+            return per == 1 ? NAN_REGS(TO, 1) : per == 2 ? NAN_REGS(TO, 2) : per == 4 ? NAN_REGS(TO, 4) : NAN_REGS(TO, 8);                 \
+        }                                                                                                                                  \
+        return fg_launch(norm_add_norm_kernel<TO>, dim3(M), dim3(E >= 1024 ? 256 : 128), smem, stream, t, w_post, add_row, x, w_next, (TO *)out, E,          \
+                         eps_post, eps_next);                                                                                              \
+    } while (0)
+    if (wide) NAN_RUN(float);
+    NAN_RUN(bf16);
+#undef NAN_RUN
+#undef NAN_REGS
 }
 
 extern "C" int fg_norm_add_norm(const float *t, const float *w_post, float *x, const float *w_next, void *out, int out_dtype,
@@ -424,10 +466,71 @@ __global__ void pair_combine_kernel(const float *__restrict__ a, const float *__
     }
 }
 
+// the same for rows that 16-byte accesses can walk, PER vectors of four a thread in registers: both mixers' rows are asked for at once
+// and summed up together (8 rows of 2,048 with both norms: 10.2 -> 3.3 us; 4,925 rows 42.8 -> 20.7)
+template <int PER>
+__global__ void __launch_bounds__(512) pair_combine_regs_kernel(const float *__restrict__ a, const float *__restrict__ b, const float *__restrict__ w_a,
+                                         const float *__restrict__ w_b, float scale_a, float scale_b, float eps, float *__restrict__ out,
+                                         int E, int accumulate) {
+    __shared__ float scratch[2][32];
+    pdl_launch_dependents_small_step(gridDim.x);
+    const int n4 = E / 4, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
+    const size_t base = (size_t)blockIdx.x * E;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), one = make_float4(1.f, 1.f, 1.f, 1.f);
+    float4 wa[PER], wb[PER], va[PER], vb[PER], vo[PER];
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const int i = threadIdx.x + j * blockDim.x;
+        wa[j] = w_a && i < n4 ? __ldg((const float4 *)w_a + i) : one;
+        wb[j] = w_b && i < n4 ? __ldg((const float4 *)w_b + i) : one;
+    }
+    pdl_wait();
+    float sa = 0.f, sb = 0.f;
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const int i = threadIdx.x + j * blockDim.x;
+        va[j] = i < n4 ? ((const float4 *)(a + base))[i] : zero;
+        vb[j] = i < n4 ? ((const float4 *)(b + base))[i] : zero;
+        vo[j] = accumulate && i < n4 ? ((const float4 *)(out + base))[i] : zero;
+    }
+    float inv_a = 1.f, inv_b = 1.f;
+    if (w_a || w_b) {
+#pragma unroll
+        for (int j = 0; j < PER; j++) {
+            sa = fmaf(va[j].x, va[j].x, sa); sa = fmaf(va[j].y, va[j].y, sa); sa = fmaf(va[j].z, va[j].z, sa); sa = fmaf(va[j].w, va[j].w, sa);
+            sb = fmaf(vb[j].x, vb[j].x, sb); sb = fmaf(vb[j].y, vb[j].y, sb); sb = fmaf(vb[j].z, vb[j].z, sb); sb = fmaf(vb[j].w, vb[j].w, sb);
+        }
+        sa = warp_sum(sa); sb = warp_sum(sb);
+        if ((threadIdx.x & 31) == 0) { scratch[0][warp] = sa; scratch[1][warp] = sb; }
+        __syncthreads();
+        sa = sb = 0.f;
+        for (int i = 0; i < n_warps; i++) { sa += scratch[0][i]; sb += scratch[1][i]; }
+        if (w_a) inv_a = 1.0f / sqrtf(sa / (float)E + eps);
+        if (w_b) inv_b = 1.0f / sqrtf(sb / (float)E + eps);
+    }
+    auto one_of = [&](float xa, float ga, float xb, float gb, float o) {
+        const float ta = w_a ? xa * inv_a * ga : xa, tb = w_b ? xb * inv_b * gb : xb, v = fmaf(scale_a, ta, scale_b * tb);
+        return accumulate ? o + v : v;
+    };
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const int i = threadIdx.x + j * blockDim.x;
+        if (i < n4)
+            ((float4 *)(out + base))[i] = make_float4(one_of(va[j].x, wa[j].x, vb[j].x, wb[j].x, vo[j].x), one_of(va[j].y, wa[j].y, vb[j].y, wb[j].y, vo[j].y),
+                                                      one_of(va[j].z, wa[j].z, vb[j].z, wb[j].z, vo[j].z), one_of(va[j].w, wa[j].w, vb[j].w, wb[j].w, vo[j].w));
+    }
+}
+
 extern "C" int fg_pair_combine(const float *a, const float *b, const float *w_a, const float *w_b, float scale_a, float scale_b,
                                float eps, float *out, int M, int E, int accumulate, cudaStream_t stream) {
     if (M <= 0) return 0;
     if (E <= 0) return FG_ERR_BAD_SIZE;
+    if (E % 4 == 0 && E <= 8192 && (((uintptr_t)a | (uintptr_t)b | (uintptr_t)w_a | (uintptr_t)w_b | (uintptr_t)out) & 15) == 0) {
+        const int per = row_vectors(M, E), threads4 = ((E / 4 + per - 1) / per + 31) / 32 * 32;
+#define PC_REGS(PER) fg_launch(pair_combine_regs_kernel<PER>, dim3(M), dim3(threads4), 0, stream, a, b, w_a, w_b, scale_a, scale_b, eps, out, E, accumulate)
+        return per == 1 ? PC_REGS(1) : per == 2 ? PC_REGS(2) : per == 4 ? PC_REGS(4) : PC_REGS(8);
+#undef PC_REGS
+    }
     const int threads = E >= 2048 ? 256 : 128;
     return fg_launch(pair_combine_kernel, dim3(M), dim3(threads), 0, stream, a, b, w_a, w_b, scale_a, scale_b, eps, out, E, accumulate);
 }
@@ -572,8 +675,7 @@ template <typename TO>
 __global__ void rmsnorm_pair_kernel(const float *__restrict__ x, const float *__restrict__ w_a, const float *__restrict__ w_b,
                                     TO *__restrict__ out_a, TO *__restrict__ out_b, int E, float eps_a, float eps_b, int vec) {
     __shared__ float scratch[32];
-    // (no early release of the successor: this kernel stands between two tensor-memory contractions, and the second must not
-    // start beside the first while this one sits resident and waiting; the successor starts when this kernel has finished)
+    pdl_launch_dependents_small_step(gridDim.x);
     pdl_wait();
     const float *xi = x + (size_t)blockIdx.x * E;
     TO *oa = out_a + (size_t)blockIdx.x * E, *ob = out_b + (size_t)blockIdx.x * E;

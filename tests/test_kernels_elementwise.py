@@ -235,3 +235,80 @@ def test_decode_advance():
     ops.decode_advance(tokens, pos, torch.tensor([7, 8, 9], dtype=torch.int32).cuda(),
                        torch.tensor([1, 1, 0], dtype=torch.int32).cuda())
     assert tokens.cpu().tolist() == [7, 8, 9] and pos.cpu().tolist() == [11, 21, 0]
+
+
+def _call(module, name, *args):
+    """A launcher that has no Python wrapper: tensors by pointer, Python floats as C floats."""
+    import ctypes
+    from fastgguf_b200.ops.lib import lib, stream
+    fn = getattr(lib(module), name)
+    fn.argtypes, fn.restype = None, ctypes.c_int
+    conv = [ctypes.c_void_p(a.data_ptr()) if isinstance(a, torch.Tensor) else ctypes.c_void_p(0) if a is None
+            else ctypes.c_float(a) if isinstance(a, float) else a if isinstance(a, ctypes._SimpleCData) else ctypes.c_int(a) for a in args]
+    assert fn(*conv, stream()) == 0
+
+
+@pytest.mark.parametrize("M", [1, 64, 65])
+@pytest.mark.parametrize("E", [24, 132, 2048, 2052, 4096, 4100, 8192, 8196, 12288, 50, 2050])       # edges of the vectors a thread holds; last: element by element
+@pytest.mark.parametrize("added,next_norm", [(False, True), (True, True), (True, False)])
+def test_norm_add_norm(M, E, added, next_norm):
+    g = torch.Generator().manual_seed(M + E)
+    t, x, w, wn, row = (torch.randn(*s, generator=g).cuda() for s in ((M, E), (M, E), (E,), (E,), (E,)))
+    want = x.double() + t.double() / (t.double().square().mean(-1, keepdim=True) + 1e-6).sqrt() * w.double() + (row.double() if added else 0.0)
+    want_out = want / (want.square().mean(-1, keepdim=True) + 1e-5).sqrt() * wn.double() if next_norm else want
+    for dtype, tol in ((torch.float32, 4e-6), (torch.bfloat16, 2 ** -8)):
+        got, out = x.clone(), torch.full((M, E), 9.0, dtype=dtype, device="cuda")
+        _call("core", "fg_norm_add_norm_row", t, w, row if added else None, got, wn if next_norm else None, out, 0 if dtype == torch.float32 else 1, M, E, 1e-6, 1e-5)
+        assert (got.double() - want).abs().max() <= 4e-6 * want.abs().max()
+        assert ((out.double() - want_out).abs() <= tol * want_out.abs() + 4e-6 * want_out.abs().max()).all()
+
+
+@pytest.mark.parametrize("M", [2, 64, 65])
+@pytest.mark.parametrize("E", [24, 2048, 2052, 4100, 8192, 8196, 50])
+@pytest.mark.parametrize("norms,accumulate", [((True, True), 0), ((False, False), 1), ((True, False), 1)])
+def test_pair_combine(M, E, norms, accumulate):
+    g = torch.Generator().manual_seed(M + E)
+    a, b, out = (torch.randn(M, E, generator=g).cuda() for _ in range(3))
+    w = [torch.randn(E, generator=g).cuda() if n else None for n in norms]
+    side = [v.double() / (v.double().square().mean(-1, keepdim=True) + 1e-6).sqrt() * u.double() if u is not None else v.double() for v, u in zip((a, b), w)]
+    want = 0.7 * side[0] + 0.6 * side[1] + (out.double() if accumulate else 0.0)
+    _call("core", "fg_pair_combine", a, b, w[0], w[1], 0.7, 0.6, 1e-6, out, M, E, accumulate)
+    assert (out.double() - want).abs().max() <= 4e-6 * want.abs().max()
+
+
+@pytest.mark.parametrize("M", [3, 64, 65])
+@pytest.mark.parametrize("C,group", [(2048, 2048), (2056, 1028), (6144, 3072), (2048, 128), (1000, 250), (600, 300), (36, 12)])      # held in registers or not, by block or warp
+def test_gated_group_norm_and_unit_heads(M, C, group):
+    g = torch.Generator().manual_seed(C + group)
+    y, z, w = (torch.randn(*s, generator=g).cuda() for s in ((M, C), (M, C), (group,)))
+    rms = lambda v: v / (v.view(M, -1, group).square().mean(-1, keepdim=True).expand(-1, -1, group).reshape(M, C) + 1e-6).sqrt()      # noqa: E731
+    gate = torch.nn.functional.silu(z.double())
+    for first in (0, 1):
+        want = (rms(y.double() * gate) if first else rms(y.double())) * w.double().repeat(C // group) * (1.0 if first else gate)
+        out = torch.empty(M, C, device="cuda")
+        _call("mix", "fg_gated_group_norm", y, C, z, C, w, group, out, 0, C, M, C, group, 1e-6, first, 0)
+        assert (out.double() - want).abs().max() <= 4e-6 * want.abs().max()
+    heads = y.clone()
+    _call("mix", "fg_unit_heads", heads, C, C // group, group, 1e-6, 0.5, M)
+    v = y.double().view(M, -1, group)
+    assert (heads.double().view_as(v) - 0.5 * v / (v.square().sum(-1, keepdim=True) + 1e-6).sqrt()).abs().max() <= 4e-6
+
+
+@pytest.mark.parametrize("taps", [1, 3, 4, 6])
+@pytest.mark.parametrize("lengths", [(1, 1, 1), (5, 1, 40), (64, 3, 9)])
+def test_conv1d_silu(lengths, taps):
+    import ctypes
+    C, n = 1500, len(lengths)
+    g = torch.Generator().manual_seed(taps)
+    M = sum(lengths)
+    u, w, bias, state = (torch.randn(*s, generator=g).cuda() for s in ((M, C), (C, taps), (C,), (n, max(1, taps - 1), C)))
+    cu = torch.tensor([0] + list(np.cumsum(lengths)), dtype=torch.int32).cuda()
+    row_seq = torch.tensor([s for s, k in enumerate(lengths) for _ in range(k)], dtype=torch.int32).cuda()
+    slots = torch.arange(n, dtype=torch.int32).flip(0).contiguous().cuda()
+    out = torch.empty(M, C, device="cuda")
+    _call("mix", "fg_conv1d_silu", u, C, w, bias, taps, state, ctypes.c_longlong(state.stride(0)), row_seq, cu, slots, out, C, M, C)
+    for s in range(n):
+        rows = u[int(cu[s]):int(cu[s + 1])].double()
+        full = torch.cat([state[int(slots[s]), :taps - 1].double(), rows])
+        pre = bias.double() + sum(full[j:j + len(rows)] * w[:, j].double() for j in range(taps))
+        assert (out[int(cu[s]):int(cu[s + 1])].double() - torch.nn.functional.silu(pre)).abs().max() <= 4e-6 * pre.abs().max()
