@@ -8,14 +8,14 @@
 // 64 GB of keys and values a layer through L2, 5.6 ms a layer of Llama 1B (float32, 2,048 tokens) against 0.25 ms of arithmetic
 // at the FMA units' rate.  Here a CTA owns 128 rows = TQ consecutive tokens x the query heads of one KV head, and walks the
 // pages (64 keys) its rows may see, so a key is read once a CTA:
-//   S = Q K^T       8 x 8 (head size 64) or 8 x 4 scores a thread, operands in shared memory: 4 vector loads for 64 FMAs
+//   S = Q K^T       4 x 8 (head size 64) or 4 x 4 scores a thread, operands in shared memory as vectors of four
 //   online softmax  a row's scores lie in 8 (16) neighbouring lanes
-//   O = O c + P V   8 x 8 outputs a thread; a page's 64 products are summed from zero and then added to the scaled output, so
+//   O = O c + P V   4 x 8 outputs a thread; a page's 64 products are summed from zero and then added to the scaled output, so
 //                   that an output's chain of additions is 64 + pages long instead of one per key
 // K and V of a page have one buffer each, filled by cp.async: K of the next page arrives under the softmax and P V, V under
-// Q K^T.  Two CTAs an SM at head size 64 (101 KB of shared memory, 128 threads), one at 128 (169 KB, 256 threads).
-// One layer of Llama 1B, 2,048 tokens: 5,583 -> 772 us (22 TFLOP/s; with two warps a scheduler the latency of the shared-memory reads
-// still shows).
+// Q K^T.  Two CTAs an SM at head size 64 (101 KB of shared memory, 256 threads), one at 128 (169 KB, 512 threads).
+// One layer of Llama 1B, 2,048 tokens: 5,583 -> 723 us (24 TFLOP/s).  Eight rows a thread read shared memory less often but leave
+// two warps a scheduler: 772 us.
 // A row's keys are visited in ascending page order, so its result does not depend on the other rows of the step.
 #include "common.cuh"
 
@@ -29,7 +29,7 @@ __device__ __forceinline__ void f32_cp_commit() { asm volatile("cp.async.commit_
 __device__ __forceinline__ void f32_cp_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
 template <int HD> struct PrefillF32 {
-    static constexpr int TX = HD / 8, THREADS = 16 * TX, NK = PAGE / TX;       // lanes a row, threads, keys a thread
+    static constexpr int RPT = 4, TX = HD / 8, THREADS = ROWS / RPT * TX, NK = PAGE / TX;       // rows a thread, lanes a row, threads, keys a thread
     static constexpr int LDQ = ROWS + 4, LDK = HD + 4;
     // Q^T [HD][LDQ], P [PAGE][LDQ], K [PAGE][LDK], V [PAGE][HD]
     static constexpr int SMEM = (HD * LDQ + PAGE * LDQ + PAGE * LDK + PAGE * HD) * 4;
@@ -41,7 +41,7 @@ attn_prefill_f32_kernel(const float *__restrict__ q, int ldq, float *__restrict_
                         const int *__restrict__ seq_start, const int *__restrict__ block_table, int table_width,
                         const float *__restrict__ k_pool, const float *__restrict__ v_pool, int KV, int G, float scale, int window) {
     using C = PrefillF32<HD>;
-    constexpr int TX = C::TX, NT = C::THREADS, NK = C::NK, LDQ = C::LDQ, LDK = C::LDK;
+    constexpr int RPT = C::RPT, TX = C::TX, NT = C::THREADS, NK = C::NK, LDQ = C::LDQ, LDK = C::LDK;
     extern __shared__ __align__(16) float fsm[];
     float *Qs = fsm, *Ps = Qs + HD * LDQ, *Ks = Ps + PAGE * LDQ, *Vs = Ks + PAGE * LDK;
     const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
@@ -54,11 +54,11 @@ attn_prefill_f32_kernel(const float *__restrict__ q, int ldq, float *__restrict_
     const int *bt = block_table + (size_t)b * table_width;
     const size_t H_row = (size_t)kvh * G + g0;                           // the first query head of this CTA
 
-    // row r of the tile is token q0 + r / Gc and head g0 + r % Gc; a thread's rows are ty * 4 + i and 64 + ty * 4 + i
-    int hi[8], lo[8];
+    // row r of the tile is token q0 + r / Gc and head g0 + r % Gc; a thread's rows are ty * 4 + i
+    int hi[RPT], lo[RPT];
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const int r = ty * 4 + (i & 3) + (i >> 2) * 64, t = r / Gc;
+    for (int i = 0; i < RPT; i++) {
+        const int r = ty * RPT + i, t = r / Gc;
         const bool valid = t < tq && g0 + r % Gc < G;
         hi[i] = valid ? start + q0 + t : -1;
         lo[i] = valid ? first_visible_key(hi[i], window) : 0;
@@ -87,9 +87,9 @@ attn_prefill_f32_kernel(const float *__restrict__ q, int ldq, float *__restrict_
         Qs[c * LDQ + r] = v.x; Qs[(c + 1) * LDQ + r] = v.y; Qs[(c + 2) * LDQ + r] = v.z; Qs[(c + 3) * LDQ + r] = v.w;
     }
 
-    float acc[8][8], m_run[8], l_run[8];
+    float acc[RPT][8], m_run[RPT], l_run[RPT];
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
+    for (int i = 0; i < RPT; i++) {
         m_run[i] = -INFINITY; l_run[i] = 0.f;
 #pragma unroll
         for (int j = 0; j < 8; j++) acc[i][j] = 0.f;
@@ -97,9 +97,9 @@ attn_prefill_f32_kernel(const float *__restrict__ q, int ldq, float *__restrict_
     for (int page = page_begin; page < page_end; page++) {
         f32_cp_wait1();
         __syncthreads();                                                  // K of this page (and, the first time, Q) is here
-        float s[8][NK];
+        float s[RPT][NK];
 #pragma unroll
-        for (int i = 0; i < 8; i++)
+        for (int i = 0; i < RPT; i++)
 #pragma unroll
             for (int j = 0; j < NK; j++) s[i][j] = 0.f;
 #pragma unroll 2
@@ -109,13 +109,13 @@ attn_prefill_f32_kernel(const float *__restrict__ q, int ldq, float *__restrict_
             for (int j = 0; j < NK; j++) k4[j] = *(const float4 *)(Ks + (tx + TX * j) * LDK + d);
 #pragma unroll
             for (int dd = 0; dd < 4; dd++) {
-                const float4 a0 = *(const float4 *)(Qs + (d + dd) * LDQ + ty * 4), a1 = *(const float4 *)(Qs + (d + dd) * LDQ + ty * 4 + 64);
-                const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+                const float4 a0 = *(const float4 *)(Qs + (d + dd) * LDQ + ty * 4);
+                const float a[4] = {a0.x, a0.y, a0.z, a0.w};
 #pragma unroll
                 for (int j = 0; j < NK; j++) {
                     const float kk = dd == 0 ? k4[j].x : dd == 1 ? k4[j].y : dd == 2 ? k4[j].z : k4[j].w;
 #pragma unroll
-                    for (int i = 0; i < 8; i++) s[i][j] = fmaf(a[i], kk, s[i][j]);
+                    for (int i = 0; i < RPT; i++) s[i][j] = fmaf(a[i], kk, s[i][j]);
                 }
             }
         }
@@ -124,9 +124,9 @@ attn_prefill_f32_kernel(const float *__restrict__ q, int ldq, float *__restrict_
         f32_cp_commit();
         const bool whole = page >= whole_begin && page < whole_end;
         const int p0 = page * PAGE + tx;                                  // this thread's keys: p0 + TX * j
-        float corr[8];
+        float corr[RPT];
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
+        for (int i = 0; i < RPT; i++) {
             float mx = -INFINITY;
 #pragma unroll
             for (int j = 0; j < NK; j++) {
@@ -159,7 +159,6 @@ attn_prefill_f32_kernel(const float *__restrict__ q, int ldq, float *__restrict_
         for (int j = 0; j < NK; j++) {
             float *dst = Ps + (tx + TX * j) * LDQ + ty * 4;
             *(float4 *)dst = make_float4(s[0][j], s[1][j], s[2][j], s[3][j]);
-            *(float4 *)(dst + 64) = make_float4(s[4][j], s[5][j], s[6][j], s[7][j]);
         }
         f32_cp_wait1();
         __syncthreads();                                                  // P is written, V of this page is here
@@ -171,19 +170,19 @@ attn_prefill_f32_kernel(const float *__restrict__ q, int ldq, float *__restrict_
             for (int e = tid; e < PAGE * HD; e += NT) bad |= !(fabsf(Vs[e]) <= 3.402823466e38f);
             guarded = __syncthreads_or(bad);
         }
-        float pv[8][8];
+        float pv[RPT][8];
 #pragma unroll
-        for (int i = 0; i < 8; i++)
+        for (int i = 0; i < RPT; i++)
 #pragma unroll
             for (int j = 0; j < 8; j++) pv[i][j] = 0.f;
         if (!guarded) {
 #pragma unroll 4
             for (int k = 0; k < PAGE; k++) {
-                const float4 a0 = *(const float4 *)(Ps + k * LDQ + ty * 4), a1 = *(const float4 *)(Ps + k * LDQ + ty * 4 + 64);
+                const float4 a0 = *(const float4 *)(Ps + k * LDQ + ty * 4);
                 const float4 v0 = *(const float4 *)(Vs + k * HD + tx * 4), v1 = *(const float4 *)(Vs + k * HD + tx * 4 + HD / 2);
-                const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+                const float a[4] = {a0.x, a0.y, a0.z, a0.w}, v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
 #pragma unroll
-                for (int i = 0; i < 8; i++)
+                for (int i = 0; i < RPT; i++)
 #pragma unroll
                     for (int j = 0; j < 8; j++) pv[i][j] = fmaf(a[i], v[j], pv[i][j]);
             }
@@ -192,16 +191,16 @@ attn_prefill_f32_kernel(const float *__restrict__ q, int ldq, float *__restrict_
             for (int k = 0; k < PAGE; k++) {
                 const int p = page * PAGE + k;
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
+                for (int i = 0; i < RPT; i++) {
                     if (p > hi[i] || p < lo[i]) continue;
-                    const float a = Ps[k * LDQ + ty * 4 + (i & 3) + (i >> 2) * 64];
+                    const float a = Ps[k * LDQ + ty * 4 + i];
 #pragma unroll
                     for (int j = 0; j < 8; j++) pv[i][j] = fmaf(a, Vs[k * HD + tx * 4 + (j & 3) + (j >> 2) * (HD / 2)], pv[i][j]);
                 }
             }
         }
 #pragma unroll
-        for (int i = 0; i < 8; i++)
+        for (int i = 0; i < RPT; i++)
 #pragma unroll
             for (int j = 0; j < 8; j++) acc[i][j] = fmaf(acc[i][j], corr[i], pv[i][j]);
         __syncthreads();                                                  // V and P are free
@@ -209,9 +208,9 @@ attn_prefill_f32_kernel(const float *__restrict__ q, int ldq, float *__restrict_
         f32_cp_commit();
     }
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
+    for (int i = 0; i < RPT; i++) {
         if (hi[i] < 0) continue;
-        const int r = ty * 4 + (i & 3) + (i >> 2) * 64;
+        const int r = ty * 4 + i;
         float *dst = out + (size_t)(row0 + q0 + r / Gc) * ldo + (H_row + r % Gc) * HD + tx * 4;
         const float inv = l_run[i] > 0.f ? 1.0f / l_run[i] : 0.f;
         *(float4 *)dst = make_float4(acc[i][0] * inv, acc[i][1] * inv, acc[i][2] * inv, acc[i][3] * inv);
