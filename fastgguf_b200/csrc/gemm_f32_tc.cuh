@@ -317,10 +317,10 @@ static F32Plan f32_plan(int M, int N, int K) {
 
 // Scratch memory fg_gemm_f32_tc needs; 0: sizes it does not take.  Rows up to 16 belong to the weight-streaming kernel.  Short
 // reductions and narrow outputs (K < 512, N < 256) stay with the plain kernels: one or two rounds of their tiles take about
-// what the three launches here do.  From 17 rows on the planes won at every size measured (K 2,048 and 8,192, N 2,048 to 16,384, 24 to
+// what the three launches here do; so do small matrices (a megabyte) at up to 64 rows, which the weight-streaming kernel takes.  From 17 rows on the planes won at every size measured (K 2,048 and 8,192, N 2,048 to 16,384, 24 to
 // 2,048 rows: 2.7 to 13 times).
 extern "C" long long fg_gemm_f32_tc_workspace_bytes(int M, int N, int K) {
-    if (M <= 16 || N < 256 || K < 512 || K % 8) return 0;
+    if (M <= 16 || N < 256 || K < 512 || K % 8 || (M <= 64 && (long long)N * K <= 1 << 18)) return 0;
     const F32Plan p = f32_plan(M, N, K);
     return (long long)(p.a_bytes + p.w_bytes + p.part_bytes);
 }

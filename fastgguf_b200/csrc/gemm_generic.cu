@@ -2,7 +2,7 @@
 //
 // This is the true 32-bit path of every projection (no tensor cores, no TF32, no reduced
 // precision anywhere) and the any-size fallback of the bf16 path.  Three kernels by row count: a
-// weight-streaming one for up to 16 rows (a decode step), 64 x 64 tiles up to 64 rows, 128 x 128
+// weight-streaming one for up to 16 rows (a decode step; up to 64 rows of a small matrix), 64 x 64 tiles up to 64 rows, 128 x 128
 // tiles beyond.  In each the order of additions for an output depends on K alone, so a row's result
 // does not depend on how many other rows are in the batch; between the kernels the order differs
 // (rounding only).
@@ -21,6 +21,8 @@ gemm_generic_kernel(const TA *__restrict__ A, int lda, const TW *__restrict__ W,
                     void *__restrict__ C, int ldc, int out_dtype, int accumulate, int M, int N, int K) {
     __shared__ float As[TK][TM + 1];
     __shared__ float Ws[TK][TN + 1];
+    pdl_launch_dependents();               // (up to 64 rows: a small step)
+    pdl_wait();
     int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // tx: n direction, ty: m direction
     int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
     float acc[4][4];
@@ -166,6 +168,8 @@ gemv_rows_kernel(const TA *__restrict__ A, int lda, const TW *__restrict__ W, in
                  int out_dtype, int accumulate, int M, int N, int K) {
     constexpr int KC = MB <= 4 ? 2048 : MB == 8 ? 1024 : 512;       // 32 KB of activations at a time
     __shared__ __align__(16) float As[MB][KC];
+    pdl_launch_dependents();
+    pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n0 = (blockIdx.x * GEMV_WARPS + warp) * RPW;
     float acc[RPW][MB];
@@ -227,12 +231,18 @@ gemv_rows_kernel(const TA *__restrict__ A, int lda, const TW *__restrict__ W, in
 
 // The same for matrices of few rows (the projections of a layer): a block owns R weight rows and its warps split
 // the reduction length among them, each reading its part of the activations straight from global memory; the warps'
-// partial sums are added in warp order.  More, smaller blocks than above, and no stop-and-go between chunks.
+// partial sums are added in warp order.  More, smaller blocks than above, and no stop-and-go between chunks.  blockIdx.y counts
+// blocks of MB token rows: small matrices meet up to 64 rows this way.
 template <int MB, int R, typename TA, typename TW>
 __global__ void __launch_bounds__(GEMV_WARPS * 32)
 gemv_splitk_kernel(const TA *__restrict__ A, int lda, const TW *__restrict__ W, int ldw, void *__restrict__ C, int ldc,
                    int out_dtype, int accumulate, int M, int N, int K) {
     __shared__ float part[GEMV_WARPS][R][MB];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int m0 = blockIdx.y * MB;
+    A += (size_t)m0 * lda;
+    M -= m0;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n0 = blockIdx.x * R;
     const int slice = ((K + 127) / 128 + GEMV_WARPS - 1) / GEMV_WARPS * 128;     // a multiple of the warp's stride
@@ -278,26 +288,28 @@ gemv_splitk_kernel(const TA *__restrict__ A, int lda, const TW *__restrict__ W, 
         float v = 0.f;
 #pragma unroll
         for (int w = 0; w < GEMV_WARPS; w++) v += part[w][r][m];       // warp order
-        size_t idx = (size_t)m * ldc + n0 + r;
+        size_t idx = (size_t)(m0 + m) * ldc + n0 + r;
         if (accumulate) v += ((float *)C)[idx];
         store_as(C, out_dtype, idx, v);
     }
 }
 
 template <typename TA, typename TW>
-static void launch_gemv(const void *A, int lda, const void *W, int ldw, void *C, int ldc, int out_dtype, int accumulate, int M,
+static int launch_gemv(const void *A, int lda, const void *W, int ldw, void *C, int ldc, int out_dtype, int accumulate, int M,
                         int N, int K, cudaStream_t stream) {
     const bool many = N >= 16384;         // enough weight rows for four a warp to fill the GPU
     const int a_bytes = sizeof(TA);
     // the block-split kernel reads the activations with vector loads too
     const bool split = !many && lda % 4 == 0 && ((uintptr_t)A % (4 * a_bytes)) == 0;
     const int rows_per_block = many ? GEMV_WARPS * 4 : split ? (M <= 8 ? 4 : 2) : GEMV_WARPS;
-    dim3 grid((N + rows_per_block - 1) / rows_per_block);
+    if (M > 16 && !split) return FG_ERR_BAD_SIZE;         // (blocks of rows: the block-split kernel alone)
+    dim3 grid((N + rows_per_block - 1) / rows_per_block, (M + 15) / 16), block(GEMV_WARPS * 32);
+    int e = 0;
 #define GEMV_ARGS (const TA *)A, lda, (const TW *)W, ldw, C, ldc, out_dtype, accumulate, M, N, K
 #define GEMV(MB) do { \
-        if (many) gemv_rows_kernel<MB, 4, 2, TA, TW><<<grid, GEMV_WARPS * 32, 0, stream>>>(GEMV_ARGS); \
-        else if (split) gemv_splitk_kernel<MB, (MB <= 8 ? 4 : 2), TA, TW><<<grid, GEMV_WARPS * 32, 0, stream>>>(GEMV_ARGS); \
-        else gemv_rows_kernel<MB, 1, 8, TA, TW><<<grid, GEMV_WARPS * 32, 0, stream>>>(GEMV_ARGS); } while (0)
+        if (many) e = fg_launch(gemv_rows_kernel<MB, 4, 2, TA, TW>, grid, block, 0, stream, GEMV_ARGS); \
+        else if (split) e = fg_launch(gemv_splitk_kernel<MB, (MB <= 8 ? 4 : 2), TA, TW>, grid, block, 0, stream, GEMV_ARGS); \
+        else e = fg_launch(gemv_rows_kernel<MB, 1, 8, TA, TW>, grid, block, 0, stream, GEMV_ARGS); } while (0)
     if (M <= 1) GEMV(1);
     else if (M <= 2) GEMV(2);
     else if (M <= 4) GEMV(4);
@@ -305,6 +317,7 @@ static void launch_gemv(const void *A, int lda, const void *W, int ldw, void *C,
     else GEMV(16);
 #undef GEMV
 #undef GEMV_ARGS
+    return e;
 }
 
 // a_dtype / w_dtype / out_dtype: FG_F32 or FG_BF16.  accumulate=1 needs out_dtype == FG_F32.
@@ -315,13 +328,15 @@ extern "C" int fg_gemm_generic(const void *A, int a_dtype, int lda, const void *
     if (accumulate && out_dtype != FG_F32) return FG_ERR_BAD_DTYPE;
     // few rows and weight rows that 16-byte (f32) / 8-byte (bf16) loads can walk: the weight-streaming kernel
     const int w_bytes = w_dtype == FG_F32 ? 4 : 2;
-    if (M <= 16 && K % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)W % (4 * w_bytes)) == 0) {
-        if (a_dtype == FG_F32 && w_dtype == FG_F32) launch_gemv<float, float>(A, lda, W, ldw, C, ldc, out_dtype, accumulate, M, N, K, stream);
-        else if (a_dtype == FG_BF16 && w_dtype == FG_BF16) launch_gemv<bf16, bf16>(A, lda, W, ldw, C, ldc, out_dtype, accumulate, M, N, K, stream);
-        else if (a_dtype == FG_BF16 && w_dtype == FG_F32) launch_gemv<bf16, float>(A, lda, W, ldw, C, ldc, out_dtype, accumulate, M, N, K, stream);
-        else if (a_dtype == FG_F32 && w_dtype == FG_BF16) launch_gemv<float, bf16>(A, lda, W, ldw, C, ldc, out_dtype, accumulate, M, N, K, stream);
-        else return FG_ERR_BAD_DTYPE;
-        return FG_LAUNCH_CHECK();
+    // Up to 64 rows of a small matrix go there too, 16 rows a block: the 64 x 64 tiles below are one or two blocks then, whose
+    // walk along K waits for every load (39 rows x 64 x 192: 23 us, 16 rows a block 4.2).
+    if ((M <= 16 || (M <= 64 && (long long)N * K <= 1 << 18)) && K % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)W % (4 * w_bytes)) == 0) {
+        int e = FG_ERR_BAD_DTYPE;
+        if (a_dtype == FG_F32 && w_dtype == FG_F32) e = launch_gemv<float, float>(A, lda, W, ldw, C, ldc, out_dtype, accumulate, M, N, K, stream);
+        else if (a_dtype == FG_BF16 && w_dtype == FG_BF16) e = launch_gemv<bf16, bf16>(A, lda, W, ldw, C, ldc, out_dtype, accumulate, M, N, K, stream);
+        else if (a_dtype == FG_BF16 && w_dtype == FG_F32) e = launch_gemv<bf16, float>(A, lda, W, ldw, C, ldc, out_dtype, accumulate, M, N, K, stream);
+        else if (a_dtype == FG_F32 && w_dtype == FG_BF16) e = launch_gemv<float, bf16>(A, lda, W, ldw, C, ldc, out_dtype, accumulate, M, N, K, stream);
+        if (e != FG_ERR_BAD_SIZE) return e;
     }
     if (M > 64) {
         dim3 g2((N + T2 - 1) / T2, (M + T2 - 1) / T2);
@@ -342,7 +357,8 @@ extern "C" int fg_gemm_generic(const void *A, int a_dtype, int lda, const void *
     }
     dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM);
     if (grid.y > 65535) return FG_ERR_BAD_SIZE;
-#define LAUNCH(TA, TW) gemm_generic_kernel<TA, TW><<<grid, 256, 0, stream>>>( \
+    int e = 0;
+#define LAUNCH(TA, TW) e = fg_launch(gemm_generic_kernel<TA, TW>, grid, dim3(256), 0, stream, \
         (const TA *)A, lda, (const TW *)W, ldw, C, ldc, out_dtype, accumulate, M, N, K)
     if (a_dtype == FG_F32 && w_dtype == FG_F32) LAUNCH(float, float);
     else if (a_dtype == FG_BF16 && w_dtype == FG_BF16) LAUNCH(bf16, bf16);
@@ -350,5 +366,5 @@ extern "C" int fg_gemm_generic(const void *A, int a_dtype, int lda, const void *
     else if (a_dtype == FG_F32 && w_dtype == FG_BF16) LAUNCH(float, bf16);
     else return FG_ERR_BAD_DTYPE;
 #undef LAUNCH
-    return FG_LAUNCH_CHECK();
+    return e;
 }

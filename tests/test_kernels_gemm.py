@@ -25,6 +25,7 @@ def _check(got, a, w, want, out_is_bf16):
                                      (torch.bfloat16, torch.float32)])
 @pytest.mark.parametrize("M,N,K", [(1, 7, 5), (3, 200, 72), (70, 130, 257), (129, 65, 64),
                                    (16, 333, 1100), (9, 1000, 4096), (2, 31, 516),        # few rows: the weight-streaming kernel
+                                   (17, 64, 64), (24, 192, 64), (39, 64, 192), (64, 256, 1024), (33, 130, 516), (64, 512, 516),      # small matrices by 16 rows, and the first above
                                    (300, 260, 1000), (65, 128, 36), (200, 129, 130)])    # many rows: 128 x 128 tiles
 def test_gemm_generic(M, N, K, adt, wdt):
     from fastgguf_b200 import ops
@@ -215,7 +216,7 @@ def test_gemm_tc_prefill_split_along_k(M, N, K):
     assert fast_gemm.pipeline_error() == 0
 
 
-@pytest.mark.parametrize("M,N,K", [(17, 256, 512), (64, 300, 520), (129, 1000, 2048), (257, 512, 8192), (300, 257, 1000), (700, 3072, 2048),
+@pytest.mark.parametrize("M,N,K", [(17, 516, 512), (64, 700, 520), (65, 256, 512), (129, 1000, 2048), (257, 512, 8192), (300, 257, 1000), (700, 3072, 2048),
                                    (513, 2048, 4096), (32, 90000, 512), (90000, 256, 512)])     # the last two: planes made in two portions
 def test_gemm_f32_on_planes(M, N, K):
     """float32 by three bfloat16 planes: no further from float64 than the plain chain of fused multiply-adds is."""
@@ -237,7 +238,7 @@ def test_gemm_f32_on_planes(M, N, K):
     assert torch.equal(into[:, 1:N + 1], got) and (into[:, 0] == 9).all() and (into[:, N + 1:] == 9).all()
 
 
-@pytest.mark.parametrize("M,N,K", [(40, 260, 512), (300, 2048, 2048)])
+@pytest.mark.parametrize("M,N,K", [(40, 520, 512), (300, 2048, 2048)])
 def test_gemm_f32_on_planes_keeps_what_the_split_does_not_carry(M, N, K):
     """Infinities, NaN, magnitudes above bfloat16's largest and sums that overflow on the way give what the plain kernel gives."""
     from fastgguf_b200 import ops
@@ -259,7 +260,7 @@ def test_gemm_f32_on_planes_keeps_what_the_split_does_not_carry(M, N, K):
 
 def test_gemm_f32_on_planes_refuses_other_sizes():
     from fastgguf_b200.ops import fast_gemm
-    for M, N, K in ((16, 512, 1024), (64, 128, 1024), (64, 512, 256), (64, 512, 1028)):
+    for M, N, K in ((16, 512, 1024), (64, 256, 1024), (100, 128, 1024), (100, 512, 256), (100, 512, 1028)):
         a, w = _operands(M, N, K, torch.float32, 7)
         assert fast_gemm.gemm_f32(a, w) is None
     a, w = _operands(64, 512, 1025, torch.float32, 7)
