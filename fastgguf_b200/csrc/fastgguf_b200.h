@@ -278,6 +278,7 @@ int fg_gemm_f32_tc(const float *A, int lda, const float *W, int ldw, float *C, i
 /* the same product for up to 16 rows on the FMA units, weights streamed through shared memory */
 int fg_gemm_f32_stream(const float *A, int lda, const float *W, int ldw, float *C, int ldc, int accumulate, int M, int N, int K,
                        cudaStream_t stream);
+int fg_gemm_f32_stream_plan(int M, int N, int *out);   /* tests only */
 int fg_gemm_tc_error(void);
 /* tests only: shorten the bounded waits and make the decode kernel's pipeline stall, see gemm_tc.cu */
 int fg_gemm_tc_test_hook(long long wait_limit_cycles, int skip_copy);

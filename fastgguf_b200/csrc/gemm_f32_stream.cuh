@@ -164,15 +164,37 @@ gemm_f32_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
     }
 }
 
+// How the weight rows and the ring are cut.  With boxes dealt out over k_groups (low tiles, one tile a CTA) the ring's depth is a
+// multiple of k_groups, so that a stage always belongs to the same warps.  Otherwise a warp whose box lands early could come to a stage
+// for its second filling while the first, another warp's, is still under way, and the parity it waits for would be that of
+// the phase before: the wait would return at once.
+struct StreamPlan { int tile_rows, n_tiles, row_groups, k_groups, stages, part_bytes; };
+static StreamPlan stream_plan(int MB, int N) {
+    StreamPlan p{};
+    const int ctas = 2 * sm_count(), most = FST_WARPS * FST_RW, rounds = (N + ctas * most - 1) / (ctas * most);
+    p.tile_rows = (N + ctas * rounds - 1) / (ctas * rounds);
+    p.n_tiles = (N + p.tile_rows - 1) / p.tile_rows;
+    p.row_groups = (p.tile_rows + FST_RW - 1) / FST_RW;
+    p.k_groups = p.n_tiles <= ctas ? FST_WARPS / p.row_groups : 1;
+    p.part_bytes = p.k_groups > 1 ? FST_WARPS * ((FST_RW * MB + 31) / 32) * 128 : 0;
+    p.stages = (FST_RING - p.part_bytes) / ((p.tile_rows + MB) * FST_KC * 4);
+    if (p.stages > FST_MAX_STAGES) p.stages = FST_MAX_STAGES;
+    p.stages -= p.stages % p.k_groups;
+    return p;
+}
+// for the tests: {tile_rows, n_tiles, row_groups, k_groups, stages, bytes of shared memory}
+extern "C" int fg_gemm_f32_stream_plan(int M, int N, int *out) {
+    const int MB = M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : M <= 8 ? 8 : 16;
+    const StreamPlan p = stream_plan(MB, N);
+    out[0] = p.tile_rows; out[1] = p.n_tiles; out[2] = p.row_groups; out[3] = p.k_groups; out[4] = p.stages;
+    out[5] = p.stages * (p.tile_rows + MB) * FST_KC * 4 + p.part_bytes;
+    return 0;
+}
+
 template <int MB>
 static int launch_f32_stream(const float *A, int lda, const float *W, int ldw, float *C, int ldc, int accumulate, int M, int N, int K, cudaStream_t stream) {
-    const int ctas = 2 * sm_count(), most = FST_WARPS * FST_RW, rounds = (N + ctas * most - 1) / (ctas * most);
-    const int tile_rows = (N + ctas * rounds - 1) / (ctas * rounds), n_tiles = (N + tile_rows - 1) / tile_rows;
-    const int stage_bytes = (tile_rows + MB) * FST_KC * 4;
-    const int row_groups = (tile_rows + FST_RW - 1) / FST_RW, k_groups = FST_WARPS / row_groups;
-    const int part_bytes = k_groups > 1 ? FST_WARPS * ((FST_RW * MB + 31) / 32) * 128 : 0;
-    int stages = (FST_RING - part_bytes) / stage_bytes;
-    if (stages > FST_MAX_STAGES) stages = FST_MAX_STAGES;
+    const StreamPlan p = stream_plan(MB, N);
+    const int ctas = 2 * sm_count(), tile_rows = p.tile_rows;
     CUtensorMap tmW, tmX;
     int e = make_map_f32(&tmW, W, N, K, ldw, tile_rows);
     if (e) return e;
@@ -183,8 +205,9 @@ static int launch_f32_stream(const float *A, int lda, const float *W, int ldw, f
         cudaError_t ce = cudaFuncSetAttribute(gemm_f32_stream_kernel<MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, FST_RING + 128);
         if (ce != cudaSuccess) return (int)ce;
     }
-    return fg_launch(gemm_f32_stream_kernel<MB>, dim3(n_tiles < ctas ? n_tiles : ctas), dim3(FST_THREADS), (size_t)stages * stage_bytes + part_bytes + 128,
-                     stream, tmW, tmX, C, ldc, accumulate, M, N, K, tile_rows, n_tiles, stages, row_groups, k_groups);
+    return fg_launch(gemm_f32_stream_kernel<MB>, dim3(p.n_tiles < ctas ? p.n_tiles : ctas), dim3(FST_THREADS),
+                     (size_t)p.stages * (tile_rows + MB) * FST_KC * 4 + p.part_bytes + 128, stream, tmW, tmX, C, ldc, accumulate, M, N, K, tile_rows,
+                     p.n_tiles, p.stages, p.row_groups, p.k_groups);
 }
 
 // Up to 16 rows, everything float32.  FG_ERR_BAD_SIZE for what it does not take (gemm_generic.cu's kernels do): rows that 16-byte copies

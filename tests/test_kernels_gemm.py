@@ -300,3 +300,32 @@ def test_gemm_f32_stream_refuses_other_sizes():
         assert fast_gemm.gemm_f32_stream(a, w) is None
     a, w = _operands(4, 1024, 1025, torch.float32, 7)
     assert fast_gemm.gemm_f32_stream(a[:, 1:], w[:, 1:]) is None
+
+
+def test_gemm_f32_stream_ring_belongs_to_the_same_warps():
+    """Where boxes are dealt out over groups of warps, a stage of the ring always falls to the same group and a CTA has one tile:
+    the wait for a stage by its parity rests on that.  (A race: with ring depths that are no such multiple, an early box of a later round
+    now and then let a warp through; a wrong sum showed in one of a few runs.)"""
+    import ctypes
+    from fastgguf_b200.ops.lib import lib
+    out = (ctypes.c_int * 6)()
+    dealt = 0
+    for M in (1, 2, 4, 8, 16):
+        for N in list(range(512, 9000, 61)) + [16384, 28672, 128256]:
+            lib("tc").fg_gemm_f32_stream_plan(ctypes.c_int(M), ctypes.c_int(N), out)
+            rows, tiles, row_groups, k_groups, stages, bytes_ = out
+            assert rows * tiles >= N > rows * (tiles - 1) and row_groups * 4 >= rows and row_groups * k_groups <= 7
+            assert 2 <= stages <= 16 and stages >= k_groups and bytes_ <= 108 * 1024
+            if k_groups > 1:
+                dealt += 1
+                assert stages % k_groups == 0 and tiles <= 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    assert dealt > 100
+
+
+def test_gemm_f32_stream_repeats_bit_for_bit():
+    from fastgguf_b200.ops import fast_gemm
+    for M, N, K in ((9, 1000, 2048), (8, 2048, 8192), (3, 3072, 2048)):
+        a, w = _operands(M, N, K, torch.float32, 9)
+        first = fast_gemm.gemm_f32_stream(a, w)
+        for _ in range(300):
+            assert torch.equal(fast_gemm.gemm_f32_stream(a, w), first)
