@@ -321,31 +321,35 @@ extern "C" int fg_kv_append(const void *qkv, int dtype, int ld, int k_off, const
 // the row instead of three kernels.  Statistics and the sum are 32-bit; one block a row, fixed reduction order.
 // Without w_next, out (when given) receives the updated x[m] itself: the input of a sublayer that reads the stream as it is.
 // add_row ([E] or null) joins every row of x in the same sum.
-// Two kernels: with rows that 16-byte accesses can walk (E % 4 == 0, aligned), a row lives in the block's registers, PER vectors of four a
-// thread: everything is asked for at once, the norm weights before the wait on the preceding kernel, and nothing is read twice.
-// The other walks the row element by element.  (The register form stands for a walk in three passes by 128 threads,
-// where each pass waited for its loads: 8 rows of 2,048 took 6.6 us, now 3.7.)
-// Vectors of four a thread holds, for a row of E numbers (at most 512 threads, E up to 16,384): with few rows (a decode step) latency counts, and a row is spread over many
-// threads; with many, memory bounds the kernel, and small blocks keep more rows in flight (4,925 rows of 2,048, norm_add_norm: 25.4 us in three passes, 29.8 at one vector a thread, 22.8 at four).
-static int row_vectors(int M, int E) {
-    if (M > 64) return E <= 4096 ? 4 : 8;
-    return E <= 2048 ? 1 : E <= 4096 ? 2 : E <= 8192 ? 4 : 8;
-}
+// Three forms, one order of additions: the order depends on E and the alignment alone, never on the number of rows, so that a row
+// gives the same numbers in every step.  A thread sums every threads-th vector of four (element, where 16-byte accesses cannot walk the
+// rows) in rising order, the block adds lanes and then warps.
+//   registers (E up to 12,288) everything is asked for at once, the norm weights before the wait on the preceding kernel, nothing
+//                              is read twice.  Three passes, each waiting for its loads, against this, us a launch alone: 8 rows of
+//                              2,048 3.3 : 2.3, 4,925 rows 24.0 : 20.6 (5.9 TB/s); 8 of 8,192 5.3 : 3.7, 4,925 rows 101 : 92
+//   three passes               longer rows, whose numbers do not fit the registers of 256 threads (with a next norm they are refused: they would
+//                              have to fit the 48 KB of shared memory where the updated row waits)
+//   element by element         rows that 16-byte accesses cannot walk
+static int row_threads(int per_row) { return per_row >= 1024 ? 256 : per_row >= 256 ? 128 : 64; }
+
+// PER: vectors of four a thread holds.  From eight on, the next norm's weights are fetched when they are used: with them in registers
+// a second block would not fit the SM.
 template <typename TO, int PER>
-__global__ void __launch_bounds__(512) norm_add_norm_regs_kernel(const float *__restrict__ t, const float *__restrict__ w_post, const float *__restrict__ add_row,
-                                          float *__restrict__ x, const float *__restrict__ w_next, TO *__restrict__ out, int E, float eps_post,
-                                          float eps_next) {
+__global__ void __launch_bounds__(256, PER == 8 ? 2 : 1)
+norm_add_norm_regs_kernel(const float *__restrict__ t, const float *__restrict__ w_post, const float *__restrict__ add_row, float *__restrict__ x,
+                          const float *__restrict__ w_next, TO *__restrict__ out, int E, float eps_post, float eps_next) {
     __shared__ float scratch[32];
     pdl_launch_dependents_small_step(gridDim.x);
+    constexpr bool AHEAD = PER <= 4;
     const int n4 = E / 4;
     const size_t base = (size_t)blockIdx.x * E;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 g[PER], gn[PER], a[PER], v[PER];
+    float4 g[PER], gn[AHEAD ? PER : 1], a[PER], v[PER];
 #pragma unroll
     for (int j = 0; j < PER; j++) {
         const int i = threadIdx.x + j * blockDim.x;
         g[j] = i < n4 ? __ldg((const float4 *)w_post + i) : zero;
-        gn[j] = i < n4 && w_next ? __ldg((const float4 *)w_next + i) : zero;
+        if (AHEAD) gn[AHEAD ? j : 0] = i < n4 && w_next ? __ldg((const float4 *)w_next + i) : zero;
     }
     pdl_wait();
 #pragma unroll
@@ -379,59 +383,89 @@ __global__ void __launch_bounds__(512) norm_add_norm_regs_kernel(const float *__
 #pragma unroll
     for (int j = 0; j < PER; j++) {
         const int i = threadIdx.x + j * blockDim.x;
-        if (i < n4) store4<TO>(out + base + 4 * i, v[j].x * inv2 * gn[j].x, v[j].y * inv2 * gn[j].y, v[j].z * inv2 * gn[j].z, v[j].w * inv2 * gn[j].w);
+        if (i >= n4) continue;
+        const float4 n = AHEAD ? gn[AHEAD ? j : 0] : __ldg((const float4 *)w_next + i);
+        store4<TO>(out + base + 4 * i, v[j].x * inv2 * n.x, v[j].y * inv2 * n.y, v[j].z * inv2 * n.z, v[j].w * inv2 * n.w);
     }
 }
 
-template <typename TO>
+template <typename TO, bool VEC>
 __global__ void norm_add_norm_kernel(const float *__restrict__ t, const float *__restrict__ w_post, const float *__restrict__ add_row, float *__restrict__ x,
                                      const float *__restrict__ w_next, TO *__restrict__ out, int E, float eps_post,
                                      float eps_next) {
+    extern __shared__ __align__(16) float row[];
     __shared__ float scratch[32];
-    extern __shared__ __align__(16) float row[];        // [E] the updated residual row, when a next norm is wanted
     pdl_launch_dependents_small_step(gridDim.x);
     pdl_wait();
     const size_t base = (size_t)blockIdx.x * E;
     float ss = 0.f;
-    for (int i = threadIdx.x; i < E; i += blockDim.x) { float v = t[base + i]; ss += v * v; }
+    if (VEC) {
+        const float4 *t4 = (const float4 *)(t + base);
+        for (int i = threadIdx.x; i < E / 4; i += blockDim.x) { float4 v = t4[i]; ss += v.x * v.x; ss += v.y * v.y; ss += v.z * v.z; ss += v.w * v.w; }
+    } else {
+        for (int i = threadIdx.x; i < E; i += blockDim.x) { float v = t[base + i]; ss += v * v; }
+    }
     ss = block_sum(ss, scratch);
     const float inv = 1.0f / sqrtf(ss / (float)E + eps_post);
     float ss2 = 0.f;
-    for (int i = threadIdx.x; i < E; i += blockDim.x) {
-        float v = x[base + i] + t[base + i] * inv * w_post[i];
-        if (add_row) v += add_row[i];
-        x[base + i] = v;
-        if (w_next) { row[i] = v; ss2 += v * v; }
-        else if (out) out[base + i] = from_f32<TO>(v);
+    if (VEC) {
+        const float4 *t4 = (const float4 *)(t + base), *w4 = (const float4 *)w_post;
+        float4 *x4 = (float4 *)(x + base), *r4 = (float4 *)row;
+        for (int i = threadIdx.x; i < E / 4; i += blockDim.x) {
+            float4 a = t4[i], g = w4[i], v = x4[i];
+            v.x += a.x * inv * g.x; v.y += a.y * inv * g.y; v.z += a.z * inv * g.z; v.w += a.w * inv * g.w;
+            if (add_row) { const float4 b = ((const float4 *)add_row)[i]; v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w; }
+            x4[i] = v;
+            if (w_next) { r4[i] = v; ss2 += v.x * v.x; ss2 += v.y * v.y; ss2 += v.z * v.z; ss2 += v.w * v.w; }
+            else if (out) store4<TO>(out + base + 4 * i, v.x, v.y, v.z, v.w);
+        }
+    } else {
+        for (int i = threadIdx.x; i < E; i += blockDim.x) {
+            float v = x[base + i] + t[base + i] * inv * w_post[i];
+            if (add_row) v += add_row[i];
+            x[base + i] = v;
+            if (w_next) { row[i] = v; ss2 += v * v; }
+            else if (out) out[base + i] = from_f32<TO>(v);
+        }
     }
     if (!w_next) return;
     ss2 = block_sum(ss2, scratch);
     const float inv2 = 1.0f / sqrtf(ss2 / (float)E + eps_next);
-    for (int i = threadIdx.x; i < E; i += blockDim.x) out[base + i] = from_f32<TO>(row[i] * inv2 * w_next[i]);
+    if (VEC) {
+        const float4 *r4 = (const float4 *)row, *w4 = (const float4 *)w_next;
+        for (int i = threadIdx.x; i < E / 4; i += blockDim.x) {
+            float4 v = r4[i], g = w4[i];
+            store4<TO>(out + base + 4 * i, v.x * inv2 * g.x, v.y * inv2 * g.y, v.z * inv2 * g.z, v.w * inv2 * g.w);
+        }
+    } else {
+        for (int i = threadIdx.x; i < E; i += blockDim.x) out[base + i] = from_f32<TO>(row[i] * inv2 * w_next[i]);
+    }
 }
 
 extern "C" int fg_norm_add_norm_row(const float *t, const float *w_post, const float *add_row, float *x, const float *w_next, void *out, int out_dtype,
                                     int M, int E, float eps_post, float eps_next, cudaStream_t stream) {
     if (M <= 0) return 0;
-    size_t smem = w_next ? (size_t)E * sizeof(float) : 0;
-    if (smem > 48 * 1024) return FG_ERR_BAD_SIZE;
     const bool vec = E % 4 == 0 && ((((uintptr_t)t) | ((uintptr_t)w_post) | ((uintptr_t)x) | ((uintptr_t)w_next) | ((uintptr_t)out) | ((uintptr_t)add_row)) & 15) == 0;
     const bool wide = out_dtype == FG_F32 || (!w_next && !out);
     if (!wide && out_dtype != FG_BF16) return FG_ERR_BAD_DTYPE;
-#define NAN_REGS(TO, PER) fg_launch(norm_add_norm_regs_kernel<TO, PER>, dim3(M), dim3(threads), 0, stream, t, w_post, add_row, x, w_next, (TO *)out, E, eps_post, eps_next)
-#define NAN_RUN(TO)                                                                                                                        \
-    do {                                                                                                                                   \
-        if (vec && E <= 4096 * 4) {                                                                                                        \
-            const int per = row_vectors(M, E), threads = ((E / 4 + per - 1) / per + 31) / 32 * 32;                                         \
-            return per == 1 ? NAN_REGS(TO, 1) : per == 2 ? NAN_REGS(TO, 2) : per == 4 ? NAN_REGS(TO, 4) : NAN_REGS(TO, 8);                 \
-        }                                                                                                                                  \
-        return fg_launch(norm_add_norm_kernel<TO>, dim3(M), dim3(E >= 1024 ? 256 : 128), smem, stream, t, w_post, add_row, x, w_next, (TO *)out, E,          \
-                         eps_post, eps_next);                                                                                              \
+    const int per_row = vec ? E / 4 : E, threads = row_threads(per_row), per = (per_row + threads - 1) / threads;
+    const bool regs = vec && per <= 12;
+    const size_t smem = w_next ? (size_t)E * sizeof(float) : 0;
+    if (!regs && smem > 48 * 1024 - 128) return FG_ERR_BAD_SIZE;        // (128 bytes: the block sums)
+#define NAN_ARGS t, w_post, add_row, x, w_next
+#define NAN_REGS(TO, PER) fg_launch(norm_add_norm_regs_kernel<TO, PER>, dim3(M), dim3(threads), 0, stream, NAN_ARGS, (TO *)out, E, eps_post, eps_next)
+#define NAN_PASSES(TO, VEC) fg_launch(norm_add_norm_kernel<TO, VEC>, dim3(M), dim3(threads), smem, stream, NAN_ARGS, (TO *)out, E, eps_post, eps_next)
+#define NAN_RUN(TO) \
+    do { \
+        if (!regs) return vec ? NAN_PASSES(TO, true) : NAN_PASSES(TO, false); \
+        return per <= 1 ? NAN_REGS(TO, 1) : per <= 2 ? NAN_REGS(TO, 2) : per <= 4 ? NAN_REGS(TO, 4) : per <= 8 ? NAN_REGS(TO, 8) : NAN_REGS(TO, 12); \
     } while (0)
     if (wide) NAN_RUN(float);
     NAN_RUN(bf16);
 #undef NAN_RUN
+#undef NAN_PASSES
 #undef NAN_REGS
+#undef NAN_ARGS
 }
 
 extern "C" int fg_norm_add_norm(const float *t, const float *w_post, float *x, const float *w_next, void *out, int out_dtype,
@@ -466,40 +500,50 @@ __global__ void pair_combine_kernel(const float *__restrict__ a, const float *__
     }
 }
 
-// the same for rows that 16-byte accesses can walk, PER vectors of four a thread in registers: both mixers' rows are asked for at once
-// and summed up together (8 rows of 2,048 with both norms: 10.2 -> 3.3 us; 4,925 rows 42.8 -> 20.7)
+// The same, bit for bit, for rows that 16-byte accesses can walk: both mixers' rows are asked for at once, PER vectors of four a thread in
+// registers, the weights before the wait on the preceding kernel (up to four vectors).  The order of additions is that of the form
+// above - a thread sums every threads-th number - so the rows pass through shared memory on their way to the sums.
+// Against the form above, both norms, us a launch alone: 8 rows of 2,048 5.9 : 2.4, 4,925 rows 55 : 25.7 (4.7 TB/s); 8 of 8,192 18.4 : 5.5,
+// 4,925 rows 228 : 103.  (Sums of a thread's own vectors would spare the way through shared memory, 4,925 rows of 2,048 22.9 us, but they
+// are added in another order.)
 template <int PER>
-__global__ void __launch_bounds__(512) pair_combine_regs_kernel(const float *__restrict__ a, const float *__restrict__ b, const float *__restrict__ w_a,
-                                         const float *__restrict__ w_b, float scale_a, float scale_b, float eps, float *__restrict__ out,
-                                         int E, int accumulate) {
+__global__ void __launch_bounds__(256, PER > 4 ? 2 : 1)
+pair_combine_regs_kernel(const float *__restrict__ a, const float *__restrict__ b, const float *__restrict__ w_a, const float *__restrict__ w_b,
+                         float scale_a, float scale_b, float eps, float *__restrict__ out, int E, int accumulate) {
+    extern __shared__ __align__(16) float rows[];          // [2][E] where there is a norm
     __shared__ float scratch[2][32];
     pdl_launch_dependents_small_step(gridDim.x);
+    constexpr bool AHEAD = PER <= 4;
     const int n4 = E / 4, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
     const size_t base = (size_t)blockIdx.x * E;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), one = make_float4(1.f, 1.f, 1.f, 1.f);
-    float4 wa[PER], wb[PER], va[PER], vb[PER], vo[PER];
+    float4 wa[AHEAD ? PER : 1], wb[AHEAD ? PER : 1], va[PER], vb[PER];
+    if (AHEAD) {
 #pragma unroll
-    for (int j = 0; j < PER; j++) {
-        const int i = threadIdx.x + j * blockDim.x;
-        wa[j] = w_a && i < n4 ? __ldg((const float4 *)w_a + i) : one;
-        wb[j] = w_b && i < n4 ? __ldg((const float4 *)w_b + i) : one;
+        for (int j = 0; j < PER; j++) {
+            const int i = threadIdx.x + j * blockDim.x;
+            wa[AHEAD ? j : 0] = w_a && i < n4 ? __ldg((const float4 *)w_a + i) : one;
+            wb[AHEAD ? j : 0] = w_b && i < n4 ? __ldg((const float4 *)w_b + i) : one;
+        }
     }
     pdl_wait();
-    float sa = 0.f, sb = 0.f;
 #pragma unroll
     for (int j = 0; j < PER; j++) {
         const int i = threadIdx.x + j * blockDim.x;
         va[j] = i < n4 ? ((const float4 *)(a + base))[i] : zero;
         vb[j] = i < n4 ? ((const float4 *)(b + base))[i] : zero;
-        vo[j] = accumulate && i < n4 ? ((const float4 *)(out + base))[i] : zero;
     }
     float inv_a = 1.f, inv_b = 1.f;
     if (w_a || w_b) {
 #pragma unroll
         for (int j = 0; j < PER; j++) {
-            sa = fmaf(va[j].x, va[j].x, sa); sa = fmaf(va[j].y, va[j].y, sa); sa = fmaf(va[j].z, va[j].z, sa); sa = fmaf(va[j].w, va[j].w, sa);
-            sb = fmaf(vb[j].x, vb[j].x, sb); sb = fmaf(vb[j].y, vb[j].y, sb); sb = fmaf(vb[j].z, vb[j].z, sb); sb = fmaf(vb[j].w, vb[j].w, sb);
+            const int i = threadIdx.x + j * blockDim.x;
+            if (i < n4) { ((float4 *)rows)[i] = va[j]; ((float4 *)(rows + E))[i] = vb[j]; }
         }
+        __syncthreads();
+        float sa = 0.f, sb = 0.f;
+#pragma unroll 4
+        for (int i = threadIdx.x; i < E; i += blockDim.x) { sa = fmaf(rows[i], rows[i], sa); sb = fmaf(rows[E + i], rows[E + i], sb); }
         sa = warp_sum(sa); sb = warp_sum(sb);
         if ((threadIdx.x & 31) == 0) { scratch[0][warp] = sa; scratch[1][warp] = sb; }
         __syncthreads();
@@ -508,16 +552,23 @@ __global__ void __launch_bounds__(512) pair_combine_regs_kernel(const float *__r
         if (w_a) inv_a = 1.0f / sqrtf(sa / (float)E + eps);
         if (w_b) inv_b = 1.0f / sqrtf(sb / (float)E + eps);
     }
-    auto one_of = [&](float xa, float ga, float xb, float gb, float o) {
-        const float ta = w_a ? xa * inv_a * ga : xa, tb = w_b ? xb * inv_b * gb : xb, v = fmaf(scale_a, ta, scale_b * tb);
-        return accumulate ? o + v : v;
+    auto one_of = [&](float xa, float ga, float xb, float gb) {
+        const float ta = w_a ? xa * inv_a * ga : xa, tb = w_b ? xb * inv_b * gb : xb;
+        return fmaf(scale_a, ta, scale_b * tb);
     };
 #pragma unroll
     for (int j = 0; j < PER; j++) {
         const int i = threadIdx.x + j * blockDim.x;
-        if (i < n4)
-            ((float4 *)(out + base))[i] = make_float4(one_of(va[j].x, wa[j].x, vb[j].x, wb[j].x, vo[j].x), one_of(va[j].y, wa[j].y, vb[j].y, wb[j].y, vo[j].y),
-                                                      one_of(va[j].z, wa[j].z, vb[j].z, wb[j].z, vo[j].z), one_of(va[j].w, wa[j].w, vb[j].w, wb[j].w, vo[j].w));
+        if (i >= n4) continue;
+        const float4 ga = AHEAD ? wa[AHEAD ? j : 0] : w_a ? __ldg((const float4 *)w_a + i) : one, gb = AHEAD ? wb[AHEAD ? j : 0] : w_b ? __ldg((const float4 *)w_b + i) : one;
+        float4 v = make_float4(one_of(va[j].x, ga.x, vb[j].x, gb.x), one_of(va[j].y, ga.y, vb[j].y, gb.y), one_of(va[j].z, ga.z, vb[j].z, gb.z),
+                               one_of(va[j].w, ga.w, vb[j].w, gb.w));
+        float4 *dst = (float4 *)(out + base) + i;
+        if (accumulate) {
+            const float4 o = *dst;
+            v = make_float4(o.x + v.x, o.y + v.y, o.z + v.z, o.w + v.w);
+        }
+        *dst = v;
     }
 }
 
@@ -525,13 +576,19 @@ extern "C" int fg_pair_combine(const float *a, const float *b, const float *w_a,
                                float eps, float *out, int M, int E, int accumulate, cudaStream_t stream) {
     if (M <= 0) return 0;
     if (E <= 0) return FG_ERR_BAD_SIZE;
+    const int threads = E >= 2048 ? 256 : 128;
     if (E % 4 == 0 && E <= 8192 && (((uintptr_t)a | (uintptr_t)b | (uintptr_t)w_a | (uintptr_t)w_b | (uintptr_t)out) & 15) == 0) {
-        const int per = row_vectors(M, E), threads4 = ((E / 4 + per - 1) / per + 31) / 32 * 32;
-#define PC_REGS(PER) fg_launch(pair_combine_regs_kernel<PER>, dim3(M), dim3(threads4), 0, stream, a, b, w_a, w_b, scale_a, scale_b, eps, out, E, accumulate)
-        return per == 1 ? PC_REGS(1) : per == 2 ? PC_REGS(2) : per == 4 ? PC_REGS(4) : PC_REGS(8);
+        const int per = (E / 4 + threads - 1) / threads;
+        const size_t smem = w_a || w_b ? (size_t)E * 2 * sizeof(float) : 0;
+        static FgPerDevice configured;
+        if (per > 4 && fg_needs_setup(configured)) {
+            cudaError_t e = cudaFuncSetAttribute(pair_combine_regs_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8192 * 2 * (int)sizeof(float));
+            if (e != cudaSuccess) return (int)e;
+        }
+#define PC_REGS(PER) fg_launch(pair_combine_regs_kernel<PER>, dim3(M), dim3(threads), smem, stream, a, b, w_a, w_b, scale_a, scale_b, eps, out, E, accumulate)
+        return per <= 1 ? PC_REGS(1) : per <= 2 ? PC_REGS(2) : per <= 4 ? PC_REGS(4) : PC_REGS(8);
 #undef PC_REGS
     }
-    const int threads = E >= 2048 ? 256 : 128;
     return fg_launch(pair_combine_kernel, dim3(M), dim3(threads), 0, stream, a, b, w_a, w_b, scale_a, scale_b, eps, out, E, accumulate);
 }
 

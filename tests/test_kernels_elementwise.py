@@ -312,3 +312,28 @@ def test_conv1d_silu(lengths, taps):
         full = torch.cat([state[int(slots[s]), :taps - 1].double(), rows])
         pre = bias.double() + sum(full[j:j + len(rows)] * w[:, j].double() for j in range(taps))
         assert (out[int(cu[s]):int(cu[s + 1])].double() - torch.nn.functional.silu(pre)).abs().max() <= 4e-6 * pre.abs().max()
+
+
+@pytest.mark.parametrize("E", [24, 252, 256, 1024, 2048, 2052, 4092, 4096, 4100, 8192, 8196, 12288, 50, 700, 2050])
+def test_a_row_does_not_depend_on_the_other_rows_of_the_step(E):
+    """The kernels between contractions add a row's numbers in an order that the row's length decides: bit for bit the same in a step of one
+    row, of 64 and of 65."""
+    g = torch.Generator().manual_seed(E)
+    M = 65
+    t, x, o = (torch.randn(M, E, generator=g).cuda() for _ in range(3))
+    w, wn = (torch.randn(E, generator=g).cuda() for _ in range(2))
+
+    def norms(rows):
+        got, out = x[:rows].clone(), torch.empty(rows, E, dtype=torch.bfloat16, device="cuda")
+        _call("core", "fg_norm_add_norm_row", t[:rows], w, None, got, wn, out, 1, rows, E, 1e-6, 1e-5)
+        return got, out
+
+    def pair(rows):
+        out = o[:rows].clone()
+        _call("core", "fg_pair_combine", t[:rows], x[:rows], w, wn, 0.7, 0.6, 1e-6, out, rows, E, 1)
+        return (out,)
+
+    for f in (norms, pair):
+        for rows in (1, 64):
+            for few, many in zip(f(rows), f(M)):
+                assert torch.equal(few, many[:rows])
