@@ -390,8 +390,7 @@ latent_expand_kernel(const float *__restrict__ q, int ldq, const float *__restri
                      int tbl_half, const int *__restrict__ positions, const int *__restrict__ row_seq, const int *__restrict__ table,
                      int width, bf16 *__restrict__ qx, bf16 *__restrict__ Kx, bf16 *__restrict__ Vx, int H, int D, int DR, int DV,
                      int page_size, int key_rotated) {
-    __shared__ float krot[128];
-    pdl_launch_dependents_small_step(gridDim.x);
+    __shared__ float krot[128];            // (in front of a prompt's attention: the successor starts when this kernel has ended)
     pdl_wait();
     const int m = blockIdx.x, HQ = D + DR;
     const int pos = positions[m];
@@ -422,8 +421,8 @@ latent_expand_kernel(const float *__restrict__ q, int ldq, const float *__restri
 
 template <typename T>
 __global__ void gate_slice_kernel(const T *__restrict__ x, int ldx, int stride, const float *__restrict__ gate, int ldg, T *__restrict__ out,
-                                  int ldo, int H, int DV) {
-    pdl_launch_dependents_small_step(gridDim.x);
+                                  int ldo, int H, int DV, int early) {
+    if (early) pdl_launch_dependents();
     pdl_wait();
     const int m = blockIdx.x;
     for (int e = threadIdx.x; e < H * DV; e += blockDim.x) {
@@ -566,11 +565,16 @@ extern "C" int fg_latent_fetch(const void *k_pool, const void *v_pool, int dtype
     return FG_ERR_BAD_DTYPE;
 }
 
-extern "C" int fg_gate_slice(const void *x, int ldx, int stride, const float *gate, int ldg, void *out, int ldo, int dtype, int M, int H,
-                             int DV, cudaStream_t stream) {
+extern "C" int fg_gate_slice_step(const void *x, int ldx, int stride, const float *gate, int ldg, void *out, int ldo, int dtype, int M, int H,
+                                  int DV, int early, cudaStream_t stream) {
     if (M <= 0) return 0;
     if (H <= 0 || DV <= 0 || DV > stride) return FG_ERR_BAD_SIZE;
-    if (dtype == FG_F32) return fg_launch(gate_slice_kernel<float>, dim3(M), dim3(256), 0, stream, (const float *)x, ldx, stride, gate, ldg, (float *)out, ldo, H, DV);
-    if (dtype == FG_BF16) return fg_launch(gate_slice_kernel<bf16>, dim3(M), dim3(256), 0, stream, (const bf16 *)x, ldx, stride, gate, ldg, (bf16 *)out, ldo, H, DV);
+    if (dtype == FG_F32) return fg_launch(gate_slice_kernel<float>, dim3(M), dim3(256), 0, stream, (const float *)x, ldx, stride, gate, ldg, (float *)out, ldo, H, DV, early);
+    if (dtype == FG_BF16) return fg_launch(gate_slice_kernel<bf16>, dim3(M), dim3(256), 0, stream, (const bf16 *)x, ldx, stride, gate, ldg, (bf16 *)out, ldo, H, DV, early);
     return FG_ERR_BAD_DTYPE;
+}
+
+extern "C" int fg_gate_slice(const void *x, int ldx, int stride, const float *gate, int ldg, void *out, int ldo, int dtype, int M, int H,
+                             int DV, cudaStream_t stream) {
+    return fg_gate_slice_step(x, ldx, stride, gate, ldg, out, ldo, dtype, M, H, DV, 0, stream);
 }

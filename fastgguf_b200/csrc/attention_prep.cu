@@ -34,10 +34,10 @@ qkv_prepare_kernel(const float *__restrict__ proj, int ld, const float *__restri
                    const int *__restrict__ positions, const int *__restrict__ row_seq, const int *__restrict__ cu_rows,
                    const int *__restrict__ slots, const int *__restrict__ block_table, int table_width, T *__restrict__ q_out, int ldq,
                    T *__restrict__ k_pool, T *__restrict__ v_pool, int H, int KV, int VH, int hd, int hdv, int page_size, int norm_per_head,
-                   int rot_halves, int v_from_k) {
+                   int rot_halves, int v_from_k, int early) {
     extern __shared__ __align__(16) float row[];
     __shared__ float scratch[32];
-    pdl_launch_dependents_small_step(gridDim.x);
+    if (early) pdl_launch_dependents();
     pdl_wait();
     const int m = blockIdx.x, tid = threadIdx.x, nthr = blockDim.x;
     const int Cq = H * hd, Ck = KV * hd, C = Cq + Ck + (v_from_k ? 0 : VH * hdv);
@@ -418,12 +418,12 @@ head_gemv_kernel(const void *__restrict__ A, int a_dtype, int lda, int a_stride,
 // norm_per_head: the norm weights are [hd] and every head of q and of k is normalised by itself (else: [H * hd] / [KV * hd], the
 // whole of q and of k at once); rot_halves: a rotated pair is (i, i + rot_dims / 2) of a head (else (2i, 2i + 1)); v_heads (0: KV):
 // heads of values, where several key heads share one; v_from_k: there is no value projection, the values are the keys as projected
-extern "C" int fg_qkv_prepare_ext(const float *proj, int ld, const float *bias, const float *conv_w, int taps, const float *conv_state,
+extern "C" int fg_qkv_prepare_step(const float *proj, int ld, const float *bias, const float *conv_w, int taps, const float *conv_state,
                                   const float *qn_w, const float *kn_w, float eps, const float *cos_t, const float *sin_t, int tbl_half,
                                   int rot_dims, const int *positions, const int *row_seq, const int *cu_rows, const int *slots,
                                   const int *block_table, int table_width, void *q_out, int ldq, void *k_pool, void *v_pool, int dtype, int M,
                                   int H, int KV, int hd, int hdv, int page_size, int norm_per_head, int rot_halves, int v_heads, int v_from_k,
-                                  cudaStream_t stream) {
+                                  int early, cudaStream_t stream) {
     if (M <= 0) return 0;
     const int VH = v_heads > 0 ? v_heads : KV;
     if (v_from_k && (conv_w || VH != KV || hdv != hd)) return FG_ERR_BAD_SIZE;
@@ -445,7 +445,7 @@ extern "C" int fg_qkv_prepare_ext(const float *proj, int ld, const float *bias, 
         } \
         return fg_launch(qkv_prepare_kernel<T, VEC>, dim3(M), dim3(threads), smem, stream, proj, ld, bias, conv_w, taps, conv_state, qn_w, kn_w, \
                          eps, cos_t, sin_t, tbl_half, rot_dims, positions, row_seq, cu_rows, slots, block_table, table_width, (T *)q_out, \
-                         ldq, (T *)k_pool, (T *)v_pool, H, KV, VH, hd, hdv, page_size, norm_per_head, rot_halves, v_from_k); } while (0)
+                         ldq, (T *)k_pool, (T *)v_pool, H, KV, VH, hd, hdv, page_size, norm_per_head, rot_halves, v_from_k, early); } while (0)
     if (dtype == FG_F32) {
         if (vec) PREP_RUN(float, true);
         PREP_RUN(float, false);
@@ -456,6 +456,17 @@ extern "C" int fg_qkv_prepare_ext(const float *proj, int ld, const float *bias, 
     }
 #undef PREP_RUN
     return FG_ERR_BAD_DTYPE;
+}
+
+extern "C" int fg_qkv_prepare_ext(const float *proj, int ld, const float *bias, const float *conv_w, int taps, const float *conv_state,
+                                  const float *qn_w, const float *kn_w, float eps, const float *cos_t, const float *sin_t, int tbl_half,
+                                  int rot_dims, const int *positions, const int *row_seq, const int *cu_rows, const int *slots,
+                                  const int *block_table, int table_width, void *q_out, int ldq, void *k_pool, void *v_pool, int dtype, int M,
+                                  int H, int KV, int hd, int hdv, int page_size, int norm_per_head, int rot_halves, int v_heads, int v_from_k,
+                                  cudaStream_t stream) {
+    return fg_qkv_prepare_step(proj, ld, bias, conv_w, taps, conv_state, qn_w, kn_w, eps, cos_t, sin_t, tbl_half, rot_dims, positions, row_seq,
+                               cu_rows, slots, block_table, table_width, q_out, ldq, k_pool, v_pool, dtype, M, H, KV, hd, hdv, page_size,
+                               norm_per_head, rot_halves, v_heads, v_from_k, 0, stream);
 }
 
 extern "C" int fg_qkv_prepare(const float *proj, int ld, const float *bias, const float *conv_w, int taps, const float *conv_state,
@@ -473,8 +484,8 @@ extern "C" int fg_qkv_prepare(const float *proj, int ld, const float *bias, cons
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(PREP_THREADS)
 differential_combine_kernel(const float *__restrict__ maps, int ld, T *__restrict__ out, int ldo, int H, int R, int dv, float lambda, float eps,
-                            float gain) {
-    pdl_launch_dependents_small_step(gridDim.x);
+                            float gain, int early) {
+    if (early) pdl_launch_dependents();
     pdl_wait();
     const int m = blockIdx.x, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
     for (int h = blockIdx.y * n_warps + (threadIdx.x >> 5); h < H; h += gridDim.y * n_warps) {
@@ -508,18 +519,23 @@ differential_combine_kernel(const float *__restrict__ maps, int ld, T *__restric
     }
 }
 
-extern "C" int fg_differential_combine(const float *maps, int ld, void *out, int out_dtype, int ldo, int M, int H, int KV, int dv, float lambda,
-                                       float eps, float gain, cudaStream_t stream) {
+extern "C" int fg_differential_combine_step(const float *maps, int ld, void *out, int out_dtype, int ldo, int M, int H, int KV, int dv, float lambda,
+                                            float eps, float gain, int early, cudaStream_t stream) {
     if (M <= 0) return 0;
     if (H <= 0 || KV <= 0 || H % KV || dv <= 0) return FG_ERR_BAD_SIZE;
     const bool vec = dv % 4 == 0 && ld % 4 == 0 && ldo % 4 == 0 && ((((uintptr_t)maps) | ((uintptr_t)out)) & 15) == 0;
     const dim3 grid(M, (H + 7) / 8);
 #define DIFF_LAUNCH(T, VEC) fg_launch(differential_combine_kernel<T, VEC>, grid, dim3(PREP_THREADS), 0, stream, maps, ld, (T *)out, ldo, H, H / KV, dv, lambda, \
-                                      eps, gain)
+                                      eps, gain, early)
     if (out_dtype == FG_F32) return vec ? DIFF_LAUNCH(float, true) : DIFF_LAUNCH(float, false);
     if (out_dtype == FG_BF16) return vec ? DIFF_LAUNCH(bf16, true) : DIFF_LAUNCH(bf16, false);
 #undef DIFF_LAUNCH
     return FG_ERR_BAD_DTYPE;
+}
+
+extern "C" int fg_differential_combine(const float *maps, int ld, void *out, int out_dtype, int ldo, int M, int H, int KV, int dv, float lambda,
+                                       float eps, float gain, cudaStream_t stream) {
+    return fg_differential_combine_step(maps, ld, out, out_dtype, ldo, M, H, KV, dv, lambda, eps, gain, 0, stream);
 }
 
 // ------------------------------------------------------------------ a gate per head on the heads' outputs
@@ -527,9 +543,9 @@ extern "C" int fg_differential_combine(const float *maps, int ld, void *out, int
 // behind the heads are set to (1, 0, 0, ...): with the output projection's bias stored as column H * DV of its matrix, the
 // projection adds the bias in the same pass.
 template <typename T>
-__global__ void head_gate_kernel(T *__restrict__ x, int ldx, const float *__restrict__ gate, int ldg, int H, int DV, int pad, int vec) {
+__global__ void head_gate_kernel(T *__restrict__ x, int ldx, const float *__restrict__ gate, int ldg, int H, int DV, int pad, int vec, int early) {
     extern __shared__ float head_gate_sig[];        // the row's H gates
-    pdl_launch_dependents_small_step(gridDim.x);
+    if (early) pdl_launch_dependents();
     pdl_wait();
     const int m = blockIdx.x;
     T *row = x + (size_t)m * ldx;
@@ -554,16 +570,20 @@ __global__ void head_gate_kernel(T *__restrict__ x, int ldx, const float *__rest
     for (int e = threadIdx.x; e < pad; e += blockDim.x) row[H * DV + e] = from_f32<T>(e == 0 ? 1.0f : 0.0f);
 }
 
-extern "C" int fg_head_gate(void *x, int ldx, int dtype, const float *gate, int ldg, int M, int H, int DV, int pad, cudaStream_t stream) {
+extern "C" int fg_head_gate_step(void *x, int ldx, int dtype, const float *gate, int ldg, int M, int H, int DV, int pad, int early, cudaStream_t stream) {
     if (M <= 0 || (!gate && pad <= 0)) return 0;
     if (H * DV + pad > ldx || H > 8192) return FG_ERR_BAD_SIZE;
     const int threads = H * DV >= 4096 ? 256 : 128;
     const size_t smem = (size_t)H * sizeof(float);
     const int per = dtype == FG_F32 ? 4 : 8;
     const int vec = (DV % per == 0 && ldx % per == 0 && ((uintptr_t)x & 15) == 0) ? 1 : 0;
-    if (dtype == FG_F32) return fg_launch(head_gate_kernel<float>, dim3(M), dim3(threads), smem, stream, (float *)x, ldx, gate, ldg, H, DV, pad, vec);
-    if (dtype == FG_BF16) return fg_launch(head_gate_kernel<bf16>, dim3(M), dim3(threads), smem, stream, (bf16 *)x, ldx, gate, ldg, H, DV, pad, vec);
+    if (dtype == FG_F32) return fg_launch(head_gate_kernel<float>, dim3(M), dim3(threads), smem, stream, (float *)x, ldx, gate, ldg, H, DV, pad, vec, early);
+    if (dtype == FG_BF16) return fg_launch(head_gate_kernel<bf16>, dim3(M), dim3(threads), smem, stream, (bf16 *)x, ldx, gate, ldg, H, DV, pad, vec, early);
     return FG_ERR_BAD_DTYPE;
+}
+
+extern "C" int fg_head_gate(void *x, int ldx, int dtype, const float *gate, int ldg, int M, int H, int DV, int pad, cudaStream_t stream) {
+    return fg_head_gate_step(x, ldx, dtype, gate, ldg, M, H, DV, pad, 0, stream);
 }
 
 extern "C" int fg_conv_state_update(const float *proj, int ld, const float *bias, int taps, float *conv_state, const int *cu_rows,

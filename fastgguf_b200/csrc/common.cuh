@@ -119,6 +119,10 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // successor at its start and then sat resident, waiting, let the second contraction start beside the first, and now and then
 // a prompt step never finished (a hardware wait: every wait of these kernels' own is bounded).  There the successor is
 // released when the row-wise kernel ends.
+// Kernels that stand next to ATTENTION cannot go by the rows: a prompt of 16 tokens already runs the tensor-memory attention kernel
+// (64 rows of token x query head).  They, and others that such a step may run between two tensor-memory kernels, take `early`
+// from the host, which sets it at up to 64 rows of one token a sequence (attention without tensor memory) and in float32 engines
+// (whose tensor-memory contraction neither starts early nor releases its successor early).
 __device__ __forceinline__ void pdl_launch_dependents_small_step(unsigned rows) {
     if (rows <= 64) pdl_launch_dependents();
 }

@@ -730,9 +730,9 @@ extern "C" int fg_concat2(const float *a, int lda, const float *b, int ldb, void
 // over the row.  Statistics are 32-bit; one block a row, fixed reduction order.
 template <typename TO>
 __global__ void rmsnorm_pair_kernel(const float *__restrict__ x, const float *__restrict__ w_a, const float *__restrict__ w_b,
-                                    TO *__restrict__ out_a, TO *__restrict__ out_b, int E, float eps_a, float eps_b, int vec) {
+                                    TO *__restrict__ out_a, TO *__restrict__ out_b, int E, float eps_a, float eps_b, int vec, int early) {
     __shared__ float scratch[32];
-    pdl_launch_dependents_small_step(gridDim.x);
+    if (early) pdl_launch_dependents();
     pdl_wait();
     const float *xi = x + (size_t)blockIdx.x * E;
     TO *oa = out_a + (size_t)blockIdx.x * E, *ob = out_b + (size_t)blockIdx.x * E;
@@ -765,18 +765,23 @@ __global__ void rmsnorm_pair_kernel(const float *__restrict__ x, const float *__
     }
 }
 
-extern "C" int fg_rmsnorm_pair(const float *x, const float *w_a, const float *w_b, void *out_a, void *out_b, int out_dtype, int R, int E,
-                               float eps_a, float eps_b, cudaStream_t stream) {
+extern "C" int fg_rmsnorm_pair_step(const float *x, const float *w_a, const float *w_b, void *out_a, void *out_b, int out_dtype, int R, int E,
+                               float eps_a, float eps_b, int early, cudaStream_t stream) {
     if (R <= 0) return 0;
     const int threads = E >= 4096 ? 512 : (E >= 1024 ? 256 : (E >= 256 ? 128 : 64));
     const int vec = (E % 4 == 0 && ((((uintptr_t)x) | ((uintptr_t)w_a) | ((uintptr_t)w_b) | ((uintptr_t)out_a) | ((uintptr_t)out_b)) & 15) == 0) ? 1 : 0;
     if (out_dtype == FG_F32)
         return fg_launch(rmsnorm_pair_kernel<float>, dim3(R), dim3(threads), 0, stream, x, w_a, w_b, (float *)out_a, (float *)out_b, E, eps_a, eps_b,
-                         vec);
+                         vec, early);
     if (out_dtype == FG_BF16)
         return fg_launch(rmsnorm_pair_kernel<bf16>, dim3(R), dim3(threads), 0, stream, x, w_a, w_b, (bf16 *)out_a, (bf16 *)out_b, E, eps_a, eps_b,
-                         vec);
+                         vec, early);
     return FG_ERR_BAD_DTYPE;
+}
+
+extern "C" int fg_rmsnorm_pair(const float *x, const float *w_a, const float *w_b, void *out_a, void *out_b, int out_dtype, int R, int E,
+                               float eps_a, float eps_b, cudaStream_t stream) {
+    return fg_rmsnorm_pair_step(x, w_a, w_b, out_a, out_b, out_dtype, R, E, eps_a, eps_b, 0, stream);
 }
 
 // ------------------------------------------------------------------ the stream as a contraction's input

@@ -57,6 +57,9 @@ int fg_relu_mul(const void *gu, void *out, int dtype, int M, int F, cudaStream_t
 int fg_pair_combine(const float *a, const float *b, const float *w_a, const float *w_b, float scale_a, float scale_b, float eps,
                     float *out, int M, int E, int accumulate, cudaStream_t stream);
 /* out_a = x / rms(x) * w_a and out_b = x / rms(x) * w_b of the same float32 rows, one pass */
+/* the launchers ..._step: as the ones without the suffix, with `early` != 0 the kernel releases its successor at its start (common.cuh) */
+int fg_rmsnorm_pair_step(const float *x, const float *w_a, const float *w_b, void *out_a, void *out_b, int out_dtype, int R, int E,
+                         float eps_a, float eps_b, int early, cudaStream_t stream);
 int fg_rmsnorm_pair(const float *x, const float *w_a, const float *w_b, void *out_a, void *out_b, int out_dtype, int R, int E,
                     float eps_a, float eps_b, cudaStream_t stream);
 /* the float32 rows themselves in another dtype */
@@ -65,6 +68,8 @@ int fg_cast_rows(const float *x, int ldx, void *out, int out_dtype, int ldo, int
 int fg_gelu_mul_gather(const float *z, int ldz, const void *table, int table_dtype, int ldt, int col0, const int *tokens, void *out,
                        int out_dtype, int ldo, int M, int D, cudaStream_t stream);
 int fg_decode_advance(int *tokens, int *positions, const int *next_tokens, const int *active, int B, cudaStream_t stream);
+int fg_gemm_generic_step(const void *A, int a_dtype, int lda, const void *W, int w_dtype, int ldw, void *C, int out_dtype,
+                         int ldc, int accumulate, int M, int N, int K, int early, cudaStream_t stream);
 int fg_gemm_generic(const void *A, int a_dtype, int lda, const void *W, int w_dtype, int ldw, void *C, int out_dtype,
                     int ldc, int accumulate, int M, int N, int K, cudaStream_t stream);
 int fg_attention_generic(const void *q, int ldq, void *out, int ldo, int dtype, const int *positions,
@@ -179,11 +184,20 @@ int fg_qkv_prepare_ext(const float *proj, int ld, const float *bias, const float
                        const int *block_table, int table_width, void *q_out, int ldq, void *k_pool, void *v_pool, int dtype, int M,
                        int H, int KV, int hd, int hdv, int page_size, int norm_per_head, int rot_halves, int v_heads, int v_from_k,
                        cudaStream_t stream);
+int fg_qkv_prepare_step(const float *proj, int ld, const float *bias, const float *conv_w, int taps, const float *conv_state,
+                        const float *qn_w, const float *kn_w, float eps, const float *cos_t, const float *sin_t, int tbl_half,
+                        int rot_dims, const int *positions, const int *row_seq, const int *cu_rows, const int *slots,
+                        const int *block_table, int table_width, void *q_out, int ldq, void *k_pool, void *v_pool, int dtype, int M,
+                        int H, int KV, int hd, int hdv, int page_size, int norm_per_head, int rot_halves, int v_heads, int v_from_k,
+                        int early, cudaStream_t stream);
 /* out = (a1 - lambda a2) / rms * gain per head, maps rows [key head][map][head of the group][dv] float32 */
 int fg_differential_combine(const float *maps, int ld, void *out, int out_dtype, int ldo, int M, int H, int KV, int dv, float lambda, float eps,
                             float gain, cudaStream_t stream);
+int fg_differential_combine_step(const float *maps, int ld, void *out, int out_dtype, int ldo, int M, int H, int KV, int dv, float lambda,
+                                 float eps, float gain, int early, cudaStream_t stream);
 /* x[m, h * DV + j] *= sigmoid(gate[m, h]) in place (gate null: none); `pad` columns behind the heads become (1, 0, 0, ...) */
 int fg_head_gate(void *x, int ldx, int dtype, const float *gate, int ldg, int M, int H, int DV, int pad, cudaStream_t stream);
+int fg_head_gate_step(void *x, int ldx, int dtype, const float *gate, int ldg, int M, int H, int DV, int pad, int early, cudaStream_t stream);
 int fg_conv_state_update(const float *proj, int ld, const float *bias, int taps, float *conv_state, const int *cu_rows,
                          const int *slots, int n_seq, int C, cudaStream_t stream);
 int fg_latent_append(const float *kv, int ld, const float *norm_w, float eps, const float *cos_t, const float *sin_t, int tbl_half,
@@ -220,6 +234,8 @@ int fg_latent_fetch(const void *k_pool, const void *v_pool, int dtype, const int
                     int width, int page_size, void *c_out, int ldc, float *kr_out, int ldk, int M, int R, int DR, cudaStream_t stream);
 int fg_gate_slice(const void *x, int ldx, int stride, const float *gate, int ldg, void *out, int ldo, int dtype, int M, int H,
                   int DV, cudaStream_t stream);
+int fg_gate_slice_step(const void *x, int ldx, int stride, const float *gate, int ldg, void *out, int ldo, int dtype, int M, int H,
+                       int DV, int early, cudaStream_t stream);
 int fg_moe_logits(const void *x, int ldx, const void *W, int ldw, int dtype, float *z, int M, int X, int E, cudaStream_t stream);
 int fg_moe_gather(const void *x, int ldx, int dtype, const int *order, int top, void *xs, int P, int E, cudaStream_t stream);
 int fg_moe_act(const float *gu, const int *order, const float *pair_weight, void *y, int dtype, int P, int F, float limit,

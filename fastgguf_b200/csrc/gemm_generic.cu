@@ -18,10 +18,10 @@
 template <typename TA, typename TW>
 __global__ void __launch_bounds__(256)
 gemm_generic_kernel(const TA *__restrict__ A, int lda, const TW *__restrict__ W, int ldw,
-                    void *__restrict__ C, int ldc, int out_dtype, int accumulate, int M, int N, int K) {
+                    void *__restrict__ C, int ldc, int out_dtype, int accumulate, int M, int N, int K, int early) {
     __shared__ float As[TK][TM + 1];
     __shared__ float Ws[TK][TN + 1];
-    pdl_launch_dependents();               // (up to 64 rows: a small step)
+    if (early) pdl_launch_dependents();
     pdl_wait();
     int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // tx: n direction, ty: m direction
     int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
@@ -165,10 +165,10 @@ gemm_tile128_kernel(const TA *__restrict__ A, int lda, const TW *__restrict__ W,
 template <int MB, int RPW, int U, typename TA, typename TW>
 __global__ void __launch_bounds__(GEMV_WARPS * 32)
 gemv_rows_kernel(const TA *__restrict__ A, int lda, const TW *__restrict__ W, int ldw, void *__restrict__ C, int ldc,
-                 int out_dtype, int accumulate, int M, int N, int K) {
+                 int out_dtype, int accumulate, int M, int N, int K, int early) {
     constexpr int KC = MB <= 4 ? 2048 : MB == 8 ? 1024 : 512;       // 32 KB of activations at a time
     __shared__ __align__(16) float As[MB][KC];
-    pdl_launch_dependents();
+    if (early) pdl_launch_dependents();
     pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n0 = (blockIdx.x * GEMV_WARPS + warp) * RPW;
@@ -236,9 +236,9 @@ gemv_rows_kernel(const TA *__restrict__ A, int lda, const TW *__restrict__ W, in
 template <int MB, int R, typename TA, typename TW>
 __global__ void __launch_bounds__(GEMV_WARPS * 32)
 gemv_splitk_kernel(const TA *__restrict__ A, int lda, const TW *__restrict__ W, int ldw, void *__restrict__ C, int ldc,
-                   int out_dtype, int accumulate, int M, int N, int K) {
+                   int out_dtype, int accumulate, int M, int N, int K, int early) {
     __shared__ float part[GEMV_WARPS][R][MB];
-    pdl_launch_dependents();
+    if (early) pdl_launch_dependents();
     pdl_wait();
     const int m0 = blockIdx.y * MB;
     A += (size_t)m0 * lda;
@@ -296,7 +296,7 @@ gemv_splitk_kernel(const TA *__restrict__ A, int lda, const TW *__restrict__ W, 
 
 template <typename TA, typename TW>
 static int launch_gemv(const void *A, int lda, const void *W, int ldw, void *C, int ldc, int out_dtype, int accumulate, int M,
-                        int N, int K, cudaStream_t stream) {
+                       int N, int K, int early, cudaStream_t stream) {
     const bool many = N >= 16384;         // enough weight rows for four a warp to fill the GPU
     const int a_bytes = sizeof(TA);
     // the block-split kernel reads the activations with vector loads too
@@ -305,7 +305,7 @@ static int launch_gemv(const void *A, int lda, const void *W, int ldw, void *C, 
     if (M > 16 && !split) return FG_ERR_BAD_SIZE;         // (blocks of rows: the block-split kernel alone)
     dim3 grid((N + rows_per_block - 1) / rows_per_block, (M + 15) / 16), block(GEMV_WARPS * 32);
     int e = 0;
-#define GEMV_ARGS (const TA *)A, lda, (const TW *)W, ldw, C, ldc, out_dtype, accumulate, M, N, K
+#define GEMV_ARGS (const TA *)A, lda, (const TW *)W, ldw, C, ldc, out_dtype, accumulate, M, N, K, early
 #define GEMV(MB) do { \
         if (many) e = fg_launch(gemv_rows_kernel<MB, 4, 2, TA, TW>, grid, block, 0, stream, GEMV_ARGS); \
         else if (split) e = fg_launch(gemv_splitk_kernel<MB, (MB <= 8 ? 4 : 2), TA, TW>, grid, block, 0, stream, GEMV_ARGS); \
@@ -321,9 +321,10 @@ static int launch_gemv(const void *A, int lda, const void *W, int ldw, void *C, 
 }
 
 // a_dtype / w_dtype / out_dtype: FG_F32 or FG_BF16.  accumulate=1 needs out_dtype == FG_F32.
-extern "C" int fg_gemm_generic(const void *A, int a_dtype, int lda, const void *W, int w_dtype, int ldw,
-                               void *C, int out_dtype, int ldc, int accumulate, int M, int N, int K,
-                               cudaStream_t stream) {
+// early: the kernels for up to 64 rows release their successor at their start (see common.cuh).
+extern "C" int fg_gemm_generic_step(const void *A, int a_dtype, int lda, const void *W, int w_dtype, int ldw,
+                                    void *C, int out_dtype, int ldc, int accumulate, int M, int N, int K, int early,
+                                    cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (accumulate && out_dtype != FG_F32) return FG_ERR_BAD_DTYPE;
     // few rows and weight rows that 16-byte (f32) / 8-byte (bf16) loads can walk: the weight-streaming kernel
@@ -332,10 +333,10 @@ extern "C" int fg_gemm_generic(const void *A, int a_dtype, int lda, const void *
     // walk along K waits for every load (39 rows x 64 x 192: 23 us, 16 rows a block 4.2).
     if ((M <= 16 || (M <= 64 && (long long)N * K <= 1 << 18)) && K % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)W % (4 * w_bytes)) == 0) {
         int e = FG_ERR_BAD_DTYPE;
-        if (a_dtype == FG_F32 && w_dtype == FG_F32) e = launch_gemv<float, float>(A, lda, W, ldw, C, ldc, out_dtype, accumulate, M, N, K, stream);
-        else if (a_dtype == FG_BF16 && w_dtype == FG_BF16) e = launch_gemv<bf16, bf16>(A, lda, W, ldw, C, ldc, out_dtype, accumulate, M, N, K, stream);
-        else if (a_dtype == FG_BF16 && w_dtype == FG_F32) e = launch_gemv<bf16, float>(A, lda, W, ldw, C, ldc, out_dtype, accumulate, M, N, K, stream);
-        else if (a_dtype == FG_F32 && w_dtype == FG_BF16) e = launch_gemv<float, bf16>(A, lda, W, ldw, C, ldc, out_dtype, accumulate, M, N, K, stream);
+        if (a_dtype == FG_F32 && w_dtype == FG_F32) e = launch_gemv<float, float>(A, lda, W, ldw, C, ldc, out_dtype, accumulate, M, N, K, early, stream);
+        else if (a_dtype == FG_BF16 && w_dtype == FG_BF16) e = launch_gemv<bf16, bf16>(A, lda, W, ldw, C, ldc, out_dtype, accumulate, M, N, K, early, stream);
+        else if (a_dtype == FG_BF16 && w_dtype == FG_F32) e = launch_gemv<bf16, float>(A, lda, W, ldw, C, ldc, out_dtype, accumulate, M, N, K, early, stream);
+        else if (a_dtype == FG_F32 && w_dtype == FG_BF16) e = launch_gemv<float, bf16>(A, lda, W, ldw, C, ldc, out_dtype, accumulate, M, N, K, early, stream);
         if (e != FG_ERR_BAD_SIZE) return e;
     }
     if (M > 64) {
@@ -359,7 +360,7 @@ extern "C" int fg_gemm_generic(const void *A, int a_dtype, int lda, const void *
     if (grid.y > 65535) return FG_ERR_BAD_SIZE;
     int e = 0;
 #define LAUNCH(TA, TW) e = fg_launch(gemm_generic_kernel<TA, TW>, grid, dim3(256), 0, stream, \
-        (const TA *)A, lda, (const TW *)W, ldw, C, ldc, out_dtype, accumulate, M, N, K)
+        (const TA *)A, lda, (const TW *)W, ldw, C, ldc, out_dtype, accumulate, M, N, K, early)
     if (a_dtype == FG_F32 && w_dtype == FG_F32) LAUNCH(float, float);
     else if (a_dtype == FG_BF16 && w_dtype == FG_BF16) LAUNCH(bf16, bf16);
     else if (a_dtype == FG_BF16 && w_dtype == FG_F32) LAUNCH(bf16, float);
@@ -367,4 +368,9 @@ extern "C" int fg_gemm_generic(const void *A, int a_dtype, int lda, const void *
     else return FG_ERR_BAD_DTYPE;
 #undef LAUNCH
     return e;
+}
+
+extern "C" int fg_gemm_generic(const void *A, int a_dtype, int lda, const void *W, int w_dtype, int ldw, void *C, int out_dtype, int ldc,
+                               int accumulate, int M, int N, int K, cudaStream_t stream) {
+    return fg_gemm_generic_step(A, a_dtype, lda, W, w_dtype, ldw, C, out_dtype, ldc, accumulate, M, N, K, 0, stream);
 }

@@ -36,6 +36,13 @@ void count_launch();
         ::fg::ProfileScope fg_profile_scope_(#fn);                                                           \
         ::fg::check_kernel(FG_KERNEL(module, fn)(__VA_ARGS__), #fn);                                         \
     } while (0)
+// the launcher <fn>_step, counted and profiled as <fn>
+#define FG_LAUNCH_STEP(module, fn, ...)                                                                      \
+    do {                                                                                                     \
+        ::fg::count_launch();                                                                                \
+        ::fg::ProfileScope fg_profile_scope_(#fn);                                                           \
+        ::fg::check_kernel(FG_KERNEL(module, fn##_step)(__VA_ARGS__), #fn);                                  \
+    } while (0)
 // Per-launcher device times, for `--profile`: while it is on, every launcher call is bracketed by two events on
 // `stream` (which also ends the overlap of dependent launches: the times are those of kernels running one after
 // another) and decode steps run eagerly, since events inside a recorded graph cannot be read.  One engine at a time.

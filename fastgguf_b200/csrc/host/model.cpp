@@ -473,6 +473,7 @@ Tensor DecoderModel::step(const std::vector<StepEntry> &entries) {
 }
 
 Tensor DecoderModel::forward(Runtime &rt, const Batch &batch) {
+    rt.single_token = batch.single_token;
     const bool bf16 = rt.dtype == FG_BF16;
     const size_t n = spec.schedule.size();
     auto block_at = [&](size_t i) { return blocks_[(size_t)spec.schedule[i].layer].get(); };
@@ -567,6 +568,7 @@ void DecoderModel::block_forward(int entry, const std::vector<std::pair<int, int
     size_t bytes = (size_t)M * (size_t)spec.hidden_size * 4;
     FG_CUDA(cudaMemcpyAsync(x.data, x_host, bytes, cudaMemcpyHostToDevice, runtime.stream));
     Block *blk = blocks_[(size_t)spec.schedule[(size_t)entry].layer].get();
+    runtime.single_token = batch.single_token;
     blk->forward(runtime, x, batch, io[(size_t)entry], DeferredNorm(), nullptr);
     if (blk->token_input) blk->token_input->forward(runtime, batch, x, DeferredNorm(), nullptr, nullptr);
     FG_CUDA(cudaMemcpyAsync(x_host, x.data, bytes, cudaMemcpyDeviceToHost, runtime.stream));

@@ -200,8 +200,8 @@ Tensor Linear::forward(Runtime &rt, const Tensor &a_in, const DeferredNorm *defe
             }
         }
     }
-    FG_LAUNCH("core", fg_gemm_generic, a.data, a.dtype, (int)a.ld, W.data, W.dtype, (int)W.ld, out.data, out.dtype, (int)out.ld,
-              accumulate ? 1 : 0, (int)M, (int)N, (int)K, rt.stream);
+    FG_LAUNCH_STEP("core", fg_gemm_generic, a.data, a.dtype, (int)a.ld, W.data, W.dtype, (int)W.ld, out.data, out.dtype, (int)out.ld,
+                   accumulate ? 1 : 0, (int)M, (int)N, (int)K, rt.early(M), rt.stream);
     return out;
 }
 
@@ -977,8 +977,8 @@ private:
             xa = rt.arena->matrix(M, E, rt.dtype);
             xb = rt.arena->matrix(M, E, rt.dtype);
             if (M > 0)
-                FG_LAUNCH("core", fg_rmsnorm_pair, x.ptr<float>(), mixer_norm->weight(), feed_forward_norm->weight(), xa.data, xb.data, rt.dtype, M, E,
-                          mixer_norm->eps(), feed_forward_norm->eps(), rt.stream);
+                FG_LAUNCH_STEP("core", fg_rmsnorm_pair, x.ptr<float>(), mixer_norm->weight(), feed_forward_norm->weight(), xa.data, xb.data, rt.dtype, M, E,
+                               mixer_norm->eps(), feed_forward_norm->eps(), rt.early(M), rt.stream);
         } else {
             xa = mixer_norm->forward(rt, x, nullptr, 0);
             xb = feed_forward_norm->forward(rt, x, nullptr, 0);

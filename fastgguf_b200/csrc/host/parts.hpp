@@ -29,6 +29,10 @@ struct Runtime {
     Arena *arena = nullptr;           // activations of the step being run
     bool recording = false;           // the step is being recorded into a CUDA graph
     bool plain_kernels = false;       // the safety switch: the any-size FMA kernels everywhere, bfloat16 included
+    // The step brings one token a sequence: no attention kernel that holds tensor memory runs in it.
+    bool single_token = false;
+    // what the launchers ..._step take: whether kernels beside attention may release their successor at their start (common.cuh)
+    int early(int64_t rows) const { return rows <= 64 && (single_token || dtype == FG_F32); }
     // Set by a block around ONE call of a mixer or feed-forward whose can_overwrite() is true: the `residual` handed over
     // holds nothing yet, and the part writes its output there instead of adding it (no zeroing pass in front).
     bool overwrite = false;

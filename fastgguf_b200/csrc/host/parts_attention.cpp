@@ -204,11 +204,11 @@ public:
         const int HQ = maps_ * H_, HK = maps_ * KV_;         // heads the kernels see
         Tensor q = rt.arena->matrix(M, (int64_t)HQ * hd_, rt.dtype);
         const float *bias = bias_ ? bias_w_.t.ptr<float>() : nullptr;
-        FG_LAUNCH("mix", fg_qkv_prepare_ext, proj.ptr<float>(), (int)proj.ld, bias, taps_ > 0 ? conv_w_.t.ptr<float>() : nullptr, taps_,
+        FG_LAUNCH_STEP("mix", fg_qkv_prepare, proj.ptr<float>(), (int)proj.ld, bias, taps_ > 0 ? conv_w_.t.ptr<float>() : nullptr, taps_,
                   (const float *)io.state, qk_norm_ ? qn_w_.t.ptr<float>() : nullptr, qk_norm_ ? kn_w_.t.ptr<float>() : nullptr, eps_,
                   position_ ? position_->cos_table() : nullptr, position_ ? position_->sin_table() : nullptr, hd_ / 2, position_ ? rot_dims_ : 0,
                   b.positions, b.row_seq, b.cu_rows, b.slots, table, b.table_width, q.data, (int)q.ld, io.k_pool, io.v_pool, rt.dtype, M, HQ, HK,
-                  hd_, hdv_, io.page_size, norm_per_head_ ? 1 : 0, rot_halves_ ? 1 : 0, KV_, v_from_k_ ? 1 : 0, rt.stream);
+                  hd_, hdv_, io.page_size, norm_per_head_ ? 1 : 0, rot_halves_ ? 1 : 0, KV_, v_from_k_ ? 1 : 0, rt.early(M), rt.stream);
         if (taps_ > 1)
             FG_LAUNCH("mix", fg_conv_state_update, proj.ptr<float>(), (int)proj.ld, bias, taps_, (float *)io.state, b.cu_rows, b.slots, b.n_seq,
                       (int)channels(), rt.stream);
@@ -245,14 +245,14 @@ public:
                       b.table_width, io.k_pool, io.v_pool, M, HQ, HK, hd_, hdv_, io.page_size, scale_, mask, 0, softcap_, sinks, 0, maps_, f32_out, rt.stream);
         }
         if (differential_)
-            FG_LAUNCH("mix", fg_differential_combine, each.ptr<float>(), (int)each.ld, attn.data, attn.dtype, (int)attn.ld, M, H_, KV_, hdv_, lambda_, eps_,
-                      1.0f - diff_, rt.stream);
+            FG_LAUNCH_STEP("mix", fg_differential_combine, each.ptr<float>(), (int)each.ld, attn.data, attn.dtype, (int)attn.ld, M, H_, KV_, hdv_, lambda_, eps_,
+                           1.0f - diff_, rt.early(M), rt.stream);
         if (gate_full_)           // in place: a thread reads and writes its own number
-            FG_LAUNCH("mix", fg_gate_slice, attn.data, (int)attn.ld, hdv_, proj.ptr<float>() + channels(), (int)proj.ld, attn.data, (int)attn.ld, attn.dtype, M,
-                      H_, hdv_, rt.stream);
+            FG_LAUNCH_STEP("mix", fg_gate_slice, attn.data, (int)attn.ld, hdv_, proj.ptr<float>() + channels(), (int)proj.ld, attn.data, (int)attn.ld, attn.dtype, M,
+                           H_, hdv_, rt.early(M), rt.stream);
         if ((gate_ && !gate_full_) || pad_ > 0)
-            FG_LAUNCH("mix", fg_head_gate, attn.data, (int)attn.ld, attn.dtype, (gate_ && !gate_full_) ? proj.ptr<float>() + channels() : nullptr, (int)proj.ld,
-                      M, H_, hdv_, pad_, rt.stream);
+            FG_LAUNCH_STEP("mix", fg_head_gate, attn.data, (int)attn.ld, attn.dtype, (gate_ && !gate_full_) ? proj.ptr<float>() + channels() : nullptr, (int)proj.ld,
+                           M, H_, hdv_, pad_, rt.early(M), rt.stream);
         DeferredNorm started;
         o_.forward(rt, attn, nullptr, residual, FG_F32, !rt.overwrite, emit_norm, &started);
         return started;
@@ -404,7 +404,7 @@ public:
             else
                 FG_LAUNCH("attn", fg_attention_prefill_ext, qx.data, (int)qx.ld, ox.data, (int)ox.ld, b.cu_rows, b.seq_start, tmp_table, width, Kx, Vx,
                           b.n_seq, b.max_new, H_, H_, HQ, P, scale_, 0, 0, 0.f, sinks, HQ, 1, 0, rt.stream);
-            FG_LAUNCH("mix", fg_gate_slice, ox.data, (int)ox.ld, HQ, gate, (int)down.ld, o.data, (int)o.ld, o.dtype, M, H_, dv_, rt.stream);
+            FG_LAUNCH_STEP("mix", fg_gate_slice, ox.data, (int)ox.ld, HQ, gate, (int)down.ld, o.data, (int)o.ld, o.dtype, M, H_, dv_, rt.early(M), rt.stream);
         } else {
             // per head [q_abs (kv_rank) | q_rot (rot_dim)]
             Tensor qf = rt.arena->matrix(M, (int64_t)H_ * (r_ + dr_), rt.dtype);

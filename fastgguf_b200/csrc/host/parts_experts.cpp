@@ -168,8 +168,8 @@ private:
         if (R.dtype == xn.dtype)
             FG_LAUNCH("mix", fg_moe_logits, xn.data, (int)xn.ld, R.data, (int)R.ld, xn.dtype, z.ptr<float>(), M, XR, E_, rt.stream);
         else
-            FG_LAUNCH("core", fg_gemm_generic, xn.data, xn.dtype, (int)xn.ld, R.data, R.dtype, (int)R.ld, z.data, FG_F32, (int)z.ld, 0, M, XR,
-                      E_, rt.stream);
+            FG_LAUNCH_STEP("core", fg_gemm_generic, xn.data, xn.dtype, (int)xn.ld, R.data, R.dtype, (int)R.ld, z.data, FG_F32, (int)z.ld, 0, M, XR,
+                           E_, rt.early(M), rt.stream);
         int *ints = (int *)rt.arena->alloc(((size_t)3 * P + XR + 1) * sizeof(int));
         int *pair_expert = ints, *order = ints + P, *slot_of = ints + 2 * P, *offsets = ints + 3 * P;
         float *pair_weight = (float *)rt.arena->alloc((size_t)P * sizeof(float));
