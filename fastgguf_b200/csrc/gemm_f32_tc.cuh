@@ -21,7 +21,8 @@
 // against 1,249; 24 x 2,048 x 2,048: 38 against 210.
 //
 // Numbers that the split does not carry (infinities, NaN, magnitudes whose first plane or whose partial sums overflow) leave a sum
-// that is no finite number; such an output is computed again by the plain chain of fused multiply-adds over the float32 operands.
+// that is no finite number; such an output is computed again by the plain chain of fused multiply-adds over the float32 operands, a warp
+// for 32 x 32 outputs.
 #pragma once
 
 #define F32_EPI_WARPS 8
@@ -37,12 +38,76 @@ struct F32Args {
     int accumulate, vec_ok;
 };
 
-__device__ __noinline__ float f32_plain_dot(const float *a, const float *w, int K) {
-    float s = 0.f;
-    for (int k = 0; k < K; k++) s = fmaf(a[k], w[k], s);
-    return s;
-}
 __device__ __forceinline__ bool f32_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
+// zero where all four are finite numbers (and `sum` was), NaN where one is not
+__device__ __forceinline__ float f32_check4(float4 t, float sum) { return fmaf(t.x, 0.f, fmaf(t.y, 0.f, fmaf(t.z, 0.f, fmaf(t.w, 0.f, sum)))); }
+
+// 32 x 32 outputs by the plain chain into a warp's tile T (row r, columns swizzled as the epilogue has them).  16 k of 32 rows of both
+// operands at a time lie in T, the next ones are on their way meanwhile; a lane adds up 4 x 8 outputs, each in rising k.  With
+// 2,048 rows x 16,384 x 2,048 of NaN the contraction takes 5.9 ms (3.2 on the FMA-unit tiles; a lane an output 92), with one such row 2.1 (4.0).
+__device__ __forceinline__ void f32_plain_tile(float *T, const F32Args &a, int m0, int n0) {
+    const int lane = threadIdx.x & 31, rg = lane >> 2, cg = lane & 3;          // a lane fetches four numbers of rows rg, rg + 8, ..
+    const float *pa[4], *pw[4];
+    float4 fa[4], fw[4];
+    float acc[4][8];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        pa[i] = a.A + (size_t)min(m0 + i * 8 + rg, a.M - 1) * a.lda + cg * 4;
+        pw[i] = a.W + (size_t)min(n0 + i * 8 + rg, a.N - 1) * a.ldw + cg * 4;
+#pragma unroll
+        for (int j = 0; j < 8; j++) acc[i][j] = 0.f;
+    }
+    auto fetch = [&](int k0) {                             // (K % 8 == 0, rows 16-byte aligned)
+        const bool in = k0 + cg * 4 < a.K;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            fa[i] = in ? *(const float4 *)(pa[i] + k0) : make_float4(0.f, 0.f, 0.f, 0.f);
+            fw[i] = in ? *(const float4 *)(pw[i] + k0) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    // vector q of row r: at r * 4 + (q ^ (r / 4 % 4)) for A, r / 8 for W, so that the rows read together lie in different banks
+    float4 *TA = (float4 *)T, *TW = TA + 128;
+    fetch(0);
+    for (int k0 = 0; k0 < a.K; k0 += 16) {
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int r = i * 8 + rg;
+            TA[r * 4 + (cg ^ ((r >> 2) & 3))] = fa[i];
+            TW[r * 4 + (cg ^ ((r >> 3) & 3))] = fw[i];
+        }
+        __syncwarp();
+        if (k0 + 16 < a.K) fetch(k0 + 16);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            float4 x[4], y[8];
+#pragma unroll
+            for (int i = 0; i < 4; i++) x[i] = TA[(rg * 4 + i) * 4 + (q ^ (rg & 3))];
+#pragma unroll
+            for (int j = 0; j < 8; j++) y[j] = TW[(cg * 8 + j) * 4 + (q ^ cg)];
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    float v = acc[i][j];
+                    v = fmaf(x[i].x, y[j].x, v);
+                    v = fmaf(x[i].y, y[j].y, v);
+                    v = fmaf(x[i].z, y[j].z, v);
+                    v = fmaf(x[i].w, y[j].w, v);
+                    acc[i][j] = v;
+                }
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const int r = rg * 4 + i, c = cg * 8 + j;
+            T[r * 32 + (((c >> 2) ^ (r & 7)) << 2) + (c & 3)] = acc[i][j];
+        }
+    __syncwarp();
+}
 
 // planes[p][row][k], p = 0 (hi), 1 (mid), 2 (lo).  Bound by memory: 4 bytes in, 6 out.  A thread takes eight numbers.
 __global__ void __launch_bounds__(256)
@@ -208,29 +273,35 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_const
             // 32 columns at a time through a tile in shared memory, so that a warp stores whole 128-byte lines
             const bool part = a.splits > 1;
             float *out = part ? a.out + (size_t)z * a.M * a.N : a.out;
-            const int ldc = part ? a.N : a.ldc;
+            const int ldc = part ? a.N : a.ldc, ch = lane & 7;
+            uint32_t plain[NC / 32], any_plain = 0;                // outputs of this lane's row that the plain chain has to give
 #pragma unroll
             for (int c = 0; c < NC / 32; c++) {
+                plain[c] = 0;
+                float check = 0.f;
 #pragma unroll
-                for (int ch = 0; ch < 8; ch++)
-                    *(float4 *)(T + lane * 32 + ((ch ^ (lane & 7)) << 2)) =
-                        make_float4(sum[c * 32 + 4 * ch], sum[c * 32 + 4 * ch + 1], sum[c * 32 + 4 * ch + 2], sum[c * 32 + 4 * ch + 3]);
+                for (int q = 0; q < 8; q++) {
+                    const float4 t = make_float4(sum[c * 32 + 4 * q], sum[c * 32 + 4 * q + 1], sum[c * 32 + 4 * q + 2], sum[c * 32 + 4 * q + 3]);
+                    check = f32_check4(t, check);
+                    *(float4 *)(T + lane * 32 + ((q ^ (lane & 7)) << 2)) = t;
+                }
+                const bool some = !part && __any_sync(0xffffffffu, check != 0.f);
+                if (some && m_base + lane < a.M) {
+#pragma unroll 1
+                    for (int j = 0; j < 32; j++)
+                        if (!f32_finite(T[lane * 32 + (((j >> 2) ^ (lane & 7)) << 2) + (j & 3)])) plain[c] |= 1u << j;
+                }
+                any_plain |= some;
                 __syncwarp();
-                const int ch = lane & 7, n = n_base + c * 32 + ch * 4;
+                const int n = n_base + c * 32 + ch * 4;
 #pragma unroll 2
                 for (int pass = 0; pass < 8; pass++) {
                     const int row = pass * 4 + (lane >> 3), m = m_base + row;
+                    const uint32_t later = some ? (__shfl_sync(0xffffffffu, plain[c], row) >> (4 * ch)) & 15 : 0;
                     if (m >= a.M || n >= a.N) continue;
                     float4 t = *(const float4 *)(T + row * 32 + ((ch ^ (row & 7)) << 2));
                     float *dst = out + (size_t)m * ldc + n;
-                    if (!part && !(f32_finite(t.x) && f32_finite(t.y) && f32_finite(t.z) && f32_finite(t.w))) {
-                        const float *ar = a.A + (size_t)m * a.lda, *wr = a.W + (size_t)n * a.ldw;
-                        if (!f32_finite(t.x)) t.x = f32_plain_dot(ar, wr, a.K);
-                        if (!f32_finite(t.y) && n + 1 < a.N) t.y = f32_plain_dot(ar, wr + (size_t)a.ldw, a.K);
-                        if (!f32_finite(t.z) && n + 2 < a.N) t.z = f32_plain_dot(ar, wr + 2 * (size_t)a.ldw, a.K);
-                        if (!f32_finite(t.w) && n + 3 < a.N) t.w = f32_plain_dot(ar, wr + 3 * (size_t)a.ldw, a.K);
-                    }
-                    if (a.vec_ok && n + 3 < a.N) {
+                    if (a.vec_ok && n + 3 < a.N && !later) {
                         if (a.accumulate && !part) {
                             const float4 r = __ldcg((const float4 *)dst);
                             t.x += r.x; t.y += r.y; t.z += r.z; t.w += r.w;
@@ -240,8 +311,28 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_const
                         const float tv[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
                         for (int j = 0; j < 4; j++)
-                            if (n + j < a.N) dst[j] = tv[j] + (a.accumulate && !part ? dst[j] : 0.f);
+                            if (n + j < a.N && !(later >> j & 1)) dst[j] = tv[j] + (a.accumulate && !part ? dst[j] : 0.f);
                     }
+                }
+                __syncwarp();
+            }
+            if (!any_plain) continue;
+#pragma unroll 1
+            for (int c = 0; c < NC / 32; c++) {                    // (here, where the sums are no longer needed, it costs the kernel no registers)
+                uint32_t bits = plain[0];
+#pragma unroll
+                for (int i = 1; i < NC / 32; i++) bits = c == i ? plain[i] : bits;
+                if (!__any_sync(0xffffffffu, bits != 0)) continue;
+                f32_plain_tile(T, a, m_base, n_base + c * 32);
+                const int n = n_base + c * 32 + ch * 4;
+                for (int pass = 0; pass < 8; pass++) {
+                    const int row = pass * 4 + (lane >> 3), m = m_base + row;
+                    const uint32_t mine = (__shfl_sync(0xffffffffu, bits, row) >> (4 * ch)) & 15;
+                    for (int j = 0; j < 4; j++)
+                        if ((mine >> j & 1) && m < a.M && n + j < a.N) {
+                            float *dst = out + (size_t)m * ldc + n + j;
+                            *dst = T[row * 32 + ((ch ^ (row & 7)) << 2) + j] + (a.accumulate ? *dst : 0.f);
+                        }
                 }
                 __syncwarp();
             }
@@ -257,29 +348,55 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_const
     }
 }
 
-// out[m, n] (+)= the sum of the parts [splits][M][N], in split order; four columns a thread (N % 4 == 0 where splits are taken)
-__global__ void __launch_bounds__(256)
+// out[m, n] (+)= the sum of the parts [splits][M][N], in split order.  A block takes 32 x 32 outputs, a thread four columns of a row
+// (N % 4 == 0 where splits are taken).
+__global__ void __launch_bounds__(256, 4)
 gemm_f32_finish_kernel(F32Args a, const float *__restrict__ parts) {
-    const long long i = (long long)blockIdx.x * 256 + threadIdx.x, per_row = a.N / 4;
-    if (i >= a.M * per_row) return;
-    const int m = (int)(i / per_row), n = (int)(i % per_row) * 4;
+    __shared__ float4 TA[32 * 4], TW[32 * 4];
+    const int row = threadIdx.x >> 3, ch = threadIdx.x & 7, m0 = blockIdx.y * 32, n0 = blockIdx.x * 32, m = m0 + row, n = n0 + ch * 4;
+    const bool in = m < a.M && n < a.N;
     float *dst = a.out + (size_t)m * a.ldc + n;
-    float t[4] = {0.f, 0.f, 0.f, 0.f}, res[4] = {0.f, 0.f, 0.f, 0.f};
-    if (a.accumulate) {
+    float res[4] = {0.f, 0.f, 0.f, 0.f};
+    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+    uint32_t plain = 0;
+    if (in) {
+        if (a.accumulate) {
 #pragma unroll
-        for (int j = 0; j < 4; j++) res[j] = dst[j];
-    }
-    const float *p = parts + (size_t)m * a.N + n;
+            for (int j = 0; j < 4; j++) res[j] = dst[j];
+        }
+        const float *p = parts + (size_t)m * a.N + n;
 #pragma unroll 4
-    for (int z = 0; z < a.splits; z++) {
-        const float4 v = __ldcs((const float4 *)(p + (size_t)z * a.M * a.N));
-        t[0] += v.x; t[1] += v.y; t[2] += v.z; t[3] += v.w;
+        for (int z = 0; z < a.splits; z++) {
+            const float4 v = __ldcs((const float4 *)(p + (size_t)z * a.M * a.N));
+            t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w;
+        }
+        plain = (f32_finite(t.x) ? 0 : 1) | (f32_finite(t.y) ? 0 : 2) | (f32_finite(t.z) ? 0 : 4) | (f32_finite(t.w) ? 0 : 8);
     }
+    if (__syncthreads_or(plain != 0)) {                     // the plain chain, every thread its own four
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        const bool w_side = threadIdx.x >= 128;
+        const int fr = (threadIdx.x & 127) >> 2, fq = threadIdx.x & 3;
+        const float *src = (w_side ? a.W + (size_t)min(n0 + fr, a.N - 1) * a.ldw : a.A + (size_t)min(m0 + fr, a.M - 1) * a.lda) + fq * 4;
+        float4 *into = (w_side ? TW : TA) + fr * 4 + (fq ^ ((fr >> (w_side ? 2 : 0)) & 3));
+        for (int k0 = 0; k0 < a.K; k0 += 16) {
+            const float4 v = k0 + fq * 4 < a.K ? *(const float4 *)(src + k0) : make_float4(0.f, 0.f, 0.f, 0.f);
+            __syncthreads();
+            *into = v;
+            __syncthreads();
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        if (!f32_finite(t[j])) t[j] = f32_plain_dot(a.A + (size_t)m * a.lda, a.W + (size_t)(n + j) * a.ldw, a.K);
-        dst[j] = t[j] + res[j];
+            for (int q = 0; q < 4; q++) {
+                const float4 x = TA[row * 4 + (q ^ (row & 3))];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const float4 y = TW[(ch * 4 + j) * 4 + (q ^ (ch & 3))];
+                    acc[j] = fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.x, y.x, acc[j]))));
+                }
+            }
+        }
+        t = make_float4(plain & 1 ? acc[0] : t.x, plain & 2 ? acc[1] : t.y, plain & 4 ? acc[2] : t.z, plain & 8 ? acc[3] : t.w);
     }
+    if (!in) return;
+    dst[0] = t.x + res[0]; dst[1] = t.y + res[1]; dst[2] = t.z + res[2]; dst[3] = t.w + res[3];
 }
 
 // ---------------------------------------------------------------------------- host side
@@ -383,8 +500,7 @@ extern "C" int fg_gemm_f32_tc(const float *A, int lda, const float *W, int ldw, 
             if (e) return e;
             if (split) {
                 a.out = out;
-                const long long n4 = (long long)mr * (nr / 4);
-                e = fg_launch_in_order(gemm_f32_finish_kernel, dim3((unsigned)((n4 + 255) / 256)), dim3(256), 0, stream, a, (const float *)parts);
+                e = fg_launch_in_order(gemm_f32_finish_kernel, dim3((nr + 31) / 32, (mr + 31) / 32), dim3(256), 0, stream, a, (const float *)parts);
                 if (e) return e;
             }
         }

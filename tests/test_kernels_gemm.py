@@ -258,6 +258,42 @@ def test_gemm_f32_on_planes_keeps_what_the_split_does_not_carry(M, N, K):
     assert ((got - plain).double().abs()[ok] <= 4e-6 * scale[ok]).all()
 
 
+@pytest.mark.parametrize("M,N,K", [(40, 1000, 2048), (300, 515, 1024), (1000, 8200, 2048)])      # with parts and without, ragged tiles
+def test_gemm_f32_on_planes_without_a_finite_number(M, N, K):
+    """Outputs that the plain chain has to give are computed side by side: operands full of NaN take no more than ten times the plain kernel,
+    and everything beside them keeps its bits."""
+    from fastgguf_b200 import ops
+    from fastgguf_b200.ops import fast_gemm
+    a, w = _operands(M, N, K, torch.float32, 16)
+    clean, res = fast_gemm.gemm_f32(a, w), torch.randn(M, N, device="cuda")
+    rows, cols = torch.randperm(M)[:3], torch.randperm(N)[:2]
+    some, ws = a.clone(), w.clone()
+    some[rows, 5], ws[cols, 9] = float("nan"), float("inf")
+    got, acc = fast_gemm.gemm_f32(some, ws), res.clone()
+    fast_gemm.gemm_f32(some, ws, out=acc, accumulate=True)
+    plain = ops.gemm_generic(some, ws, out_dtype=torch.float32)
+    ok = plain.isfinite()
+    assert torch.equal(got[~ok].isnan(), plain[~ok].isnan()) and torch.equal(got[~ok].sign().nan_to_num(), plain[~ok].sign().nan_to_num())
+    assert torch.equal(got[ok], clean[ok]) and torch.equal(acc[ok], clean[ok] + res[ok]) and not acc[~ok].isfinite().any()
+    nothing = torch.full_like(a, float("nan"))
+    assert fast_gemm.gemm_f32(nothing, w).isnan().all()
+
+    def us(f):
+        f()
+        t = []
+        for _ in range(3):
+            one, two = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            one.record()
+            f()
+            two.record()
+            torch.cuda.synchronize()
+            t.append(one.elapsed_time(two) * 1e3)
+        return min(t)
+
+    assert us(lambda: fast_gemm.gemm_f32(nothing, w)) < 10 * us(lambda: ops.gemm_generic(nothing, w, out_dtype=torch.float32))
+    assert fast_gemm.pipeline_error() == 0
+
+
 def test_gemm_f32_on_planes_refuses_other_sizes():
     from fastgguf_b200.ops import fast_gemm
     for M, N, K in ((16, 512, 1024), (64, 256, 1024), (100, 128, 1024), (100, 512, 256), (100, 512, 1028)):
