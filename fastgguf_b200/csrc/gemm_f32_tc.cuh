@@ -2,7 +2,12 @@
 // and results, for more rows than the weight-streaming kernel takes (part of gemm_tc.cu's translation unit, whose helpers it uses).
 //
 // A float32 number is the sum of three bfloat16 numbers: hi = bf16(a), mid = bf16(a - hi), lo = a - hi - mid, 8 bits of mantissa each
-// and the differences exact.  A product of two such sums is nine products of bfloat16 numbers, each exact in float32; the six largest
+// and the differences exact - as long as lo is not below bfloat16's smallest number, 2^-133.  A row of an operand that would lose bits
+// so, and one whose largest magnitude is not in [2^-40, 2^50), is therefore first multiplied by the power of two that brings its largest
+// magnitude just below 2^50 (at most by 2^63, which carries all that float32 holds), and its sums by the inverse power at the end: a row
+// whose largest magnitude is below 2^34 is carried whole, down to float32's smallest number, a row with a larger one down to 2^-183 of it.
+// Such rows are rare: a flag in scratch memory says whether the operands have one, and without it no power is looked at.
+// A product of two such sums is nine products of bfloat16 numbers, each exact in float32; the six largest
 // (hi hi, hi mid, mid hi, mid mid, hi lo, lo hi) are computed, the other three are below 2^-24 of the product.
 //
 // What is left is the order of additions.  The tensor cores' accumulator is float32, but its sums are cut off, not rounded, and over
@@ -20,10 +25,11 @@
 // 3,175 (248 TFLOP/s; a sixth of the bfloat16 burst rate is 270); 2,048 x 2,048 x 8,192: 306 against 1,747; 600 x 2,048 x 8,192: 143
 // against 1,249; 24 x 2,048 x 2,048: 38 against 210.
 //
-// Numbers that the split does not carry (infinities, NaN, magnitudes whose first plane or whose partial sums overflow) leave a sum
-// that is no finite number; such an output is computed again by the plain chain of fused multiply-adds over the float32 operands, a warp
-// for 32 x 32 outputs.
+// Two kinds of outputs are computed by the plain chain of fused multiply-adds over the float32 operands, a warp for a tile of 32 x 32:
+// those that come out as no finite number (infinities and NaN among the operands), and those whose rows are so large that the plain
+// chain might overflow on its way (K times the product of the rows' largest magnitudes above 2^126) - the planes, scaled, would not.
 #pragma once
+#include <atomic>
 
 #define F32_EPI_WARPS 8
 #define F32_THREADS (64 + 32 * F32_EPI_WARPS)
@@ -31,7 +37,10 @@
 
 struct F32Args {
     float *out;                            // [M, ldc], or the parts [splits][M][N]
-    const float *A, *W;                    // the float32 operands, for outputs that are computed again
+    const float *A, *W;                    // the float32 operands, for outputs that the plain chain computes
+    const int *a_shift, *w_shift;          // exponents of the powers of two that the operands' rows were multiplied by, times 2^23
+    int least_shift;                       // an output whose two exponents (times 2^23) sum up to less belongs to the plain chain
+    unsigned long long *flag, call;        // *flag == call: a row of this call's operands was multiplied (anything else that memory held says no)
     int M, N, K, ldc, lda, ldw;
     int splits, kb_per_split;
     int a_rows, w_rows;                    // rows between the planes of the operands
@@ -39,6 +48,10 @@ struct F32Args {
 };
 
 __device__ __forceinline__ bool f32_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
+// The bits of the power of two that brings a sum back to scale: 2^-(a_shift + w_shift), whose exponent is at most 126; a sum whose shifts are
+// so small that the power is no number belongs to the plain chain (f32_too_large).
+__device__ __forceinline__ uint32_t f32_back(int a_shift, int w_shift) { return 0x3f800000u - (uint32_t)a_shift - (uint32_t)w_shift; }
+__device__ __forceinline__ bool f32_too_large(int a_shift, int w_shift, int least_shift) { return (a_shift >> 23) + (w_shift >> 23) < (least_shift >> 23); }
 // zero where all four are finite numbers (and `sum` was), NaN where one is not
 __device__ __forceinline__ float f32_check4(float4 t, float sum) { return fmaf(t.x, 0.f, fmaf(t.y, 0.f, fmaf(t.z, 0.f, fmaf(t.w, 0.f, sum)))); }
 
@@ -109,20 +122,63 @@ __device__ __forceinline__ void f32_plain_tile(float *T, const F32Args &a, int m
     __syncwarp();
 }
 
-// planes[p][row][k], p = 0 (hi), 1 (mid), 2 (lo).  Bound by memory: 4 bytes in, 6 out.  A thread takes eight numbers.
-__global__ void __launch_bounds__(256)
-f32_split_kernel(const float *__restrict__ x, int ld, bf16 *__restrict__ planes, int rows, int K) {
-    const int per_row = K / 8;
-    const long long n = (long long)rows * per_row;
+// planes[p][row][k], p = 0 (hi), 1 (mid), 2 (lo) of x[row][k] * 2^shift[row].  Bound by memory: 4 bytes in, 6 out.  A row is a block's, KEEP
+// times eight numbers a thread, which stay in registers between the row's largest and smallest magnitudes and the planes (beyond 32,768
+// numbers the rest of a row comes from the caches again).  16,384 rows of 2,048 49.5 us (6.8 TB/s; 57 us when threads walked all rows in steps), 2,048 rows of 8,192 25 us,
+// 300 rows of 28,672 20 us.
+template <int KEEP>
+__global__ void __launch_bounds__(KEEP == 2 ? 256 : 512)
+f32_split_kernel(const float *__restrict__ x, int ld, bf16 *__restrict__ planes, int *__restrict__ shift, unsigned long long *flag,
+                 unsigned long long call, int rows, int K) {
+    __shared__ float scratch[32];
+    const int n8 = K / 8, r = blockIdx.x;
     const size_t plane = (size_t)rows * K;
-    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
-        const int r = (int)(i / per_row), c = (int)(i % per_row) * 8;
-        const float4 u[2] = {__ldcs((const float4 *)(x + (size_t)r * ld + c)), __ldcs((const float4 *)(x + (size_t)r * ld + c + 4))};
-        const float v[8] = {u[0].x, u[0].y, u[0].z, u[0].w, u[1].x, u[1].y, u[1].z, u[1].w};
+    const float *src = x + (size_t)r * ld;
+    float v[KEEP][8], largest = 0.f;
+    uint32_t smallest = 0xffffffffu;                       // twice the bits of the smallest number that is not a bfloat16 number, less one
+    auto fetch = [&](float (&u)[8], int i) {
+        const float4 lo = *(const float4 *)(src + i * 8), hi = *(const float4 *)(src + i * 8 + 4);
+        u[0] = lo.x; u[1] = lo.y; u[2] = lo.z; u[3] = lo.w; u[4] = hi.x; u[5] = hi.y; u[6] = hi.z; u[7] = hi.w;
+    };
+    auto look = [&](const float (&u)[8]) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            largest = fmaxf(largest, fabsf(u[j]));         // (a NaN leaves it as it is)
+            const uint32_t bits = __float_as_uint(u[j]);
+            if (bits & 0xffffu) smallest = min(smallest, (bits << 1) - 1u);
+        }
+    };
+#pragma unroll
+    for (int q = 0; q < KEEP; q++) {
+        const int i = threadIdx.x + q * blockDim.x;
+        if (i < n8) fetch(v[q], i);
+        else
+#pragma unroll
+            for (int j = 0; j < 8; j++) v[q][j] = 0.f;
+    }
+#pragma unroll
+    for (int q = 0; q < KEEP; q++) look(v[q]);
+    for (int i = threadIdx.x + KEEP * blockDim.x; i < n8; i += blockDim.x) {
+        float u[8];
+        fetch(u, i);
+        look(u);
+    }
+    const bool tiny = __syncthreads_or(smallest < (17u << 24) - 1u);           // below 2^(17 - 127): bits below 2^-133
+    largest = block_max(largest, scratch);
+    // the exponent field f says |x| < 2^(f - 126); infinities as the largest finite numbers
+    const int field = min(__float_as_int(largest) >> 23, 254), sh = tiny || field > 176 || (field < 87 && largest > 0.f) ? min(176 - field, 63) : 0;
+    const float factor = __int_as_float((sh + 127) << 23);
+    if (threadIdx.x == 0) {
+        shift[r] = sh << 23;
+        if (sh) *flag = call;                              // (every writer writes the same)
+    }
+    if (r == rows - 1)                                     // (tiles read the shifts of all their rows)
+        for (int q = rows + threadIdx.x; q < (rows + 255) / 256 * 256; q += blockDim.x) shift[q] = 0;
+    auto write = [&](const float (&u)[8], int i) {
         uint32_t w[3][4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            float a = v[2 * j], b = v[2 * j + 1];
+            float a = u[2 * j] * factor, b = u[2 * j + 1] * factor;
 #pragma unroll
             for (int p = 0; p < 3; p++) {
                 const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
@@ -132,7 +188,17 @@ f32_split_kernel(const float *__restrict__ x, int ld, bf16 *__restrict__ planes,
             }
         }
 #pragma unroll
-        for (int p = 0; p < 3; p++) *(uint4 *)(planes + p * plane + (size_t)r * K + c) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+        for (int p = 0; p < 3; p++) *(uint4 *)(planes + p * plane + (size_t)r * K + i * 8) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+    };
+#pragma unroll
+    for (int q = 0; q < KEEP; q++) {
+        const int i = threadIdx.x + q * blockDim.x;
+        if (i < n8) write(v[q], i);
+    }
+    for (int i = threadIdx.x + KEEP * blockDim.x; i < n8; i += blockDim.x) {
+        float u[8];
+        fetch(u, i);
+        write(u, i);
     }
 }
 
@@ -244,6 +310,7 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_const
         // ------------------------------------------------------------ sums and epilogue (warps 2.., both CTAs): this CTA's 128 rows
         const int lg = warp & 3, half = (warp - 2) >> 2;
         float *T = (float *)(smem + STAGES * STAGE_BYTES) + (warp - 2) * (F32_STAGING / 4);
+        const bool scaled = *a.flag == a.call;
         int i = 0;
         bool ok = true;
         for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
@@ -270,7 +337,7 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_const
                 if (lane == 0) mbar_arrive_cluster(lead_tempty0 + 8 * acc);
             }
             if (!ok) break;
-            // 32 columns at a time through a tile in shared memory, so that a warp stores whole 128-byte lines
+            // 32 columns at a time through a tile in shared memory, so that a warp stores whole 128-byte lines; parts stay scaled
             const bool part = a.splits > 1;
             float *out = part ? a.out + (size_t)z * a.M * a.N : a.out;
             const int ldc = part ? a.N : a.ldc, ch = lane & 7;
@@ -285,11 +352,16 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_const
                     check = f32_check4(t, check);
                     *(float4 *)(T + lane * 32 + ((q ^ (lane & 7)) << 2)) = t;
                 }
-                const bool some = !part && __any_sync(0xffffffffu, check != 0.f);
+                const bool some = !part && (scaled || __any_sync(0xffffffffu, check != 0.f));
                 if (some && m_base + lane < a.M) {
+                    const int row_shift = scaled ? a.a_shift[m_base + lane] : 0;
 #pragma unroll 1
-                    for (int j = 0; j < 32; j++)
-                        if (!f32_finite(T[lane * 32 + (((j >> 2) ^ (lane & 7)) << 2) + (j & 3)])) plain[c] |= 1u << j;
+                    for (int j = 0; j < 32 && n_base + c * 32 + j < a.N; j++) {
+                        float &v = T[lane * 32 + (((j >> 2) ^ (lane & 7)) << 2) + (j & 3)];
+                        const int col_shift = scaled ? a.w_shift[n_base + c * 32 + j] : 0;
+                        if (!f32_finite(v) || f32_too_large(row_shift, col_shift, a.least_shift)) plain[c] |= 1u << j;
+                        v *= __uint_as_float(f32_back(row_shift, col_shift));
+                    }
                 }
                 any_plain |= some;
                 __syncwarp();
@@ -370,7 +442,14 @@ gemm_f32_finish_kernel(F32Args a, const float *__restrict__ parts) {
             const float4 v = __ldcs((const float4 *)(p + (size_t)z * a.M * a.N));
             t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w;
         }
-        plain = (f32_finite(t.x) ? 0 : 1) | (f32_finite(t.y) ? 0 : 2) | (f32_finite(t.z) ? 0 : 4) | (f32_finite(t.w) ? 0 : 8);
+        const bool scaled = *a.flag == a.call;
+        const int sa = scaled ? a.a_shift[m] : 0;
+        const int4 w = scaled ? *(const int4 *)(a.w_shift + n) : make_int4(0, 0, 0, 0);
+        auto back = [&](float &v, int sw, uint32_t bit) {
+            if (!f32_finite(v) || f32_too_large(sa, sw, a.least_shift)) plain |= bit;
+            v *= __uint_as_float(f32_back(sa, sw));
+        };
+        back(t.x, w.x, 1); back(t.y, w.y, 2); back(t.z, w.z, 4); back(t.w, w.w, 8);
     }
     if (__syncthreads_or(plain != 0)) {                     // the plain chain, every thread its own four
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
@@ -402,7 +481,7 @@ gemm_f32_finish_kernel(F32Args a, const float *__restrict__ parts) {
 // ---------------------------------------------------------------------------- host side
 #define F32_PLANE_LIMIT ((size_t)256 << 20)            // bytes of planes of one operand at a time: scratch memory stays bounded
 
-struct F32Plan { int bn, splits, kb_per_split, a_rows, w_rows; size_t a_bytes, w_bytes, part_bytes; };
+struct F32Plan { int bn, splits, kb_per_split, a_rows, w_rows; size_t a_bytes, w_bytes, part_bytes, shift_bytes; };
 
 // How the contraction is cut: rows of the operands whose planes are made at a time, tile width, splits along K.  The times
 // are those of a K-block (microseconds), of the start and end of a tile, and of the pass that adds the parts.
@@ -429,6 +508,7 @@ static F32Plan f32_plan(int M, int N, int K) {
     best.a_rows = am; best.w_rows = wn;
     best.a_bytes = up(am * row_bytes); best.w_bytes = up(wn * row_bytes);
     best.part_bytes = best.splits > 1 ? up((size_t)best.splits * am * wn * 4) : 0;
+    best.shift_bytes = up((size_t)am * 4) + up((size_t)wn * 4) + 1024;
     return best;
 }
 
@@ -439,7 +519,7 @@ static F32Plan f32_plan(int M, int N, int K) {
 extern "C" long long fg_gemm_f32_tc_workspace_bytes(int M, int N, int K) {
     if (M <= 16 || N < 256 || K < 512 || K % 8 || (M <= 64 && (long long)N * K <= 1 << 18)) return 0;
     const F32Plan p = f32_plan(M, N, K);
-    return (long long)(p.a_bytes + p.w_bytes + p.part_bytes);
+    return (long long)(p.a_bytes + p.w_bytes + p.part_bytes + p.shift_bytes);
 }
 
 template <int BN>
@@ -461,9 +541,12 @@ static int launch_f32_pair(const CUtensorMap &tmP, const CUtensorMap &tmQ, const
     return (int)cudaLaunchKernelEx(&cfg, gemm_f32_pair_kernel<BN>, tmP, tmQ, a, n_pt, n_tiles);
 }
 
-static int launch_f32_split(const float *x, int ld, bf16 *planes, int rows, int K, cudaStream_t stream) {
-    const long long blocks = ((long long)rows * (K / 8) + 255) / 256, most = 8LL * sm_count();
-    return fg_launch_in_order(f32_split_kernel, dim3((unsigned)(blocks < most ? blocks : most)), dim3(256), 0, stream, x, ld, planes, rows, K);
+static int launch_f32_split(const float *x, int ld, bf16 *planes, int *shift, unsigned long long *flag, unsigned long long call, int rows, int K,
+                            cudaStream_t stream) {
+    if (K <= 4096)
+        return fg_launch_in_order(f32_split_kernel<2>, dim3(rows), dim3((K / 16 + 31) / 32 * 32), 0, stream, x, ld, planes, shift, flag, call, rows, K);
+    const int threads = K >= 32768 ? 512 : (K / 64 + 31) / 32 * 32;
+    return fg_launch_in_order(f32_split_kernel<8>, dim3(rows), dim3(threads), 0, stream, x, ld, planes, shift, flag, call, rows, K);
 }
 
 // C[m, n] (+)= sum_k A[m, k] W[n, k], everything float32.  Needs fg_gemm_f32_tc_workspace_bytes of 1024-byte aligned scratch
@@ -477,14 +560,22 @@ extern "C" int fg_gemm_f32_tc(const float *A, int lda, const float *W, int ldw, 
     const F32Plan p = f32_plan(M, N, K);
     bf16 *ap = (bf16 *)ws, *wp = (bf16 *)((char *)ws + p.a_bytes);
     float *parts = (float *)((char *)ws + p.a_bytes + p.w_bytes);
+    int *a_shift = (int *)((char *)ws + p.a_bytes + p.w_bytes + p.part_bytes), *w_shift = a_shift + ((size_t)p.a_rows * 4 + 1023) / 1024 * 256;
+    unsigned long long *flag = (unsigned long long *)(w_shift + ((size_t)p.w_rows * 4 + 1023) / 1024 * 256);
+    static std::atomic<unsigned long long> calls{0x5eed0000f32a11ull};
+    const unsigned long long call = calls.fetch_add(1);    // (a recorded call keeps its number: its flag may stay up, which costs time, no bits)
+    // |a| < 2^(50 - shift): K products of less than 2^(100 - a_shift - w_shift) stay below 2^126
+    int least_shift = -26;
+    while ((1LL << (least_shift + 26)) < K) least_shift++;
+    least_shift *= 1 << 23;
     for (int m0 = 0; m0 < M; m0 += p.a_rows) {
         const int mr = M - m0 < p.a_rows ? M - m0 : p.a_rows;
-        int e = launch_f32_split(A + (size_t)m0 * lda, lda, ap, mr, K, stream);
+        int e = launch_f32_split(A + (size_t)m0 * lda, lda, ap, a_shift, flag, call, mr, K, stream);
         if (e) return e;
         for (int n0 = 0; n0 < N; n0 += p.w_rows) {
             const int nr = N - n0 < p.w_rows ? N - n0 : p.w_rows;
             if (n0 > 0 || m0 == 0 || p.w_rows < N) {                        // (the planes of W are kept where all of them fit)
-                e = launch_f32_split(W + (size_t)n0 * ldw, ldw, wp, nr, K, stream);
+                e = launch_f32_split(W + (size_t)n0 * ldw, ldw, wp, w_shift, flag, call, nr, K, stream);
                 if (e) return e;
             }
             CUtensorMap tmP, tmQ;
@@ -494,7 +585,7 @@ extern "C" int fg_gemm_f32_tc(const float *A, int lda, const float *W, int ldw, 
             if (e) return e;
             float *out = C + (size_t)m0 * ldc + n0;
             const bool split = p.splits > 1;
-            F32Args a{split ? parts : out, A + (size_t)m0 * lda, W + (size_t)n0 * ldw, mr, nr, K, ldc, lda, ldw, p.splits, p.kb_per_split, mr, nr,
+            F32Args a{split ? parts : out, A + (size_t)m0 * lda, W + (size_t)n0 * ldw, a_shift, w_shift, least_shift, flag, call, mr, nr, K, ldc, lda, ldw, p.splits, p.kb_per_split, mr, nr,
                       accumulate, split ? nr % 4 == 0 : ((uintptr_t)out % 16 == 0 && ldc % 4 == 0)};
             e = p.bn == 256 ? launch_f32_pair<256>(tmP, tmQ, a, stream) : launch_f32_pair<128>(tmP, tmQ, a, stream);
             if (e) return e;

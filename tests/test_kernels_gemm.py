@@ -294,6 +294,45 @@ def test_gemm_f32_on_planes_without_a_finite_number(M, N, K):
     assert fast_gemm.pipeline_error() == 0
 
 
+@pytest.mark.parametrize("M,N,K", [(40, 1000, 2048), (300, 515, 1024), (130, 2100, 12288)])
+def test_gemm_f32_on_planes_over_float32s_range(M, N, K):
+    """Operands far below bfloat16's smallest number times operands far above one, rows whose numbers lie 2^105 apart, sums below float32's
+    normal numbers and sums above its largest: no further from float64 than the plain chain is, which carries all of it."""
+    from fastgguf_b200 import ops
+    from fastgguf_b200.ops import fast_gemm
+    a, w = _operands(M, N, K, torch.float32, 26)
+    g = torch.Generator().manual_seed(3)
+    mixed = torch.exp2(torch.randint(-115, -9, (K,), generator=g).float()).cuda()
+    down, up = 2.0 ** -115, 2.0 ** 105
+    for x, y in ((a * down, w * up), (a * up, w * down), (a * 2.0 ** -100 * 2.0 ** -22, w * 2.0 ** 100), (a * mixed, w / mixed)):
+        want = x.double() @ y.double().T
+        got, plain = fast_gemm.gemm_f32(x, y), ops.gemm_generic(x, y, out_dtype=torch.float32)
+        assert (got.double() - want).norm() <= (plain.double() - want).norm()
+    x, y = a * 2.0 ** -80, w * 2.0 ** -62                  # sums of a few units of float32's smallest number
+    want = x.double() @ y.double().T
+    assert want.abs().max() < 2.0 ** -126
+    assert (fast_gemm.gemm_f32(x, y).double() - want).abs().max() <= 0.75 * 2.0 ** -149 + 2.0 ** -22 * want.abs().max()
+    x, y = a * 2.0 ** 70, w * 2.0 ** 57                    # around float32's largest number: what overflows on the way there does so here
+    got, plain = fast_gemm.gemm_f32(x, y), ops.gemm_generic(x, y, out_dtype=torch.float32)
+    assert torch.equal(got, plain) or torch.equal(got.nan_to_num(7.0), plain.nan_to_num(7.0))
+    assert plain.isinf().any() or plain.isnan().any()
+    x, y, clean = a.clone(), w.clone(), fast_gemm.gemm_f32(a, w)     # a few such rows among ordinary ones, whose outputs keep their bits
+    x[M // 3] *= down
+    x[M - 1] *= 2.0 ** 60
+    y[N // 2] *= 2.0 ** -118
+    got, want, plain = fast_gemm.gemm_f32(x, y), x.double() @ y.double().T, ops.gemm_generic(x, y, out_dtype=torch.float32)
+    rows, cols = torch.arange(M, device="cuda"), torch.arange(N, device="cuda")
+    rows, cols = rows[(rows != M // 3) & (rows != M - 1)], cols[cols != N // 2]
+    assert torch.equal(got[rows][:, cols], clean[rows][:, cols])
+    for part in (got[M // 3], got[M - 1], got[rows, N // 2]):
+        assert part.isfinite().all()
+    for i in (M // 3, M - 1):
+        assert (got[i, cols].double() - want[i, cols]).norm() <= (plain[i, cols].double() - want[i, cols]).norm()
+    assert (got[rows, N // 2].double() - want[rows, N // 2]).norm() <= (plain[rows, N // 2].double() - want[rows, N // 2]).norm()
+    zero = torch.zeros_like(a)
+    assert not fast_gemm.gemm_f32(zero, w).any() and not fast_gemm.gemm_f32(a, torch.zeros_like(w)).any()
+
+
 def test_gemm_f32_on_planes_refuses_other_sizes():
     from fastgguf_b200.ops import fast_gemm
     for M, N, K in ((16, 512, 1024), (64, 256, 1024), (100, 128, 1024), (100, 512, 256), (100, 512, 1028)):
