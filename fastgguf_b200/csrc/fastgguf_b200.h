@@ -288,7 +288,8 @@ int fg_gemm_tc_grouped(const void *X, int ldx, int rows, const void *W, int ldw,
 int fg_gemm_tc_grouped_ext(const void *X, int ldx, int rows, const void *W, int ldw, int stack_rows, void *out, int ldc, int epi /* 1 or 4 */, int N,
                            int K, const void *tiles, int n_tiles, cudaStream_t stream);
 /* float32 operands and result: C (+)= A W^T with every operand as the sum of three bfloat16 planes made in scratch memory; 0 bytes: refused */
-long long fg_gemm_f32_tc_workspace_bytes(int M, int N, int K);
+long long fg_gemm_f32_tc_workspace_bytes(int M, int N, int K);      /* the most that helps */
+long long fg_gemm_f32_tc_least_bytes(int M, int N, int K);          /* the least it runs with, in more portions and with the same sums */
 int fg_gemm_f32_tc(const float *A, int lda, const float *W, int ldw, float *C, int ldc, int accumulate, int M, int N, int K,
                    void *ws, long long ws_bytes, cudaStream_t stream);
 /* the same product for up to 16 rows on the FMA units, weights streamed through shared memory */

@@ -479,21 +479,34 @@ gemm_f32_finish_kernel(F32Args a, const float *__restrict__ parts) {
 }
 
 // ---------------------------------------------------------------------------- host side
-#define F32_PLANE_LIMIT ((size_t)256 << 20)            // bytes of planes of one operand at a time: scratch memory stays bounded
+// Bytes of planes of one operand at a time: scratch memory stays bounded.  Half of it, a quarter or an eighth do where memory is short:
+// the sums are the same, an operand's rows go through in more portions.
+#define F32_PLANE_LIMIT ((size_t)256 << 20)
+#define F32_LEAST_LIMIT (F32_PLANE_LIMIT / 8)
 
-struct F32Plan { int bn, splits, kb_per_split, a_rows, w_rows; size_t a_bytes, w_bytes, part_bytes, shift_bytes; };
+struct F32Plan { int M, N, K, bn, splits, kb_per_split, a_rows, w_rows; size_t a_bytes, w_bytes, part_bytes, shift_bytes, bytes; };
 
-// How the contraction is cut: rows of the operands whose planes are made at a time, tile width, splits along K.  The times
-// are those of a K-block (microseconds), of the start and end of a tile, and of the pass that adds the parts.
+// The rows of the operands whose planes are made at a time, where `limit` bytes of planes of an operand are allowed.
+static int f32_rows_at_a_time(int rows, int K, size_t limit) {
+    const size_t most = limit / ((size_t)K * 6) / 256 * 256;
+    return (size_t)rows <= most ? rows : (int)(most < 256 ? 256 : most);
+}
+static void f32_portions(F32Plan &p, size_t limit) {
+    auto up = [](size_t b) { return (b + 1023) / 1024 * 1024; };
+    p.a_rows = f32_rows_at_a_time(p.M, p.K, limit); p.w_rows = f32_rows_at_a_time(p.N, p.K, limit);
+    p.a_bytes = up((size_t)p.a_rows * p.K * 6); p.w_bytes = up((size_t)p.w_rows * p.K * 6);
+    p.part_bytes = p.splits > 1 ? up((size_t)p.splits * p.a_rows * p.w_rows * 4) : 0;
+    p.shift_bytes = up((size_t)p.a_rows * 4) + up((size_t)p.w_rows * 4) + 1024;
+    p.bytes = p.a_bytes + p.w_bytes + p.part_bytes + p.shift_bytes;
+}
+
+// How the contraction is cut: tile width and splits along K.  The times are those of a K-block (microseconds), of the start and end of a
+// tile, and of the pass that adds the parts.  Both are chosen for the full limit, so that a smaller one changes no order of additions.
 static F32Plan f32_plan(int M, int N, int K) {
     F32Plan best{};
+    best.M = M; best.N = N; best.K = K;
     const int nkb = (K + BK - 1) / BK, pairs = sm_count() / 2;
-    const size_t row_bytes = (size_t)K * 6;
-    auto rows_at_a_time = [&](int rows) {
-        const size_t most = F32_PLANE_LIMIT / row_bytes / 256 * 256;
-        return (size_t)rows <= most ? rows : (int)(most < 256 ? 256 : most);
-    };
-    const int am = rows_at_a_time(M), wn = rows_at_a_time(N);
+    const int am = f32_rows_at_a_time(M, K, F32_PLANE_LIMIT), wn = f32_rows_at_a_time(N, K, F32_PLANE_LIMIT);
     double best_us = 1e30;
     for (int bn = 128; bn <= 256; bn += 128)
         for (int s = 1; s <= 16; s++) {
@@ -504,22 +517,23 @@ static F32Plan f32_plan(int M, int N, int K) {
             const double us = rounds * (per * (bn == 256 ? 1.75 : 0.95) + 4.0) + (s > 1 ? 4.0 + (s + 2.0) * am * wn * 4.0 / 4e6 : 0.0);
             if (us < best_us) { best_us = us; best.bn = bn; best.splits = s; best.kb_per_split = per; }
         }
-    auto up = [](size_t b) { return (b + 1023) / 1024 * 1024; };
-    best.a_rows = am; best.w_rows = wn;
-    best.a_bytes = up(am * row_bytes); best.w_bytes = up(wn * row_bytes);
-    best.part_bytes = best.splits > 1 ? up((size_t)best.splits * am * wn * 4) : 0;
-    best.shift_bytes = up((size_t)am * 4) + up((size_t)wn * 4) + 1024;
+    f32_portions(best, F32_PLANE_LIMIT);
     return best;
 }
 
-// Scratch memory fg_gemm_f32_tc needs; 0: sizes it does not take.  Rows up to 16 belong to the weight-streaming kernel.  Short
+// Scratch memory fg_gemm_f32_tc takes at most, and the least it needs; 0: sizes it does not take.  Rows up to 16 belong to the weight-streaming kernel.  Short
 // reductions and narrow outputs (K < 512, N < 256) stay with the plain kernels: one or two rounds of their tiles take about
 // what the three launches here do; so do small matrices (a megabyte) at up to 64 rows, which the weight-streaming kernel takes.  From 17 rows on the planes won at every size measured (K 2,048 and 8,192, N 2,048 to 16,384, 24 to
 // 2,048 rows: 2.7 to 13 times).
-extern "C" long long fg_gemm_f32_tc_workspace_bytes(int M, int N, int K) {
-    if (M <= 16 || N < 256 || K < 512 || K % 8 || (M <= 64 && (long long)N * K <= 1 << 18)) return 0;
-    const F32Plan p = f32_plan(M, N, K);
-    return (long long)(p.a_bytes + p.w_bytes + p.part_bytes + p.shift_bytes);
+static bool f32_takes(int M, int N, int K) {
+    return !(M <= 16 || N < 256 || K < 512 || K % 8 || (M <= 64 && (long long)N * K <= 1 << 18));
+}
+extern "C" long long fg_gemm_f32_tc_workspace_bytes(int M, int N, int K) { return f32_takes(M, N, K) ? (long long)f32_plan(M, N, K).bytes : 0; }
+extern "C" long long fg_gemm_f32_tc_least_bytes(int M, int N, int K) {
+    if (!f32_takes(M, N, K)) return 0;
+    F32Plan p = f32_plan(M, N, K);
+    f32_portions(p, F32_LEAST_LIMIT);
+    return (long long)p.bytes;
 }
 
 template <int BN>
@@ -549,15 +563,16 @@ static int launch_f32_split(const float *x, int ld, bf16 *planes, int *shift, un
     return fg_launch_in_order(f32_split_kernel<8>, dim3(rows), dim3(threads), 0, stream, x, ld, planes, shift, flag, call, rows, K);
 }
 
-// C[m, n] (+)= sum_k A[m, k] W[n, k], everything float32.  Needs fg_gemm_f32_tc_workspace_bytes of 1024-byte aligned scratch
-// memory; FG_ERR_BAD_SIZE for what it does not take (the plain kernels do).  Kernels are launched in plain stream order.
+// C[m, n] (+)= sum_k A[m, k] W[n, k], everything float32.  Needs 256-byte aligned scratch memory, from
+// fg_gemm_f32_tc_least_bytes to fg_gemm_f32_tc_workspace_bytes of it; FG_ERR_BAD_SIZE for what it does not take (the plain kernels do).  Kernels are launched in plain stream order.
 extern "C" int fg_gemm_f32_tc(const float *A, int lda, const float *W, int ldw, float *C, int ldc, int accumulate, int M, int N, int K,
                               void *ws, long long ws_bytes, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
-    const long long need = fg_gemm_f32_tc_workspace_bytes(M, N, K);
-    if (need == 0 || ws == nullptr || ws_bytes < need || lda % 4 || ldw % 4 || (((uintptr_t)A | (uintptr_t)W) & 15) || ((uintptr_t)ws & 255))
+    if (!f32_takes(M, N, K) || ws == nullptr || lda % 4 || ldw % 4 || (((uintptr_t)A | (uintptr_t)W) & 15) || ((uintptr_t)ws & 255))
         return FG_ERR_BAD_SIZE;
-    const F32Plan p = f32_plan(M, N, K);
+    F32Plan p = f32_plan(M, N, K);
+    for (size_t limit = F32_PLANE_LIMIT / 2; (long long)p.bytes > ws_bytes && limit >= F32_LEAST_LIMIT; limit /= 2) f32_portions(p, limit);
+    if ((long long)p.bytes > ws_bytes) return FG_ERR_BAD_SIZE;
     bf16 *ap = (bf16 *)ws, *wp = (bf16 *)((char *)ws + p.a_bytes);
     float *parts = (float *)((char *)ws + p.a_bytes + p.w_bytes);
     int *a_shift = (int *)((char *)ws + p.a_bytes + p.w_bytes + p.part_bytes), *w_shift = a_shift + ((size_t)p.a_rows * 4 + 1023) / 1024 * 256;

@@ -188,26 +188,47 @@ fg_dev_tensor Tensor::view() const {
 Arena::~Arena() {
     for (auto &l : lanes_)
         for (auto &b : l.blocks) cudaFree(b.p);
-    if (scratch_) cudaFree(scratch_);
 }
 
-void *Arena::scratch(size_t bytes) {
-    if (bytes <= scratch_bytes_) return scratch_;
-    if (frozen_) return nullptr;                       // (the warm-up run before a recording has sized it)
-    size_t size = bytes > 2 * scratch_bytes_ ? bytes : 2 * scratch_bytes_, free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b + scratch_bytes_ < size + ((size_t)1 << 30)) {
-        cudaGetLastError();
-        return nullptr;                                // a gigabyte stays free for what has no other path
+std::shared_ptr<DeviceBuffer> Scratch::get(size_t want, size_t least) {
+    if (block_ && block_->bytes() >= want) return block_;
+    if (refused_ == 0 || want < refused_) {
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); free_b = 0; }
+        const size_t mine = block_ && block_.use_count() == 1 ? block_->bytes() : 0, spare = (size_t)1 << 30;      // what has no other path needs room too
+        const size_t room = free_b + mine > spare ? free_b + mine - spare : 0;
+        // what is wanted, in steps of an eighth (a few rows more do not make another block); or as much of it as there is room for
+        size_t step = (size_t)1 << 20;
+        while (step * 8 < want) step *= 2;
+        size_t size = (want + step - 1) / step * step;
+        if (size > room) size = want;
+        while (size > room && size / 2 >= least) size /= 2;
+        if (size < want) refused_ = want;
+        if (size <= room && size >= least && (!block_ || size > block_->bytes())) {
+            block_.reset();                            // (freeing waits for the device)
+            try {
+                block_ = std::make_shared<DeviceBuffer>(size, "scratch memory");
+            } catch (const Error &) {
+                refused_ = want;
+            }
+        }
     }
-    if (scratch_) cudaFree(scratch_);                  // waits for the device
-    scratch_bytes_ = 0;
-    if (cudaMalloc(&scratch_, size) != cudaSuccess) { cudaGetLastError(); scratch_ = nullptr; return nullptr; }
-    scratch_bytes_ = size;
-    return scratch_;
+    return block_ && block_->bytes() >= least ? block_ : nullptr;
+}
+
+void *Arena::scratch(size_t want, size_t least, size_t *got) {
+    // a recorded step uses, and keeps, the block that its warm-up run sized
+    if (!frozen_) held_.reset();                       // (not the one holder that keeps a block from growing)
+    if (!frozen_) held_ = scratch_->get(want, least);
+    else if (!held_) held_ = scratch_->current();
+    if (!held_ || held_->bytes() < least) return nullptr;
+    *got = held_->bytes();
+    return held_->get();
 }
 
 void Arena::reset() {
     cur_ = 0;
+    if (!frozen_) { held_.reset(); scratch_->new_step(); }
     for (auto &l : lanes_) {
         if (l.used > l.peak) l.peak = l.used;
         l.used = 0;
@@ -255,11 +276,10 @@ void *Arena::alloc(size_t bytes) {
         size_t size = bytes > block_bytes_ ? bytes : block_bytes_;
         void *p = nullptr;
         cudaError_t e = cudaMalloc(&p, size);
-        if (e != cudaSuccess && scratch_) {
+        if (e != cudaSuccess && scratch_->current()) {
             cudaGetLastError();
-            cudaFree(scratch_);                        // waits for the device
-            scratch_ = nullptr;
-            scratch_bytes_ = 0;
+            held_.reset();
+            scratch_->give_back();                     // (freeing waits for the device)
             e = cudaMalloc(&p, size);
         }
         if (e != cudaSuccess) {
@@ -287,7 +307,7 @@ size_t Arena::bytes_reserved() const {
     size_t n = 0;
     for (auto &l : lanes_)
         for (auto &b : l.blocks) n += b.size;
-    return n + scratch_bytes_;
+    return n + (held_ ? held_->bytes() : 0);
 }
 
 DeviceBuffer::DeviceBuffer(size_t bytes, const char *what) : bytes_(bytes) {

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -71,6 +72,22 @@ struct Tensor {
 };
 int elem_size(int dtype);
 
+class DeviceBuffer;
+// Memory that one launch uses and nothing reads afterwards: ONE block for all arenas of an engine, whose work is ordered on one stream.
+// It grows as needed, and is given back when activations find no room.  A recorded step keeps the block that it was recorded with.
+class Scratch {
+public:
+    // a block of `want` bytes, or where the device has no room for that with a gigabyte to spare, of at least `least`; else null
+    std::shared_ptr<DeviceBuffer> get(size_t want, size_t least);
+    std::shared_ptr<DeviceBuffer> current() const { return block_; }
+    void give_back() { block_.reset(); }
+    void new_step() { refused_ = 0; }
+
+private:
+    std::shared_ptr<DeviceBuffer> block_;
+    size_t refused_ = 0;                // asked for in this step, and not to be had
+};
+
 // Device memory for the activations of one step.  Allocation bumps a cursor through a list of blocks; `reset`
 // starts over.  The sequence of allocations of a step is deterministic, so a step that is run once to warm up and
 // then recorded into a CUDA graph gets the same addresses both times; blocks are only added outside a recording.
@@ -82,13 +99,15 @@ int elem_size(int dtype);
 // All work of a step is ordered on one stream, so memory of layer i - 2 is free when layer i writes it.
 class Arena {
 public:
-    explicit Arena(size_t block_bytes = (size_t)64 << 20) : block_bytes_(block_bytes) {}
+    explicit Arena(size_t block_bytes = (size_t)64 << 20, std::shared_ptr<Scratch> scratch = nullptr)
+        : block_bytes_(block_bytes), scratch_(scratch ? scratch : std::make_shared<Scratch>()) {}
     ~Arena();
     Arena(const Arena &) = delete;
     void *alloc(size_t bytes);
-    // Memory that one launch uses and nothing reads afterwards: the same block for every caller, grown as needed.  Null where the
-    // device has no room to spare for it: the caller then takes a path that needs none, and an `alloc` that fails gives it back.
-    void *scratch(size_t bytes);
+    // Memory that one launch uses and nothing reads afterwards (see Scratch): `want` bytes, or at least `least`; how many it became in
+    // *got.  Null: the caller takes a path that needs none.
+    void *scratch(size_t want, size_t least, size_t *got);
+    std::shared_ptr<Scratch> shared_scratch() const { return scratch_; }
     Tensor matrix(int64_t rows, int64_t cols, int dtype);
     void reset();                       // a new step: every lane starts over
     void begin_layer(int i);            // allocations now go to the lane of layer i, which starts over
@@ -106,8 +125,8 @@ private:
     int cur_ = 0;
     size_t block_bytes_;
     bool frozen_ = false;
-    void *scratch_ = nullptr;
-    size_t scratch_bytes_ = 0;
+    std::shared_ptr<Scratch> scratch_;
+    std::shared_ptr<DeviceBuffer> held_;       // the block this arena's step uses
 };
 
 // Device memory that lives as long as its owner.

@@ -85,6 +85,7 @@ public:
     // seed_random: no source; values from the seeded generator.
     void load_weights(const TensorSource *source, bool seed_random, uint64_t seed);
     int64_t weight_bytes() const { return weight_bytes_; }
+    std::shared_ptr<Scratch> shared_scratch() const { return step_arena_.shared_scratch(); }
 
     // max_tokens: the most tokens live sequences hold at any time, each rounded up to a page
     void make_cache(int64_t max_tokens, int n_slots, int max_seq_len, int page_size, bool verbose);

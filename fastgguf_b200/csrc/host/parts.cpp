@@ -188,12 +188,13 @@ Tensor Linear::forward(Runtime &rt, const Tensor &a_in, const DeferredNorm *defe
         }
         // float32 operands as sums of three bfloat16 planes on the tensor cores (more than 16 rows, see gemm_f32_tc.cuh)
         const long long ws_bytes = M > 16 && N >= 256 && K >= 512 ? FG_KERNEL("tc", fg_gemm_f32_tc_workspace_bytes)((int)M, (int)N, (int)K) : 0;
-        void *ws = ws_bytes > 0 ? rt.arena->scratch((size_t)ws_bytes) : nullptr;
+        size_t got = 0;
+        void *ws = ws_bytes > 0 ? rt.arena->scratch((size_t)ws_bytes, (size_t)FG_KERNEL("tc", fg_gemm_f32_tc_least_bytes)((int)M, (int)N, (int)K), &got) : nullptr;
         if (ws) {
             count_launch();
             ProfileScope scope("fg_gemm_f32_tc", profile_on() ? format("%lld x %lld, %lld rows%s", (long long)N, (long long)K, (long long)M, accumulate ? ", residual add" : "").c_str() : nullptr);
             int code = FG_KERNEL("tc", fg_gemm_f32_tc)(a.ptr<float>(), (int)a.ld, W.ptr<float>(), (int)W.ld, out.ptr<float>(), (int)out.ld,
-                                                       accumulate ? 1 : 0, (int)M, (int)N, (int)K, ws, ws_bytes, rt.stream);
+                                                       accumulate ? 1 : 0, (int)M, (int)N, (int)K, ws, (long long)got, rt.stream);
             if (code != KERNEL_BAD_SIZE) {
                 check_kernel(code, "fg_gemm_f32_tc");
                 return out;

@@ -161,7 +161,7 @@ void Sampler::sample(float *logits, int B, int V, int ldl, const int *rows_dev, 
 }
 
 // ------------------------------------------------------------------------------------ recorded decode step
-DecodeGraph::DecodeGraph(Engine &e, Sampler &sampler, int width_) : width(width_), engine_(e), sampler_(sampler), arena_((size_t)16 << 20) {
+DecodeGraph::DecodeGraph(Engine &e, Sampler &sampler, int width_) : width(width_), engine_(e), sampler_(sampler), arena_((size_t)16 << 20, e.model->shared_scratch()) {
     DecoderModel &model = *e.model;
     PagedKVCache &cache = *model.cache;
     table_width = (cache.max_seq_len + cache.page_size - 1) / cache.page_size;

@@ -155,3 +155,28 @@ def test_plain_kernels_switch_gives_the_same_tokens(models, monkeypatch):
     want = plain_llama.plain_forward(cfg, W, toks).numpy()
     scale = np.abs(want).max()
     assert np.abs(got[1] - want).max() <= 1e-2 * scale and np.abs(got[0] - want).max() <= 1e-2 * scale
+
+
+def test_float32_scratch_memory_is_shared_by_the_steps_of_an_engine():
+    """Recorded float32 steps of 17 and more sequences and prompt steps use one block of scratch memory between them: a second width of the
+    step, and a second sampler, add little, and what they compute stays the same while the block grows."""
+    from helpers import TINY_B
+    from fastgguf_b200.engine.api import Engine
+    from fastgguf_b200.registry import config_from_dict
+    cfg = dict(TINY_B, hidden_size=1024, num_attention_heads=16, num_key_value_heads=4, head_dim=64, intermediate_size=2048, vocab_size=32000)
+    eng = Engine.from_random(config_from_dict(cfg), 3, dtype="float32", max_tokens=16384, max_batch=64)
+    prompts = [[(7 * i + 3 * k) % 32000 for i in range(5 + k % 7)] for k in range(40)]
+
+    def held(n, temp):
+        """tokens, and how many MB of device memory came to be held"""
+        before = torch.cuda.mem_get_info()[0]
+        done = eng.generate(prompts[:n], temp=temp, top_k=4, max_tokens=5, seed=3, ignore_eos=True, use_graphs=True)
+        torch.cuda.synchronize()
+        return [c.tokens for c in done], (before - torch.cuda.mem_get_info()[0]) / 2 ** 20
+
+    first = held(20, 0.0)                                  # planes of the head alone: 32,000 x 1,024 x 6 bytes, 188 MB
+    assert first[1] > 150
+    grown = [held(40, 0.0)[1], held(20, 0.5)[1], held(40, 0.5)[1]]
+    assert max(grown) < 150, grown
+    again = held(20, 0.0)
+    assert again[0] == first[0]

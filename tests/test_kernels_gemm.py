@@ -333,6 +333,28 @@ def test_gemm_f32_on_planes_over_float32s_range(M, N, K):
     assert not fast_gemm.gemm_f32(zero, w).any() and not fast_gemm.gemm_f32(a, torch.zeros_like(w)).any()
 
 
+@pytest.mark.parametrize("M,N,K", [(32, 40000, 2048), (6000, 4100, 8192), (600, 2048, 8192)])
+def test_gemm_f32_on_planes_with_less_scratch_memory(M, N, K):
+    """Less scratch memory means more portions of the operands and the same bits; less than the least is refused."""
+    import ctypes
+    from fastgguf_b200.ops import fast_gemm
+    from fastgguf_b200.ops.lib import lib, ptr, stream
+    a, w = _operands(M, N, K, torch.float32, 36)
+    want = fast_gemm.gemm_f32(a, w)
+    most, least = lib("tc").fg_gemm_f32_tc_workspace_bytes, lib("tc").fg_gemm_f32_tc_least_bytes
+    most.restype = least.restype = ctypes.c_longlong
+    top, low = most(M, N, K), least(M, N, K)
+    assert 0 < low <= top
+    for size in (low, low + (top - low) // 4, low + (top - low) // 2, top - 1):
+        if size < low:
+            continue
+        ws, out = torch.empty(size, dtype=torch.uint8, device="cuda"), torch.zeros(M, N, device="cuda")
+        assert lib("tc").fg_gemm_f32_tc(ptr(a), K, ptr(w), K, ptr(out), N, 0, M, N, K, ptr(ws), size, stream()) == 0
+        assert torch.equal(out, want)
+    ws = torch.empty(low, dtype=torch.uint8, device="cuda")
+    assert lib("tc").fg_gemm_f32_tc(ptr(a), K, ptr(w), K, ptr(want), N, 0, M, N, K, ptr(ws), low - 1, stream()) == 10002
+
+
 def test_gemm_f32_on_planes_refuses_other_sizes():
     from fastgguf_b200.ops import fast_gemm
     for M, N, K in ((16, 512, 1024), (64, 256, 1024), (100, 128, 1024), (100, 512, 256), (100, 512, 1028)):
