@@ -16,7 +16,13 @@
 // Q K^T.  Two CTAs an SM at head size 64 (101 KB of shared memory, 256 threads), one at 128 (169 KB, 512 threads).
 // One layer of Llama 1B, 2,048 tokens: 5,583 -> 723 us (24 TFLOP/s).  Eight rows a thread read shared memory less often but leave
 // two warps a scheduler: 772 us.
-// A row's keys are visited in ascending page order, so its result does not depend on the other rows of the step.
+// A row's keys are visited in ascending page order, so its result does not depend on the other rows of a CTA.
+//
+// A CTA walks its pages alone, 10.4 us a page at head size 64 and 16 at 128, whatever it has of rows; the any-size kernel spreads the
+// (row, head) pairs over the GPU, 83 ns and 165 ns for 1,000 keys of a pair.  So a sequence with few new tokens is the any-size
+// kernel's, however long its past is (us, this kernel : any-size, 32 heads of 64): 1 token behind 4,000 keys 664 : 78, 16 tokens 665 :
+// 204, 64 tokens 676 : 709, 128 tokens 693 : 1,398; no past, 64 tokens 20 : 22, 128 tokens 30 : 49.  24 heads of 128: 32 tokens behind 4,000
+// keys 1,012 : 595, 64 tokens 1,029 : 1,075.
 #include "common.cuh"
 
 #define PAGE 64
@@ -27,6 +33,13 @@ __device__ __forceinline__ void f32_cp_async16(float *dst, const float *src) {
 }
 __device__ __forceinline__ void f32_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void f32_cp_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+
+// Whether the any-size kernel is the faster one for a sequence alone: its work, tokens x heads x the keys a token sees on average, against
+// the keys that a tile's walk passes, by the times above.
+__host__ __device__ __forceinline__ bool f32_few_rows(int tokens, int past, int heads, int hd, int window) {
+    const long long keys = window ? (long long)min(past, window > 0 ? window : -window) : past;
+    return (long long)tokens * heads * (2 * keys + tokens) < (hd == 64 ? 2048LL : 1536LL) * 2 * (keys + tokens);
+}
 
 template <int HD> struct PrefillF32 {
     static constexpr int RPT = 4, TX = HD / 8, THREADS = ROWS / RPT * TX, NK = PAGE / TX;       // rows a thread, lanes a row, threads, keys a thread
@@ -39,7 +52,7 @@ template <int HD>
 __global__ void __launch_bounds__(PrefillF32<HD>::THREADS, HD == 64 ? 2 : 1)
 attn_prefill_f32_kernel(const float *__restrict__ q, int ldq, float *__restrict__ out, int ldo, const int *__restrict__ cu_rows,
                         const int *__restrict__ seq_start, const int *__restrict__ block_table, int table_width,
-                        const float *__restrict__ k_pool, const float *__restrict__ v_pool, int KV, int G, float scale, int window) {
+                        const float *__restrict__ k_pool, const float *__restrict__ v_pool, int KV, int G, float scale, int window, int skip_few) {
     using C = PrefillF32<HD>;
     constexpr int RPT = C::RPT, TX = C::TX, NT = C::THREADS, NK = C::NK, LDQ = C::LDQ, LDK = C::LDK;
     extern __shared__ __align__(16) float fsm[];
@@ -49,7 +62,7 @@ attn_prefill_f32_kernel(const float *__restrict__ q, int ldq, float *__restrict_
     const int kvh = blockIdx.y / chunks, g0 = (blockIdx.y % chunks) * Gc, b = blockIdx.z;
     const int row0 = cu_rows[b], n_tok = cu_rows[b + 1] - row0, start = seq_start[b];
     const int q0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * TQ;          // late tiles see the most keys: they start first
-    if (q0 >= n_tok) return;
+    if (q0 >= n_tok || (skip_few && f32_few_rows(n_tok, start, KV * G, HD, window))) return;
     const int tq = min(TQ, n_tok - q0);
     const int *bt = block_table + (size_t)b * table_width;
     const size_t H_row = (size_t)kvh * G + g0;                           // the first query head of this CTA
@@ -221,7 +234,7 @@ attn_prefill_f32_kernel(const float *__restrict__ q, int ldq, float *__restrict_
 template <int HD>
 static int launch_prefill_f32(const float *q, int ldq, float *out, int ldo, const int *cu_rows, const int *seq_start,
                               const int *block_table, int table_width, const float *k_pool, const float *v_pool, int n_seq,
-                              int max_new, int H, int KV, float scale, int window, cudaStream_t stream) {
+                              int max_new, int H, int KV, float scale, int window, int skip_few, cudaStream_t stream) {
     static FgPerDevice configured;
     if (fg_needs_setup(configured)) {
         cudaError_t e = cudaFuncSetAttribute(attn_prefill_f32_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, PrefillF32<HD>::SMEM);
@@ -231,23 +244,46 @@ static int launch_prefill_f32(const float *q, int ldq, float *out, int ldo, cons
     dim3 grid((max_new + TQ - 1) / TQ, KV * ((G + Gc - 1) / Gc), n_seq);
     if (grid.y > 65535) return FG_ERR_BAD_SIZE;
     return fg_launch_in_order(attn_prefill_f32_kernel<HD>, grid, dim3(PrefillF32<HD>::THREADS), (size_t)PrefillF32<HD>::SMEM, stream, q, ldq,
-                              out, ldo, cu_rows, seq_start, block_table, table_width, k_pool, v_pool, KV, G, scale, window);
+                              out, ldo, cu_rows, seq_start, block_table, table_width, k_pool, v_pool, KV, G, scale, window, skip_few);
 }
 
 // q: [rows, ldq] float32 rows of all sequences one after another (cu_rows[b] = first row of sequence b, seq_start[b] = its length
 // before the step); pools [pages, KV, 64, hd] float32; out [rows, ldo] float32.  max_new: most rows any sequence brings.
+// skip_few: sequences that fg_attention_f32_few_rows names are left out (the any-size kernel has them).
 // Refuses (FG_ERR_BAD_SIZE) other head sizes and pages and rows that are not 16-byte aligned; the any-size kernel takes those.
-extern "C" int fg_attention_prefill_f32(const void *q, int ldq, void *out, int ldo, const int *cu_rows, const int *seq_start,
-                                        const int *block_table, int table_width, const void *k_pool, const void *v_pool, int n_seq,
-                                        int max_new, int H, int KV, int hd, int page_size, float scale, int window, cudaStream_t stream) {
+extern "C" int fg_attention_prefill_f32_ext(const void *q, int ldq, void *out, int ldo, const int *cu_rows, const int *seq_start,
+                                            const int *block_table, int table_width, const void *k_pool, const void *v_pool, int n_seq,
+                                            int max_new, int H, int KV, int hd, int page_size, float scale, int window, int skip_few,
+                                            cudaStream_t stream) {
     if (n_seq <= 0 || max_new <= 0) return 0;
     if (page_size != PAGE || KV <= 0 || H % KV || n_seq > 65535 || ldq % 4 || ldo % 4 ||
         (((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_pool | (uintptr_t)v_pool) & 15))
         return FG_ERR_BAD_SIZE;
 #define PF32_RUN(HD) launch_prefill_f32<HD>((const float *)q, ldq, (float *)out, ldo, cu_rows, seq_start, block_table, table_width, \
-                                            (const float *)k_pool, (const float *)v_pool, n_seq, max_new, H, KV, scale, window, stream)
+                                            (const float *)k_pool, (const float *)v_pool, n_seq, max_new, H, KV, scale, window, skip_few, stream)
     if (hd == 64) return PF32_RUN(64);
     if (hd == 128) return PF32_RUN(128);
 #undef PF32_RUN
     return FG_ERR_BAD_SIZE;
+}
+
+extern "C" int fg_attention_prefill_f32(const void *q, int ldq, void *out, int ldo, const int *cu_rows, const int *seq_start,
+                                        const int *block_table, int table_width, const void *k_pool, const void *v_pool, int n_seq,
+                                        int max_new, int H, int KV, int hd, int page_size, float scale, int window, cudaStream_t stream) {
+    return fg_attention_prefill_f32_ext(q, ldq, out, ldo, cu_rows, seq_start, block_table, table_width, k_pool, v_pool, n_seq, max_new, H, KV, hd,
+                                        page_size, scale, window, 0, stream);
+}
+
+extern "C" int fg_attention_f32_few_rows(int tokens, int past, int heads, int hd, int window) { return f32_few_rows(tokens, past, heads, hd, window); }
+
+// Pages of 64 keys that the longest tile of a sequence walks (*walk), and the times of both kernels in such walks: of the any-size kernel
+// (*any_size) and of all the sequence's tiles on a GPU of n_sm SMs (*tiles).
+extern "C" int fg_attention_f32_cost(int tokens, int past, int H, int KV, int hd, int window, int n_sm, double *any_size, double *tiles, double *walk) {
+    const double keys = window ? min(past, window > 0 ? window : -window) : past, seen = keys + 0.5 * tokens;
+    const int G = H / KV, Gc = G < 16 ? G : 16, TQ = ROWS / Gc;
+    const double ctas = (double)((tokens + TQ - 1) / TQ) * KV * ((G + Gc - 1) / Gc);
+    *walk = (keys + tokens) / PAGE + 1.0;
+    *any_size = (double)tokens * H * seen / PAGE / (hd == 64 ? 2048.0 : 1536.0);
+    *tiles = ctas * (seen / PAGE + 1.0) / (hd == 64 ? 2 * n_sm : n_sm);
+    return 0;
 }

@@ -80,6 +80,12 @@ int fg_attention_generic(const void *q, int ldq, void *out, int ldo, int dtype, 
 int fg_attention_prefill_f32(const void *q, int ldq, void *out, int ldo, const int *cu_rows, const int *seq_start,
                              const int *block_table, int table_width, const void *k_pool, const void *v_pool, int n_seq,
                              int max_new, int H, int KV, int hd, int page_size, float scale, int window, cudaStream_t stream);
+/* the same with skip_few: without the sequences that fg_attention_f32_few_rows names (few new tokens, see there); and what each kernel takes */
+int fg_attention_prefill_f32_ext(const void *q, int ldq, void *out, int ldo, const int *cu_rows, const int *seq_start,
+                                 const int *block_table, int table_width, const void *k_pool, const void *v_pool, int n_seq,
+                                 int max_new, int H, int KV, int hd, int page_size, float scale, int window, int skip_few, cudaStream_t stream);
+int fg_attention_f32_few_rows(int tokens, int past, int heads, int hd, int window);
+int fg_attention_f32_cost(int tokens, int past, int H, int KV, int hd, int window, int n_sm, double *any_size, double *tiles, double *walk);
 /* the same with values of head size hdv and, with a window, the sequence's first keep_first keys visible as well */
 /* softcap > 0: scores capped by softcap * tanh(score / softcap); sinks: a float per query head that joins the softmax's denominator;
    latent: the cache holds a latent (v_pool, hdv numbers, also the value) and a rotated key part (k_pool, hd numbers) a position,

@@ -298,6 +298,42 @@ static bool fast_attention_ok(const Runtime &rt, const Tensor &q, const LayerIO 
            a.v_head_dim == a.head_dim && io.page_size == 64 && q.ld % 2 == 0 && ((uintptr_t)q.data % 4) == 0;
 }
 
+// Float32 prompts: tiles of 128 rows that share the keys they read, or the any-size kernel's block a (row, head).  Which one a sequence's rows
+// take: a sequence with few new tokens is the any-size kernel's (attention_prefill_f32.cu has the figures), unless the step has so many of
+// them that their tiles, which run side by side, are done first.
+struct F32AttentionSplit {
+    bool tiles = false;                              // the tiled kernel runs
+    std::vector<std::pair<int, int>> any_size;       // (first row, rows) of the runs it leaves to the any-size kernel
+};
+static F32AttentionSplit split_f32_attention(const Batch &b, int H, int KV, int hd, int window, int n_sm) {
+    F32AttentionSplit s;
+    if ((int)b.host_cu_rows.size() <= b.n_seq || (int)b.host_seq_start.size() < b.n_seq) {      // the host does not know the lengths
+        s.tiles = (long long)b.max_new * H >= 4096;
+        return s;
+    }
+    double few_any = 0.0, few_tiles = 0.0, few_walk = 0.0, many_tiles = 0.0, many_walk = 0.0;
+    for (int i = 0; i < b.n_seq; i++) {
+        const int row0 = b.host_cu_rows[(size_t)i], n = b.host_cu_rows[(size_t)i + 1] - row0, past = b.host_seq_start[(size_t)i];
+        if (n <= 0) continue;
+        double any = 0.0, tiles = 0.0, walk = 0.0;
+        FG_KERNEL("core", fg_attention_f32_cost)(n, past, H, KV, hd, window, n_sm, &any, &tiles, &walk);
+        if (FG_KERNEL("core", fg_attention_f32_few_rows)(n, past, H, hd, window)) {
+            few_any += any;
+            few_tiles += tiles;
+            few_walk = std::max(few_walk, walk);
+            if (!s.any_size.empty() && s.any_size.back().first + s.any_size.back().second == row0) s.any_size.back().second += n;
+            else s.any_size.emplace_back(row0, n);
+        } else {
+            many_tiles += tiles;
+            many_walk = std::max(many_walk, walk);
+        }
+    }
+    const double many = std::max(many_walk, many_tiles), all = std::max(std::max(many_walk, few_walk), many_tiles + few_tiles);
+    if (all - many <= few_any + 1.2 * (double)s.any_size.size()) s.any_size.clear();     // (1.2: a launch of the any-size kernel, at least 12 us)
+    s.tiles = many_walk > 0.0 || (s.any_size.empty() && few_walk > 0.0);
+    return s;
+}
+
 static Tensor attention(Runtime &rt, const Tensor &q, const Batch &b, const LayerIO &io, const AttentionShape &a) {
     const int H = a.n_heads, KV = a.n_kv_heads, hd = a.head_dim;
     const int *table = b.block_tables.at((size_t)io.group);
@@ -329,25 +365,34 @@ static Tensor attention(Runtime &rt, const Tensor &q, const Batch &b, const Laye
         return out;
     }
     if (q.dtype != io.cache_dtype) fail(FG_E_INTERNAL, "attention: q and the cache must share a dtype");
-    // Float32 with 64 and more (token, head of a group) rows a sequence: tiles of 128 rows that share the keys they read.  Fewer
-    // rows leave most of a tile idle, and a block a row keeps more of the GPU busy.
-    if (!rt.plain_kernels && q.dtype == FG_F32 && a.v_head_dim == hd && (hd == 64 || hd == 128) && io.page_size == 64 &&
-        !(a.window > 0 && a.keep_first > 0) && b.max_new * (H / KV) >= 64) {
-        count_launch();
-        ProfileScope scope("fg_attention_prefill_f32");
-        int code = FG_KERNEL("core", fg_attention_prefill_f32)(q.data, (int)q.ld, out.data, (int)out.ld, b.cu_rows, b.seq_start, table, b.table_width,
-                                                               io.k_pool, io.v_pool, b.n_seq, b.max_new, H, KV, hd, io.page_size, a.scale, a.window,
-                                                               rt.stream);
-        if (code != KERNEL_BAD_SIZE) {
-            check_kernel(code, "fg_attention_prefill_f32");
-            return out;
+    auto any_size = [&](int row0, int rows) {
+        const int es = elem_size(q.dtype);
+        FG_LAUNCH("core", fg_attention_generic_kept, (const char *)q.data + (size_t)row0 * q.ld * es, (int)q.ld, (char *)out.data + (size_t)row0 * out.ld * es,
+                  (int)out.ld, q.dtype, b.positions + row0, b.row_seq + row0, table, b.table_width, io.k_pool, io.v_pool, rows, H, KV, hd, a.v_head_dim,
+                  io.page_size, a.scale, a.window, a.keep_first, rt.stream);
+    };
+    if (!rt.plain_kernels && !b.single_token && q.dtype == FG_F32 && a.v_head_dim == hd && (hd == 64 || hd == 128) && io.page_size == 64 &&
+        !(a.window > 0 && a.keep_first > 0)) {
+        const F32AttentionSplit split = split_f32_attention(b, H, KV, hd, a.window, rt.n_sm);
+        if (split.tiles) {
+            count_launch();
+            int code;
+            {
+                ProfileScope scope("fg_attention_prefill_f32");
+                code = FG_KERNEL("core", fg_attention_prefill_f32_ext)(q.data, (int)q.ld, out.data, (int)out.ld, b.cu_rows, b.seq_start, table, b.table_width,
+                                                                       io.k_pool, io.v_pool, b.n_seq, b.max_new, H, KV, hd, io.page_size, a.scale, a.window,
+                                                                       split.any_size.empty() ? 0 : 1, rt.stream);
+            }
+            if (code != KERNEL_BAD_SIZE) {
+                check_kernel(code, "fg_attention_prefill_f32");
+                for (auto &run : split.any_size) any_size(run.first, run.second);
+                return out;
+            }
         }
     }
     if (hd > 256 || a.v_head_dim > 256)
         fail(FG_E_KERNEL, format("attention: head size %d / %d exceeds 256, the largest the any-size kernel takes", hd, a.v_head_dim));
-    FG_LAUNCH("core", fg_attention_generic_kept, q.data, (int)q.ld, out.data, (int)out.ld, q.dtype, b.positions, b.row_seq, table,
-              b.table_width, io.k_pool, io.v_pool, (int)q.rows, H, KV, hd, a.v_head_dim, io.page_size, a.scale, a.window, a.keep_first,
-              rt.stream);
+    any_size(0, (int)q.rows);
     return out;
 }
 

@@ -180,3 +180,33 @@ def test_float32_scratch_memory_is_shared_by_the_steps_of_an_engine():
     assert max(grown) < 150, grown
     again = held(20, 0.0)
     assert again[0] == first[0]
+
+
+def test_float32_steps_of_prompts_beside_running_sequences():
+    """In a float32 step that brings a prompt and the next tokens of other sequences, the prompt's rows take the tiled attention kernel and the
+    single tokens the any-size one, runs of them between prompts included; the logits are those of the sequences alone."""
+    from helpers import TINY_B
+    from fastgguf_b200 import StepEntry
+    from fastgguf_b200.engine.api import Engine
+    from fastgguf_b200.registry import config_from_dict
+    cfg = dict(TINY_B, hidden_size=512, num_attention_heads=16, num_key_value_heads=4, head_dim=64, intermediate_size=1024, num_hidden_layers=2, max_position_embeddings=4096)
+    eng = Engine.from_random(config_from_dict(cfg), 3, dtype="float32", max_tokens=16384, max_batch=8, max_seq_len=4096)
+    rng = np.random.default_rng(5)
+    draw = lambda n: [int(t) for t in rng.integers(0, cfg["vocab_size"], size=n)]  # noqa: E731
+    running, prompts = [draw(1500), draw(70), draw(2900)], [draw(400), draw(333)]
+    slots = [eng.acquire() for _ in running]
+    eng.step_host([StepEntry(s, t[:-1], []) for s, t in zip(slots, running)])
+    new = [eng.acquire() for _ in prompts]
+    one = lambda i: StepEntry(slots[i], running[i][-1:], [0])  # noqa: E731
+    whole = lambda i: StepEntry(new[i], prompts[i], [len(prompts[i]) - 1])  # noqa: E731
+    eng.profile(True)
+    got = eng.step_host([one(0), whole(0), one(1), one(2), whole(1)])
+    calls = {r["name"].split(" ")[0]: r["calls"] for r in eng.profile_report()}
+    eng.profile(False)
+    layers = 2
+    assert calls["fg_attention_prefill_f32"] == layers and calls["fg_attention_generic_kept"] == 2 * layers
+    for logits, toks in zip(got, [running[0], prompts[0], running[1], running[2], prompts[1]]):
+        s = eng.acquire()
+        alone = eng.step_host([StepEntry(s, toks, [len(toks) - 1])])[0]
+        eng.release(s)
+        assert np.abs(logits - alone).max() <= 2e-5 * np.abs(alone).max()

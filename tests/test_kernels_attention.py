@@ -132,6 +132,31 @@ def test_attention_prefill_f32(H, KV, hd, window):
     assert torch.equal(bad[:150], got[:150]) and torch.equal(bad[200:], got[200:])
 
 
+def test_attention_prefill_f32_leaves_out_sequences_of_few_rows():
+    """With skip_few the rows of every sequence that the rule names keep what the output held, all others have their values."""
+    import ctypes
+    from fastgguf_b200.ops import fast_attention
+    from fastgguf_b200.ops.lib import lib, ptr, stream
+    H, KV, hd = 32, 8, 64
+    before, new = [0, 300, 2000, 0, 700, 64], [200, 1, 70, 40, 130, 63]
+    case = make_case(before, new, H, KV, hd, torch.float32, 14)
+    few = [bool(lib("core").fg_attention_f32_few_rows(n, p, H, hd, 0)) for n, p in zip(new, before)]
+    assert few == [False, True, False, True, False, True]
+    q, scale = case["q"], 1.0 / math.sqrt(hd)
+    want = fast_attention.attention_prefill_f32(q, case["cu_rows"], case["seq_start"], case["table"], case["k_pool"], case["v_pool"], len(new), max(new),
+                                                H, KV, hd, scale, 0)
+    out = torch.full_like(want, 9.0)
+    f = ctypes.c_float
+    assert lib("core").fg_attention_prefill_f32_ext(ptr(q), q.stride(0), ptr(out), out.stride(0), ptr(case["cu_rows"]), ptr(case["seq_start"]),
+                                                    ptr(case["table"]), case["table"].shape[1], ptr(case["k_pool"]), ptr(case["v_pool"]), len(new),
+                                                    max(new), H, KV, hd, 64, f(scale), 0, 1, stream()) == 0
+    at = 0
+    for n, left_out in zip(new, few):
+        rows = out[at:at + n]
+        assert (rows == 9.0).all() if left_out else torch.equal(rows, want[at:at + n])
+        at += n
+
+
 @pytest.mark.parametrize("n_splits", [None, 1, 2, 3, 8, 16])
 @pytest.mark.parametrize("H,KV,hd,window", [(8, 2, 64, 0), (3, 1, 128, 0), (24, 8, 128, 0), (20, 1, 64, 0),
                                             (4, 4, 64, 100), (4, 2, 64, 64), (4, 2, 64, 128), (8, 2, 64, 65),
