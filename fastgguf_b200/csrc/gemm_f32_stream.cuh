@@ -11,8 +11,8 @@
 //                same number of bytes
 //   two CTAs an SM, seven warps of sums each: with one, every warp's read of the activations from shared memory stood in
 //                line with its multiplications (gate/up at 8 rows 31.8 us, with two 25.5; down 27.4, with two 19.3)
-// 8 rows of Llama 1B (us, against gemm_generic.cu): gate/up 25.5 (5.3 TB/s) : 49.2, down 19.3 : 25.6, head 171 (6.1 TB/s) : 312; 16 rows,
-// where the multiplications bound it: 51 : 79, 33 : 49, 370 : 510; one row: 20.8 : 28.3, 17.3 : 16.6, 150 : 162.
+// 8 rows of Llama 1B (us, against gemm_generic.cu): gate/up 25.1 (5.3 TB/s) : 49.2, down 18.7 : 25.6, head 171 to 189 (5.6 to 6.1 TB/s) : 312; 16
+// rows, where the multiplications bound it: 51 : 79, 33 : 49, 370 to 394 : 510; one row: 20.7 (6.5 TB/s) : 28.3, 16.3 : 16.6, 149 (7.0 TB/s) : 162.
 #pragma once
 
 #define FST_WARPS 7                        // warps that compute; one more feeds the ring

@@ -1,7 +1,7 @@
 // Plain tiled contraction C[m, n] = sum_k A[m, k] * W[n, k] on the FMA units, f32 accumulation.
 //
-// This is the true 32-bit path of every projection (no tensor cores, no TF32, no reduced
-// precision anywhere) and the any-size fallback of the bf16 path.  Three kernels by row count: a
+// The plain chain of multiplications and additions: the any-size fallback of both paths, everything under FASTGGUF_PLAIN_KERNELS=1, and the
+// 32-bit path's small matrices (larger ones: gemm_f32_stream.cuh up to 16 rows, gemm_f32_tc.cuh beyond).  Three kernels by row count: a
 // weight-streaming one for up to 16 rows (a decode step; up to 64 rows of a small matrix), 64 x 64 tiles up to 64 rows, 128 x 128
 // tiles beyond.  In each the order of additions for an output depends on K alone, so a row's result
 // does not depend on how many other rows are in the batch; between the kernels the order differs
@@ -329,8 +329,11 @@ extern "C" int fg_gemm_generic_step(const void *A, int a_dtype, int lda, const v
     if (accumulate && out_dtype != FG_F32) return FG_ERR_BAD_DTYPE;
     // few rows and weight rows that 16-byte (f32) / 8-byte (bf16) loads can walk: the weight-streaming kernel
     const int w_bytes = w_dtype == FG_F32 ? 4 : 2;
-    // Up to 64 rows of a small matrix go there too, 16 rows a block: the 64 x 64 tiles below are one or two blocks then, whose
-    // walk along K waits for every load (39 rows x 64 x 192: 23 us, 16 rows a block 4.2).
+    // Up to 64 rows of a small matrix go there too, 16 rows a block: the 64 x 64 tiles below are a few blocks then, whose walk along K waits
+    // for every load.  By 16 rows against tiles, us alone, float32 (bfloat16): 39 rows of 64 x 192 2.2 : 23; 17 rows of 768 x 512 7 : 51 (12 : 51),
+    // 64 rows 13 : 52 (23 : 52); 64 rows of 1,024 x 1,024 19 : 104 (37 : 103), of 2,048 x 2,048 59 : 205 (84 : 205).  The line lies at 2^18 numbers because
+    // beyond it the kernels that run by default are others: float32 by planes at 18 us whatever the rows (64 rows of 1,024 x 1,024 17, of
+    // 2,048 x 2,048 27), bfloat16 on the tensor cores; what still comes here has rows those refuse, and keeps the order of the tiles.
     if ((M <= 16 || (M <= 64 && (long long)N * K <= 1 << 18)) && K % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)W % (4 * w_bytes)) == 0) {
         int e = FG_ERR_BAD_DTYPE;
         if (a_dtype == FG_F32 && w_dtype == FG_F32) e = launch_gemv<float, float>(A, lda, W, ldw, C, ldc, out_dtype, accumulate, M, N, K, early, stream);

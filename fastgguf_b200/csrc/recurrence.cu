@@ -289,8 +289,10 @@ gated_group_norm_kernel(const float *__restrict__ y, int ldy, const float *__res
     TO *orow = out + (size_t)m * ldo;
     const bool whole = w_period >= C, by_group = w_period == group;
     // Few rows: a group that fits the registers of its threads (the block, or a warp for narrow ones) is read once, all of it in
-    // flight together (8 rows of 2,048 9.7 -> 6.2 us); the sums are those of the loops below, which are faster where many rows hide
-    // each other's latency (4,925 rows: 42 us, this way 49).
+    // flight together.  In a step, where its rows come from memory, 8 rows of 2,048 9.7 -> 6.2 us; the sums are those of the loops below.  Alone,
+    // with everything in L2 (registers against loops, us): one group of 2,048 3.4 : 4.6 up to 64 rows, 3.7 : 4.8 at 256, 5.3 : 5.3 at 512, 33 : 34 at
+    // 4,925; groups of 128 of 2,048 5.5 : 4.3 up to 96 rows, 9.0 : 4.9 at 512, 60 : 33 at 4,925.  Narrow groups' loops would win alone, but not in
+    // a step (Saluzen's decode case 35.09 ms this way, 35.18 with loops for narrow groups).
     const bool wide = group >= 1024;
     const int step = wide ? 256 : 32, lane0 = wide ? (int)threadIdx.x : lane;
     if (FEW && group <= step * REC_KEEP) {
@@ -363,8 +365,10 @@ extern "C" int fg_conv1d_silu(const float *in, int ld, const float *w, const flo
                               int M, int C, cudaStream_t stream) {
     if (M <= 0) return 0;
     if (C <= 0 || taps <= 0 || (taps > 1 && !state)) return FG_ERR_BAD_SIZE;
-    // With few rows latency counts: the weights come before the wait on the preceding kernel and a channel's inputs together
-    // (8 rows of 4,096 channels 10.3 -> 7.3 us); with many, fewer registers a thread do (4,925 rows 126 us, the other way 138).
+    // With few rows latency counts: the weights come before the wait on the preceding kernel and a channel's inputs together.  That pays in
+    // a step, where the weights come from memory (8 rows of 4,096 channels 10.3 -> 7.3 us); alone, with everything in L2, the plain form is as
+    // fast (8 rows 4.1 us against 5.1, 64 rows 4.6 against 5.5) and leaves the other behind as the rows grow (256 rows 8.2 against 10.7, 4,925 rows
+    // 128 against 297), so the line lies where a step stops being a decode step.
     return fg_launch(M <= 64 ? conv1d_silu_kernel<true> : conv1d_silu_kernel<false>, dim3(M, (C + 1023) / 1024), dim3(256), 0, stream, in, ld, w, bias,
                      taps, state, state_stride, row_seq, cu_rows, slots, out, ldo, C);
 }
