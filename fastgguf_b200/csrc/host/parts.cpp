@@ -311,13 +311,15 @@ static F32AttentionSplit split_f32_attention(const Batch &b, int H, int KV, int 
         s.tiles = (long long)b.max_new * H >= 4096;
         return s;
     }
+    const auto cost = FG_KERNEL("core", fg_attention_f32_cost);            // (looked up once: a step of many sequences asks often)
+    const auto few_rows = FG_KERNEL("core", fg_attention_f32_few_rows);
     double few_any = 0.0, few_tiles = 0.0, few_walk = 0.0, many_tiles = 0.0, many_walk = 0.0;
     for (int i = 0; i < b.n_seq; i++) {
         const int row0 = b.host_cu_rows[(size_t)i], n = b.host_cu_rows[(size_t)i + 1] - row0, past = b.host_seq_start[(size_t)i];
         if (n <= 0) continue;
         double any = 0.0, tiles = 0.0, walk = 0.0;
-        FG_KERNEL("core", fg_attention_f32_cost)(n, past, H, KV, hd, window, n_sm, &any, &tiles, &walk);
-        if (FG_KERNEL("core", fg_attention_f32_few_rows)(n, past, H, hd, window)) {
+        cost(n, past, H, KV, hd, window, n_sm, &any, &tiles, &walk);
+        if (few_rows(n, past, H, hd, window)) {
             few_any += any;
             few_tiles += tiles;
             few_walk = std::max(few_walk, walk);
