@@ -54,8 +54,8 @@ MODELS = {"1b": ("Llama-3.2-1B shapes", LLAMA_3_2_1B), "3b": ("Llama-3.2-3B shap
 WORKLOADS = {"1b": (4096, 128, 1024), "3b": (4096, 64, 2048), "8b": (8192, 7168, 7680)}
 PREFILL_TOKENS = 2048
 REPEATS = 5
-#: peak of the FP32 FMA units: 148 SMs x 128 lanes x 2 flops at the maximum SM clock (no measured figure exists)
-FP32_TFLOPS = 148 * 128 * 2 * 1.965e9 / 1e12
+#: a float32 product on the tensor cores is six bfloat16 products (csrc/gemm_f32_tc.cuh): what they leave of the measured bfloat16 rate
+FP32_PRODUCTS = 6
 FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0}
 
 
@@ -556,11 +556,11 @@ def main():
                 times.append(t0.elapsed_time(t1))
         pms = sorted(times)[len(times) // 2]
         fl = prefill_flops(c, layers, PREFILL_TOKENS)
-        peak = FP32_TFLOPS if f32 else pk["bf16_tflops"]
+        peak = pk["bf16_tflops"] / (FP32_PRODUCTS if f32 else 1)
         rec["prefill"] = {"value": round(PREFILL_TOKENS / (pms * 1e-3), 1), "tokens": PREFILL_TOKENS, "ms": round(pms, 3),
                           "frac": round(fl / (pms * 1e-3) / 1e12 / peak, 4)}
         if f32:
-            rec["prefill"]["peak_tflops"] = round(FP32_TFLOPS, 1)
+            rec["prefill"]["peak_tflops"] = round(peak, 1)
     if points_at:
         points, detail = {}, {}
         for b in points_at:

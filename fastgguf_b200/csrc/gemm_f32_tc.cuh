@@ -21,9 +21,9 @@
 //   gemm_f32_finish_kernel  adds the parts of a contraction that is split along K (few output tiles), in split order
 //
 // Distance from float64 (2-norm, normal operands, 600 rows): 1.1e-7 at K = 2,048 and 1.5e-7 at 8,192, where the chain of fused multiply-adds
-// has 8.1e-7 and 1.6e-6.  Times with the planes' making, against gemm_tile128_kernel (us): 2,048 rows x 16,384 x 2,048: 554 against
-// 3,175 (248 TFLOP/s; a sixth of the bfloat16 burst rate is 270); 2,048 x 2,048 x 8,192: 306 against 1,747; 600 x 2,048 x 8,192: 143
-// against 1,249; 24 x 2,048 x 2,048: 38 against 210.
+// has 8.1e-7 and 1.6e-6.  Times with the planes' making, against gemm_tile128_kernel (us): 2,048 rows x 16,384 x 2,048: 566 against
+// 3,175 (243 TFLOP/s; a sixth of the bfloat16 burst rate is 270); 2,048 x 2,048 x 8,192: 314 against 1,747; 600 x 2,048 x 8,192: 144
+// against 1,249; 24 x 2,048 x 2,048: 28 (the kernels alone) against 205.
 //
 // Two kinds of outputs are computed by the plain chain of fused multiply-adds over the float32 operands, a warp for a tile of 32 x 32:
 // those that come out as no finite number (infinities and NaN among the operands), and those whose rows are so large that the plain
