@@ -210,3 +210,47 @@ def test_float32_steps_of_prompts_beside_running_sequences():
         alone = eng.step_host([StepEntry(s, toks, [len(toks) - 1])])[0]
         eng.release(s)
         assert np.abs(logits - alone).max() <= 2e-5 * np.abs(alone).max()
+
+
+def test_float32_steps_where_device_memory_is_short():
+    """Without room for all of the scratch memory a float32 step takes its operands in more portions, with the same bits; without room for the
+    least of it the plain chain computes the step."""
+    import gc
+    from helpers import TINY_B
+    from fastgguf_b200 import StepEntry
+    from fastgguf_b200.engine.api import Engine
+    from fastgguf_b200.registry import config_from_dict
+    cfg = dict(TINY_B, hidden_size=1024, num_attention_heads=16, num_key_value_heads=4, head_dim=64, intermediate_size=2048, vocab_size=32000)
+    rng = np.random.default_rng(5)
+    toks = [int(t) for t in rng.integers(0, 32000, size=40)]
+
+    def logits(left):
+        """of every place of a prompt, in an engine that has `left` bytes of device memory left (None: all of it); the head's planes are 188 MB"""
+        eng = Engine.from_random(config_from_dict(cfg), 3, dtype="float32", max_tokens=1024, max_batch=2)
+        s = eng.acquire()
+        eng.step_host([StepEntry(s, toks[:8], [7])])       # (activations, modules; eight rows need no scratch memory)
+        eng.release(s)
+        hold = None
+        if left is not None:
+            torch.cuda.synchronize()
+            hold = torch.empty(torch.cuda.mem_get_info()[0] - left, dtype=torch.uint8, device="cuda")
+        try:
+            eng.profile(True)
+            s = eng.acquire()
+            got = np.array(eng.step_host([StepEntry(s, toks, list(range(40)))]))
+            names = {r["name"] for r in eng.profile_report()}
+            eng.profile(False)
+        finally:
+            del hold
+            torch.cuda.empty_cache()
+        del eng
+        gc.collect()
+        return got, any(n.startswith("fg_gemm_f32_tc") for n in names)
+
+    gib = 1 << 30
+    want, planes = logits(None)
+    assert planes
+    portions, planes = logits(gib + (120 << 20))
+    assert planes and np.array_equal(portions, want)
+    plain, planes = logits(gib - (100 << 20))
+    assert not planes and 0 < np.abs(plain - want).max() <= 1e-5 * np.abs(want).max()
