@@ -136,7 +136,7 @@ void *kernel_symbol(const char *module, const char *name) {
 }
 
 void raise_on_device_error(const char *where) {
-    static const char *flags[][2] = {{"tc", "fg_gemm_tc_error"}, {"attn", "fg_attention_prefill_tc_error"}};
+    static const char *flags[][2] = {{"tc", "fg_gemm_tc_error"}, {"attn", "fg_attention_prefill_tc_error"}, {"core", "fg_attention_prefill_f32_error"}};
     for (auto &f : flags) {
         void *h = nullptr;
         {

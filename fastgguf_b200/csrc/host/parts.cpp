@@ -312,7 +312,7 @@ static F32AttentionSplit split_f32_attention(const Batch &b, int H, int KV, int 
         return s;
     }
     const auto cost = FG_KERNEL("core", fg_attention_f32_cost);            // (looked up once: a step of many sequences asks often)
-    const auto few_rows = FG_KERNEL("core", fg_attention_f32_few_rows);
+    const auto few_rows = FG_KERNEL("core", fg_attention_f32_left_out);
     double few_any = 0.0, few_tiles = 0.0, few_walk = 0.0, many_tiles = 0.0, many_walk = 0.0;
     for (int i = 0; i < b.n_seq; i++) {
         const int row0 = b.host_cu_rows[(size_t)i], n = b.host_cu_rows[(size_t)i + 1] - row0, past = b.host_seq_start[(size_t)i];
@@ -331,7 +331,7 @@ static F32AttentionSplit split_f32_attention(const Batch &b, int H, int KV, int 
         }
     }
     const double many = std::max(many_walk, many_tiles), all = std::max(std::max(many_walk, few_walk), many_tiles + few_tiles);
-    if (all - many <= few_any + 1.2 * (double)s.any_size.size()) s.any_size.clear();     // (1.2: a launch of the any-size kernel, at least 12 us)
+    if (all - many <= few_any + 3.5 * (double)s.any_size.size()) s.any_size.clear();     // (3.5: a launch of the any-size kernel, at least 12 us)
     s.tiles = many_walk > 0.0 || (s.any_size.empty() && few_walk > 0.0);
     return s;
 }
@@ -383,7 +383,7 @@ static Tensor attention(Runtime &rt, const Tensor &q, const Batch &b, const Laye
                 ProfileScope scope("fg_attention_prefill_f32");
                 code = FG_KERNEL("core", fg_attention_prefill_f32_ext)(q.data, (int)q.ld, out.data, (int)out.ld, b.cu_rows, b.seq_start, table, b.table_width,
                                                                        io.k_pool, io.v_pool, b.n_seq, b.max_new, H, KV, hd, io.page_size, a.scale, a.window,
-                                                                       split.any_size.empty() ? 0 : 1, rt.stream);
+                                                                       split.any_size.empty() ? 0 : FG_KERNEL("core", fg_attention_f32_skip_few)(hd), rt.stream);
             }
             if (code != KERNEL_BAD_SIZE) {
                 check_kernel(code, "fg_attention_prefill_f32");

@@ -96,7 +96,7 @@ def attention_prefill(q, cu_rows, seq_start, block_table, k_pool, v_pool, n_seq,
 
 def attention_prefill_f32(q, cu_rows, seq_start, block_table, k_pool, v_pool, n_seq, max_new, n_heads, n_kv_heads,
                           head_dim, scale, window=0, out=None):
-    """The same contract as ``attention_prefill`` in float32 on the FMA units (head sizes 64 and 128)."""
+    """The same contract as ``attention_prefill`` in float32 on the tensor cores, by bfloat16 planes (head sizes 64 and 128)."""
     if out is None:
         out = torch.empty((q.shape[0], n_heads * head_dim), dtype=torch.float32, device=q.device)
     check(lib("core").fg_attention_prefill_f32(ptr(q), q.stride(0), ptr(out), out.stride(0), ptr(cu_rows), ptr(seq_start),

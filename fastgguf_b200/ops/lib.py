@@ -108,7 +108,7 @@ def register_signatures(module: str, signatures: dict) -> None:
 
 
 #: (library, reader of its device-side error flag): a bounded wait that ran out leaves wrong output behind
-_ERROR_FLAGS = (("tc", "fg_gemm_tc_error"), ("attn", "fg_attention_prefill_tc_error"))
+_ERROR_FLAGS = (("tc", "fg_gemm_tc_error"), ("attn", "fg_attention_prefill_tc_error"), ("core", "fg_attention_prefill_f32_error"))
 
 
 def raise_on_device_error(where: str = "") -> None:

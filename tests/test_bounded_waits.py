@@ -88,3 +88,34 @@ def _attention_gives_up(ops, fast_attention, _err, make_case, plain):
     assert fast_attention.prefill_tc_error() == 0
     again = run()
     assert fast_attention.prefill_tc_error() == 0 and torch.equal(again, want)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+def test_float32_prefill_attention_gives_up_and_the_next_launch_is_correct(hd):
+    """(The two warps of a row meet at a barrier in every iteration: both get there, whichever wait ran out.)"""
+    from fastgguf_b200 import ops
+    from fastgguf_b200.ops import fast_attention
+    from test_kernels_attention import _err, make_case, plain
+    H, KV, new = 4, 2, [130]
+    case = make_case([70], new, H, KV, hd, torch.float32, 31)
+    scale = 1.0 / math.sqrt(hd)
+
+    def run():
+        out = fast_attention.attention_prefill_f32(case["q"], case["cu_rows"], case["seq_start"], case["table"], case["k_pool"],
+                                                   case["v_pool"], 1, 130, H, KV, hd, scale, 0)
+        torch.cuda.synchronize()
+        return out
+
+    want, error = run(), ops.lib("core").fg_attention_prefill_f32_error
+    assert error() == 0 and _err(want, plain(case, H, KV, hd, scale, 0)) < 5e-6
+    hook = _hook(ops.lib("core"), "fg_attention_prefill_f32_test_hook")
+    try:
+        assert hook(LIMIT, 1) == 0
+        t0 = time.time()
+        run()
+        assert time.time() - t0 < 2.0
+        assert error() >> 8 == 10003
+    finally:
+        assert hook(0, 0) == 0
+    assert error() == 0
+    assert torch.equal(run(), want) and error() == 0

@@ -132,6 +132,49 @@ def test_attention_prefill_f32(H, KV, hd, window):
     assert torch.equal(bad[:150], got[:150]) and torch.equal(bad[200:], got[200:])
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("what", ["large keys", "large queries", "large values", "small values", "a rare value alone", "infinite key", "infinite query",
+                                  "no number among the values"])
+def test_attention_prefill_f32_outside_the_range_of_the_planes(what, hd):
+    """Numbers that three bfloat16 planes do not carry (or whose products overflow) come out as the any-size kernel has them, and a value that
+    only a key of tiny probability has keeps its digits."""
+    from fastgguf_b200 import ops
+    from fastgguf_b200.ops import fast_attention
+    H, KV, new = 8, 2, [130, 70]
+    case = make_case([0, 100], new, H, KV, hd, torch.float32, 17, boost=False)
+    k, v, q = case["k_pool"], case["v_pool"], case["q"]
+    page = [int(p) for p in case["table"][0, :2]]
+    if what == "large keys":
+        k.mul_(2.0 ** 64); q.mul_(2.0 ** -64)
+    elif what == "large queries":
+        q.mul_(2.0 ** 70); k.mul_(2.0 ** -70)
+    elif what == "large values":
+        v.mul_(2.0 ** 100)
+    elif what == "small values":
+        v.mul_(2.0 ** -118)
+    elif what == "a rare value alone":
+        k[page[0], 0, 10] = -q[90, :hd] * (84.0 / float(q[90, :hd] @ q[90, :hd]) * hd ** 0.5)     # row 90, head 0: about e^-86
+        v[:, 0, :, 3] = 0.0
+        v[page[0], 0, 10, 3] = 1.2345678 * 2.0 ** 20
+    elif what == "infinite key":
+        k[page[1], 1, 5, 7] = float("inf")
+    elif what == "infinite query":
+        q[20, 3] = -float("inf")
+    else:
+        v[page[0], 0, 9, 2] = float("nan")
+    scale = 1.0 / math.sqrt(hd)
+    got = fast_attention.attention_prefill_f32(q, case["cu_rows"], case["seq_start"], case["table"], k, v, 2, 130, H, KV, hd, scale, 0)
+    want = ops.attention_generic(q, case["positions"], case["row_seq"], case["table"], k, v, H, KV, hd, scale, 0)
+    assert torch.equal(got.isnan(), want.isnan())
+    got, want = got.double().nan_to_num(), want.double().nan_to_num()
+    assert (got - want).abs().max() <= 5e-6 * want.abs().max()
+    if what == "a rare value alone":
+        # a score of -84 by a chain of hd additions is off by hd * 84 * 2^-24 at most, in either; a probability of 2^-124 in planes that end
+        # at 2^-133 would be off by 2^-9
+        x, y = got[90, 3], want[90, 3]
+        assert y > 0 and abs(x - y) <= 2 * hd * 84 * 2.0 ** -24 * y
+
+
 def test_attention_prefill_f32_leaves_out_sequences_of_few_rows():
     """With skip_few the rows of every sequence that the rule names keep what the output held, all others have their values."""
     import ctypes
