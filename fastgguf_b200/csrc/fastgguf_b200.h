@@ -118,6 +118,10 @@ int fg_argmax(const float *logits, int B, int V, int ldl, int *out, cudaStream_t
 int fg_retention(const float *proj, int ld, void *out, int out_dtype, int ldo, const int *positions, const int *cu_rows,
                  const int *slots, const float *cos_t, const float *sin_t, const float *decay, float *state, int n_seq,
                  int H, int dk, int dv, float k_scale, float eps, int opts, cudaStream_t stream);
+/* the same; early: the state is fetched before the wait on the kernel in front, which must not have written it */
+int fg_retention_step(const float *proj, int ld, void *out, int out_dtype, int ldo, const int *positions, const int *cu_rows,
+                      const int *slots, const float *cos_t, const float *sin_t, const float *decay, float *state, int n_seq,
+                      int H, int dk, int dv, float k_scale, float eps, int opts, int early, cudaStream_t stream);
 int fg_retention_chunk_tokens(void);
 int fg_retention_chunked_ok(int dk, int dv);
 int fg_retention_chunked(const float *proj, int ld, void *out, int out_dtype, int ldo, const int *positions,
@@ -179,6 +183,16 @@ int fg_conv1d_state(const float *in, int ld, int taps, float *state, long long s
 int fg_decay_gates(const float *a_raw, int lda, const float *b_raw, int ldb, const float *A_log, const float *dt_bias, int mode,
                    float *decay, float *step, int M, int H, cudaStream_t stream);
 int fg_unit_heads(float *x, int ld, int n_heads, int d, float eps, float scale, int M, cudaStream_t stream);
+/* n_heads heads, the first n_scaled of them times scale, the others times 1 */
+int fg_unit_heads_pair(float *x, int ld, int n_heads, int d, float eps, float scale, int n_scaled, int M, cudaStream_t stream);
+/* one token a sequence: convolution and its state in one kernel (up to eight taps), and gates and recurrence in one (delta: mode 1 of
+   fg_decay_gates, else mode 0); early: the state is fetched before the wait on the kernel in front, which must not have written it */
+int fg_conv1d_step(const float *in, int ld, const float *w, const float *bias, int taps, float *state, long long state_stride,
+                   const int *row_seq, const int *slots, float *out, int ldo, int M, int C, int early, cudaStream_t stream);
+int fg_decay_recurrence_step(const float *q, int ldq, const float *k, int ldk, const float *v, int ldv, const float *a_raw, int lda,
+                             const float *b_raw, int ldb, const float *A_log, const float *dt_bias, const float *skip, float *out, int ldo,
+                             const int *cu_rows, const int *slots, float *state, long long state_stride, int n_seq, int H, int Hq, int d, int dv,
+                             int delta, int early, cudaStream_t stream);
 /* gate_first: t = y silu(g), out = t / rms(t) * w over groups of `group` channels; else out = y / rms(y) * w[c % w_period] * silu(g);
    sigmoid_gate: sigmoid(g) for silu(g) */
 int fg_gated_group_norm(const float *y, int ldy, const float *g, int ldg, const float *w, int w_period, void *out, int out_dtype,

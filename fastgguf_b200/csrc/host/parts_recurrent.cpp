@@ -128,8 +128,8 @@ public:
                       b.slots, cos_t, sin_t, decay_dev_.t.ptr<float>(), (float *)io.state, plan, U, b.n_seq, n_chunks, H_, dk_, dv_,
                       k_scale_, eps_, opts, rt.stream);
         } else {
-            FG_LAUNCH("mix", fg_retention, proj.ptr<float>(), (int)proj.ld, o.data, o.dtype, (int)o.ld, b.positions, b.cu_rows, b.slots, cos_t,
-                      sin_t, decay_dev_.t.ptr<float>(), (float *)io.state, b.n_seq, H_, dk_, dv_, k_scale_, eps_, opts, rt.stream);
+            FG_LAUNCH("mix", fg_retention_step, proj.ptr<float>(), (int)proj.ld, o.data, o.dtype, (int)o.ld, b.positions, b.cu_rows, b.slots, cos_t,
+                      sin_t, decay_dev_.t.ptr<float>(), (float *)io.state, b.n_seq, H_, dk_, dv_, k_scale_, eps_, opts, b.single_token ? 1 : 0, rt.stream);
         }
         if (whole_norm_)
             FG_LAUNCH("mix", fg_gated_group_norm, o.ptr<float>(), (int)o.ld, proj.ptr<float>() + (int64_t)2 * H_ * dk_ + (int64_t)H_ * dv_, (int)proj.ld,
@@ -340,17 +340,25 @@ public:
         const int M = (int)proj.rows, ld = (int)proj.ld;
         float *state = (float *)io.state;
         Tensor xbc = rt.arena->matrix(M, C, FG_F32);
-        FG_LAUNCH("mix", fg_conv1d_silu, proj.ptr<float>() + I, ld, conv_w_.t.ptr<float>(), conv_b_.t.ptr<float>(), taps_, state, stride, b.row_seq, b.cu_rows,
-                  b.slots, xbc.ptr<float>(), (int)xbc.ld, M, C, rt.stream);
-        if (taps_ > 1)
-            FG_LAUNCH("mix", fg_conv1d_state, proj.ptr<float>() + I, ld, taps_, state, stride, b.cu_rows, b.slots, b.n_seq, C, rt.stream);
-        float *decay = (float *)rt.arena->alloc((size_t)2 * M * H_ * sizeof(float)), *step = decay + (size_t)M * H_;
-        FG_LAUNCH("mix", fg_decay_gates, proj.ptr<float>() + I + C, ld, nullptr, 0, a_log_.t.ptr<float>(), dt_bias_.t.ptr<float>(), 0, decay, step, M, H_,
-                  rt.stream);
-        Tensor y = rt.arena->matrix(M, I, FG_F32);
         const int xl = (int)xbc.ld;
-        FG_LAUNCH("mix", fg_decay_recurrence, xbc.ptr<float>() + I + GN, xl, xbc.ptr<float>() + I, xl, xbc.ptr<float>(), xl, decay, step, skip_.t.ptr<float>(),
-                  y.ptr<float>(), (int)y.ld, b.cu_rows, b.slots, state + conv_floats(), stride, b.n_seq, H_, G_, N_, dv_, 0, rt.stream);
+        Tensor y = rt.arena->matrix(M, I, FG_F32);
+        if (b.single_token && taps_ <= 8) {                  // a decode step: what is read of the state is on its way before the projection is done
+            FG_LAUNCH("mix", fg_conv1d_step, proj.ptr<float>() + I, ld, conv_w_.t.ptr<float>(), conv_b_.t.ptr<float>(), taps_, state, stride, b.row_seq, b.slots,
+                      xbc.ptr<float>(), xl, M, C, 1, rt.stream);
+            FG_LAUNCH("mix", fg_decay_recurrence_step, xbc.ptr<float>() + I + GN, xl, xbc.ptr<float>() + I, xl, xbc.ptr<float>(), xl, proj.ptr<float>() + I + C, ld,
+                      nullptr, 0, a_log_.t.ptr<float>(), dt_bias_.t.ptr<float>(), skip_.t.ptr<float>(), y.ptr<float>(), (int)y.ld, b.cu_rows, b.slots,
+                      state + conv_floats(), stride, b.n_seq, H_, G_, N_, dv_, 0, 1, rt.stream);
+        } else {
+            FG_LAUNCH("mix", fg_conv1d_silu, proj.ptr<float>() + I, ld, conv_w_.t.ptr<float>(), conv_b_.t.ptr<float>(), taps_, state, stride, b.row_seq, b.cu_rows,
+                      b.slots, xbc.ptr<float>(), xl, M, C, rt.stream);
+            if (taps_ > 1)
+                FG_LAUNCH("mix", fg_conv1d_state, proj.ptr<float>() + I, ld, taps_, state, stride, b.cu_rows, b.slots, b.n_seq, C, rt.stream);
+            float *decay = (float *)rt.arena->alloc((size_t)2 * M * H_ * sizeof(float)), *step = decay + (size_t)M * H_;
+            FG_LAUNCH("mix", fg_decay_gates, proj.ptr<float>() + I + C, ld, nullptr, 0, a_log_.t.ptr<float>(), dt_bias_.t.ptr<float>(), 0, decay, step, M, H_,
+                      rt.stream);
+            FG_LAUNCH("mix", fg_decay_recurrence, xbc.ptr<float>() + I + GN, xl, xbc.ptr<float>() + I, xl, xbc.ptr<float>(), xl, decay, step,
+                      skip_.t.ptr<float>(), y.ptr<float>(), (int)y.ld, b.cu_rows, b.slots, state + conv_floats(), stride, b.n_seq, H_, G_, N_, dv_, 0, rt.stream);
+        }
         Tensor yn = rt.arena->matrix(M, I, rt.dtype);
         FG_LAUNCH("mix", fg_gated_group_norm, y.ptr<float>(), (int)y.ld, proj.ptr<float>(), ld, norm_.t.ptr<float>(), I, yn.data, yn.dtype, (int)yn.ld, M, I,
                   I / norm_groups_, eps_, 1, 0, rt.stream);
@@ -439,17 +447,28 @@ public:
         float *state = (float *)io.state;
         Tensor qkv = rt.arena->matrix(M, C, FG_F32);
         const int xl = (int)qkv.ld;
-        FG_LAUNCH("mix", fg_conv1d_silu, proj.ptr<float>(), ld, conv_w_.t.ptr<float>(), nullptr, taps_, state, stride, b.row_seq, b.cu_rows, b.slots,
-                  qkv.ptr<float>(), xl, M, C, rt.stream);
-        if (taps_ > 1) FG_LAUNCH("mix", fg_conv1d_state, proj.ptr<float>(), ld, taps_, state, stride, b.cu_rows, b.slots, b.n_seq, C, rt.stream);
-        FG_LAUNCH("mix", fg_unit_heads, qkv.ptr<float>(), xl, G_, d_, unit_eps_, q_scale_, M, rt.stream);
-        FG_LAUNCH("mix", fg_unit_heads, qkv.ptr<float>() + Q, xl, G_, d_, unit_eps_, 1.0f, M, rt.stream);
-        float *decay = (float *)rt.arena->alloc((size_t)2 * M * H_ * sizeof(float)), *step = decay + (size_t)M * H_;
-        FG_LAUNCH("mix", fg_decay_gates, proj.ptr<float>() + C + H_, ld, proj.ptr<float>() + C, ld, a_log_.t.ptr<float>(), dt_bias_.t.ptr<float>(), 1, decay,
-                  step, M, H_, rt.stream);
+        const bool one = b.single_token && taps_ <= 8;       // a decode step: what is read of the state is on its way before the projection is done
+        if (one) {
+            FG_LAUNCH("mix", fg_conv1d_step, proj.ptr<float>(), ld, conv_w_.t.ptr<float>(), nullptr, taps_, state, stride, b.row_seq, b.slots, qkv.ptr<float>(), xl,
+                      M, C, 1, rt.stream);
+        } else {
+            FG_LAUNCH("mix", fg_conv1d_silu, proj.ptr<float>(), ld, conv_w_.t.ptr<float>(), nullptr, taps_, state, stride, b.row_seq, b.cu_rows, b.slots,
+                      qkv.ptr<float>(), xl, M, C, rt.stream);
+            if (taps_ > 1) FG_LAUNCH("mix", fg_conv1d_state, proj.ptr<float>(), ld, taps_, state, stride, b.cu_rows, b.slots, b.n_seq, C, rt.stream);
+        }
+        FG_LAUNCH("mix", fg_unit_heads_pair, qkv.ptr<float>(), xl, 2 * G_, d_, unit_eps_, q_scale_, G_, M, rt.stream);       // q's heads, then k's
         Tensor o = rt.arena->matrix(M, V, FG_F32);
-        FG_LAUNCH("mix", fg_decay_recurrence, qkv.ptr<float>(), xl, qkv.ptr<float>() + Q, xl, qkv.ptr<float>() + 2 * Q, xl, decay, step, nullptr, o.ptr<float>(),
-                  (int)o.ld, b.cu_rows, b.slots, state + conv_floats(), stride, b.n_seq, H_, G_, d_, dv_, 1, rt.stream);
+        const float *beta = proj.ptr<float>() + C, *decay_raw = beta + H_;
+        if (one) {
+            FG_LAUNCH("mix", fg_decay_recurrence_step, qkv.ptr<float>(), xl, qkv.ptr<float>() + Q, xl, qkv.ptr<float>() + 2 * Q, xl, decay_raw, ld, beta, ld,
+                      a_log_.t.ptr<float>(), dt_bias_.t.ptr<float>(), nullptr, o.ptr<float>(), (int)o.ld, b.cu_rows, b.slots, state + conv_floats(), stride,
+                      b.n_seq, H_, G_, d_, dv_, 1, 1, rt.stream);
+        } else {
+            float *decay = (float *)rt.arena->alloc((size_t)2 * M * H_ * sizeof(float)), *step = decay + (size_t)M * H_;
+            FG_LAUNCH("mix", fg_decay_gates, decay_raw, ld, beta, ld, a_log_.t.ptr<float>(), dt_bias_.t.ptr<float>(), 1, decay, step, M, H_, rt.stream);
+            FG_LAUNCH("mix", fg_decay_recurrence, qkv.ptr<float>(), xl, qkv.ptr<float>() + Q, xl, qkv.ptr<float>() + 2 * Q, xl, decay, step, nullptr, o.ptr<float>(),
+                      (int)o.ld, b.cu_rows, b.slots, state + conv_floats(), stride, b.n_seq, H_, G_, d_, dv_, 1, rt.stream);
+        }
         Tensor y = rt.arena->matrix(M, V, rt.dtype);
         FG_LAUNCH("mix", fg_gated_group_norm, o.ptr<float>(), (int)o.ld, proj.ptr<float>() + C + 2 * H_, ld, norm_.t.ptr<float>(), dv_, y.data, y.dtype,
                   (int)y.ld, M, V, dv_, eps_, 0, 0, rt.stream);

@@ -23,6 +23,7 @@
 #define REC_THREADS 256
 #define REC_RPL 16                  // rows of a column a lane holds at most
 #define REC_KEEP 8                  // numbers of a group that a lane of the norms holds in registers
+#define REC_TAPS 8                  // taps of a convolution that the single-token kernel takes
 #define REC_TC 16                   // tokens staged at a time (fewer where a head's rows are many)
 
 __device__ __forceinline__ float rec_silu(float z) { return z / (1.0f + expf(-z)); }
@@ -94,9 +95,46 @@ conv1d_state_kernel(const float *__restrict__ in, int ld, int taps, float *__res
     }
 }
 
+// One token a sequence: the output and the state's shift by one, in one kernel - a thread owns a channel of a row, and nobody else reads or
+// writes that channel's inputs.  Weights, and with AHEAD the state, are fetched before the wait (see decay_step_kernel below).  8 rows of 4,352
+// channels inside a step: 7.1 + 2.2 us as two kernels (what it takes here: see decay_step_kernel).
+template <bool AHEAD>
+__global__ void __launch_bounds__(256)
+conv1d_step_kernel(const float *__restrict__ in, int ld, const float *__restrict__ w, const float *__restrict__ bias, int taps, float *state,
+                   long long state_stride, const int *__restrict__ row_seq, const int *__restrict__ slots, float *__restrict__ out, int ldo, int C) {
+    pdl_launch_dependents_small_step(gridDim.x);
+    const int m = blockIdx.x, c = blockIdx.y * 256 + threadIdx.x;
+    const bool live = c < C;
+    float wc[REC_TAPS], u[REC_TAPS], acc = 0.f;
+    if (live) {
+        acc = bias ? bias[c] : 0.f;
+#pragma unroll
+        for (int j = 0; j < REC_TAPS; j++) wc[j] = j < taps ? w[(size_t)c * taps + j] : 0.f;
+    }
+    if (!AHEAD) pdl_wait();
+    float *st = state + (size_t)slots[row_seq[m]] * state_stride + c;
+#pragma unroll
+    for (int j = 0; j < REC_TAPS; j++) u[j] = live && j < taps - 1 ? st[(size_t)j * C] : 0.f;
+    if (AHEAD) pdl_wait();
+    if (!live) return;
+    const float x = in[(size_t)m * ld + c];
+#pragma unroll
+    for (int j = 0; j < REC_TAPS; j++)
+        if (j < taps) acc = fmaf(wc[j], j < taps - 1 ? u[j] : x, acc);
+    out[(size_t)m * ldo + c] = rec_silu(acc);
+#pragma unroll
+    for (int j = 0; j < REC_TAPS - 1; j++)
+        if (j < taps - 1) st[(size_t)j * C] = j + 1 < taps - 1 ? u[j + 1] : x;
+}
+
 // ------------------------------------------------------------------ decays and steps
 // mode 0: b = softplus(a_raw + dt_bias), a = exp(-exp(A_log) b)                    (one raw number a head)
 // mode 1: a = exp(-exp(A_log) softplus(a_raw + dt_bias)), b = sigmoid(b_raw)
+__device__ __forceinline__ void rec_gates(float a_raw, const float *b_raw, float A_log, float dt_bias, int mode, float &decay, float &step) {
+    const float sp = rec_softplus(a_raw + dt_bias);
+    decay = expf(-expf(A_log) * sp);
+    step = mode == 0 ? sp : rec_sigmoid(*b_raw);
+}
 __global__ void decay_gates_kernel(const float *__restrict__ a_raw, int lda, const float *__restrict__ b_raw, int ldb,
                                    const float *__restrict__ A_log, const float *__restrict__ dt_bias, int mode,
                                    float *__restrict__ decay, float *__restrict__ step, int M, int H) {
@@ -105,19 +143,18 @@ __global__ void decay_gates_kernel(const float *__restrict__ a_raw, int lda, con
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= M * H) return;
     const int m = e / H, h = e % H;
-    const float sp = rec_softplus(a_raw[(size_t)m * lda + h] + dt_bias[h]);
-    decay[e] = expf(-expf(A_log[h]) * sp);
-    step[e] = mode == 0 ? sp : rec_sigmoid(b_raw[(size_t)m * ldb + h]);
+    rec_gates(a_raw[(size_t)m * lda + h], mode ? b_raw + (size_t)m * ldb + h : nullptr, A_log[h], dt_bias[h], mode, decay[e], step[e]);
 }
 
-// x[m, h, :] <- x / sqrt(sum(x^2) + eps) * scale, a warp a (row, head)
+// x[m, h, :] <- x / sqrt(sum(x^2) + eps) * scale (heads from n_scaled on: * 1), a warp a (row, head)
 __global__ void __launch_bounds__(256)
-unit_heads_kernel(float *__restrict__ x, int ld, int n_heads, int d, float eps, float scale, int M) {
+unit_heads_kernel(float *__restrict__ x, int ld, int n_heads, int d, float eps, float scale_of, int n_scaled, int M) {
     pdl_launch_dependents_small_step(M);
     pdl_wait();
     const int id = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (id >= M * n_heads) return;
     float *p = x + (size_t)(id / n_heads) * ld + (size_t)(id % n_heads) * d;
+    const float scale = id % n_heads < n_scaled ? scale_of : 1.0f;
     float ss = 0.f;
     if (d <= 32 * REC_KEEP) {                               // a head in the warp's registers: its loads are in flight together
         float v[REC_KEEP];
@@ -271,6 +308,66 @@ decay_recurrence_kernel(const float *__restrict__ q, int ldq, const float *__res
             if (e < epl) Sg[((size_t)e * dv + c) * R + r] = S[e];
 }
 
+// The same for one token a sequence (a decode step): nothing to stage, so a lane reads its rows of k and q from the caches, the gates are computed
+// where they are used, and the state is in flight before the wait on the kernel in front (AHEAD: state rows are written by this entry's kernels
+// alone, once a step, and slots by the copy that opens a step, see common.cuh).  Lanes, rows and order of additions are those of the kernel above.
+// Bound by memory: 2 x 1 MB of state a sequence, 2.6 us for 8.  Inside a step of 8 sequences 12.3 us at 32 heads of 128 x 64 and 12.8 for the
+// delta rule at 16 heads of 128 x 128, 2 more for the gates' kernel, before.  This kernel, conv1d_step_kernel and the norms of q and k in one launch take
+// a step with two layers of each from 712 to 644 us.
+#define STEP_THREADS 128
+template <bool DELTA, int NJ, bool AHEAD>
+__global__ void __launch_bounds__(STEP_THREADS)
+decay_step_kernel(const float *__restrict__ q, int ldq, const float *__restrict__ k, int ldk, const float *__restrict__ v, int ldv,
+                  const float *__restrict__ a_raw, int lda, const float *__restrict__ b_raw, int ldb, const float *__restrict__ A_log,
+                  const float *__restrict__ dt_bias, const float *__restrict__ skip, float *__restrict__ out, int ldo,
+                  const int *__restrict__ cu_rows, const int *__restrict__ slots, float *state, long long state_stride, int H, int Hq, int d,
+                  int dv, int R, int logR) {
+    pdl_launch_dependents_small_step(gridDim.x);
+    const int seq = blockIdx.x, h = blockIdx.y, at = blockIdx.z * STEP_THREADS + threadIdx.x;
+    const int epl = (d + R - 1) / R, c = at >> logR, r = at & (R - 1), hq = h / (H / Hq);
+    const bool live = c < dv;
+    if (!AHEAD) pdl_wait();
+    float *Sg = state + (size_t)slots[seq] * state_stride + (size_t)h * epl * dv * R + (size_t)c * R + r;
+    const size_t next = (size_t)dv * R;
+    float S[4 * NJ];
+#pragma unroll
+    for (int e = 0; e < 4 * NJ; e++) S[e] = live && e < epl ? Sg[e * next] : 0.f;
+    const float Dh = skip ? skip[h] : 0.f, al = A_log[h], bias = dt_bias[h];
+    if (AHEAD) pdl_wait();
+    const int row = cu_rows[seq];
+    if (cu_rows[seq + 1] <= row) return;
+    const float *kg = k + (size_t)row * ldk + (size_t)hq * d, *qg = q + (size_t)row * ldq + (size_t)hq * d;
+    float kk[4 * NJ], qq[4 * NJ];
+#pragma unroll
+    for (int e = 0; e < 4 * NJ; e++) {
+        const int i = (e << logR) + r;
+        kk[e] = i < d ? kg[i] : 0.f;
+        qq[e] = i < d ? qg[i] : 0.f;
+    }
+    const float vj = live ? v[(size_t)row * ldv + (size_t)h * dv + c] : 0.f;
+    float a, b;
+    rec_gates(a_raw[(size_t)row * lda + h], DELTA ? b_raw + (size_t)row * ldb + h : nullptr, al, bias, DELTA, a, b);
+    float d0 = 0.f, d1 = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4 * NJ; e += 2) {
+        S[e] *= a; S[e + 1] *= a;
+        if (DELTA) { d0 = fmaf(S[e], kk[e], d0); d1 = fmaf(S[e + 1], kk[e + 1], d1); }
+    }
+    const float w = b * (vj - (DELTA ? rec_lanes_sum(d0 + d1, R) : 0.f));
+    float o0 = 0.f, o1 = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4 * NJ; e += 2) {
+        S[e] = fmaf(kk[e], w, S[e]); S[e + 1] = fmaf(kk[e + 1], w, S[e + 1]);
+        o0 = fmaf(S[e], qq[e], o0); o1 = fmaf(S[e + 1], qq[e + 1], o1);
+    }
+    const float o = rec_lanes_sum(o0 + o1, R);
+    if (!live) return;
+    if (r == 0) out[(size_t)row * ldo + (size_t)h * dv + c] = fmaf(Dh, vj, o);
+#pragma unroll
+    for (int e = 0; e < 4 * NJ; e++)
+        if (e < epl) Sg[e * next] = S[e];
+}
+
 // ------------------------------------------------------------------ gate and norm behind the recurrence
 // gate_first: t = y * silu(g), out = t / rms_group(t) * w[c]                         (groups of `group` neighbouring channels)
 // else:       out = y / rms_group(y) * w[c % w_period] * silu(g)
@@ -389,10 +486,14 @@ extern "C" int fg_decay_gates(const float *a_raw, int lda, const float *b_raw, i
                               decay, step, M, H);
 }
 
-extern "C" int fg_unit_heads(float *x, int ld, int n_heads, int d, float eps, float scale, int M, cudaStream_t stream) {
+// heads of two neighbouring projections in one launch: the first n_scaled take the scale
+extern "C" int fg_unit_heads_pair(float *x, int ld, int n_heads, int d, float eps, float scale, int n_scaled, int M, cudaStream_t stream) {
     if (M <= 0) return 0;
     if (n_heads <= 0 || d <= 0) return FG_ERR_BAD_SIZE;
-    return fg_launch(unit_heads_kernel, dim3((M * n_heads + 7) / 8), dim3(256), 0, stream, x, ld, n_heads, d, eps, scale, M);
+    return fg_launch(unit_heads_kernel, dim3((M * n_heads + 7) / 8), dim3(256), 0, stream, x, ld, n_heads, d, eps, scale, n_scaled, M);
+}
+extern "C" int fg_unit_heads(float *x, int ld, int n_heads, int d, float eps, float scale, int M, cudaStream_t stream) {
+    return fg_unit_heads_pair(x, ld, n_heads, d, eps, scale, n_heads, M, stream);
 }
 
 // lanes that share a column of the state: the smallest power of two that leaves a lane at most REC_RPL rows
@@ -451,6 +552,43 @@ extern "C" int fg_decay_recurrence(const float *q, int ldq, const float *k, int 
     if (NJ == 3) REC_LAUNCH(false, 3);
     REC_LAUNCH(false, 4);
 #undef REC_LAUNCH
+}
+
+// One token a sequence, gates included (raw numbers as for fg_decay_gates, mode 0 without the delta term, 1 with it).  early: the state is
+// fetched before the wait on the kernel in front, which must not have written it (see decay_step_kernel).
+extern "C" int fg_decay_recurrence_step(const float *q, int ldq, const float *k, int ldk, const float *v, int ldv, const float *a_raw, int lda,
+                                        const float *b_raw, int ldb, const float *A_log, const float *dt_bias, const float *skip, float *out, int ldo,
+                                        const int *cu_rows, const int *slots, float *state, long long state_stride, int n_seq, int H, int Hq, int d,
+                                        int dv, int delta, int early, cudaStream_t stream) {
+    if (n_seq <= 0) return 0;
+    const int R = fg_decay_recurrence_lanes(d);
+    if (!R || H <= 0 || Hq <= 0 || H % Hq || dv <= 0 || H > 65535 || (delta && !b_raw)) return FG_ERR_BAD_SIZE;
+    int logR = 0;
+    while ((1 << logR) < R) logR++;
+    const long long tiles = ((long long)dv * R + STEP_THREADS - 1) / STEP_THREADS;
+    if (tiles > 65535) return FG_ERR_BAD_SIZE;
+    const dim3 grid(n_seq, H, (unsigned)tiles);
+    const int NJ = ((d + R - 1) / R + 3) / 4;
+#define STEP_RUN(DELTA, NJ_, AHEAD) fg_launch(decay_step_kernel<DELTA, NJ_, AHEAD>, grid, dim3(STEP_THREADS), 0, stream, q, ldq, k, ldk, v, ldv, a_raw, lda, b_raw, \
+                                              ldb, A_log, dt_bias, skip, out, ldo, cu_rows, slots, state, state_stride, H, Hq, d, dv, R, logR)
+#define STEP_NJ(NJ_) do { \
+        if (delta) return early ? STEP_RUN(true, NJ_, true) : STEP_RUN(true, NJ_, false); \
+        return early ? STEP_RUN(false, NJ_, true) : STEP_RUN(false, NJ_, false); } while (0)
+    if (NJ == 1) STEP_NJ(1);
+    if (NJ == 2) STEP_NJ(2);
+    if (NJ == 3) STEP_NJ(3);
+    STEP_NJ(4);
+#undef STEP_NJ
+#undef STEP_RUN
+}
+
+// One token a sequence: fg_conv1d_silu and fg_conv1d_state in one (early: as above).  FG_ERR_BAD_SIZE beyond eight taps.
+extern "C" int fg_conv1d_step(const float *in, int ld, const float *w, const float *bias, int taps, float *state, long long state_stride,
+                              const int *row_seq, const int *slots, float *out, int ldo, int M, int C, int early, cudaStream_t stream) {
+    if (M <= 0) return 0;
+    if (C <= 0 || taps <= 0 || taps > REC_TAPS || (taps > 1 && !state)) return FG_ERR_BAD_SIZE;
+    return fg_launch(early ? conv1d_step_kernel<true> : conv1d_step_kernel<false>, dim3(M, (C + 255) / 256), dim3(256), 0, stream, in, ld, w, bias, taps, state,
+                     state_stride, row_seq, slots, out, ldo, C);
 }
 
 extern "C" int fg_gated_group_norm(const float *y, int ldy, const float *g, int ldg, const float *w, int w_period, void *out,

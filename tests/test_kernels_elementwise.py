@@ -337,3 +337,85 @@ def test_a_row_does_not_depend_on_the_other_rows_of_the_step(E):
         for rows in (1, 64):
             for few, many in zip(f(rows), f(M)):
                 assert torch.equal(few, many[:rows])
+
+
+@pytest.mark.parametrize("early", [0, 1])
+@pytest.mark.parametrize("taps", [1, 2, 4, 8])
+def test_conv1d_step(taps, early):
+    """One token a sequence in one kernel: bit for bit what the convolution and the state's update give, one after the other."""
+    import ctypes
+    C, n = 1500, 5
+    g = torch.Generator().manual_seed(taps)
+    u, w, bias, state = (torch.randn(*s, generator=g).cuda() for s in ((n, C), (C, taps), (C,), (n + 1, max(1, taps - 1), C)))
+    cu, row_seq = torch.arange(n + 1, dtype=torch.int32).cuda(), torch.arange(n, dtype=torch.int32).cuda()
+    slots = torch.tensor([4, 0, 5, 1, 2], dtype=torch.int32).cuda()
+    want, want_state, stride = torch.empty(n, C, device="cuda"), state.clone(), ctypes.c_longlong(state.stride(0))
+    _call("mix", "fg_conv1d_silu", u, C, w, bias, taps, want_state, stride, row_seq, cu, slots, want, C, n, C)
+    if taps > 1:
+        _call("mix", "fg_conv1d_state", u, C, taps, want_state, stride, cu, slots, n, C)
+    torch.cuda.synchronize()
+    out = torch.empty(n, C, device="cuda")
+    _call("mix", "fg_conv1d_step", u, C, w, bias, taps, state, stride, row_seq, slots, out, C, n, C, early)
+    assert torch.equal(out, want) and torch.equal(state, want_state)
+
+
+@pytest.mark.parametrize("early", [0, 1])
+@pytest.mark.parametrize("H,Hq,d,dv,delta", [(4, 1, 128, 64, 0), (4, 2, 128, 128, 1), (3, 3, 16, 24, 1), (2, 1, 20, 7, 0), (4, 4, 300, 40, 1), (2, 2, 1, 3, 0), (2, 1, 512, 9, 1)])
+def test_decay_recurrence_step(H, Hq, d, dv, delta, early):
+    """One token a sequence with the gates in the kernel: bit for bit the gates' kernel and the recurrence over tokens behind it."""
+    import ctypes
+    from fastgguf_b200.ops.lib import lib
+    n = 5
+    g = torch.Generator().manual_seed(d + dv)
+    floats = lib("mix").fg_decay_recurrence_state_floats
+    floats.restype = ctypes.c_longlong
+    q, k, v, raw, state = (torch.randn(*s, generator=g).cuda() for s in ((n, Hq * d), (n, Hq * d), (n, H * dv), (n, 2 * H), (n + 1, floats(H, d, dv))))
+    A_log, bias, skip = (torch.randn(H, generator=g).cuda() for _ in range(3))
+    k /= d ** 0.5
+    cu, slots = torch.arange(n + 1, dtype=torch.int32).cuda(), torch.tensor([4, 0, 5, 1, 2], dtype=torch.int32).cuda()
+    stride = ctypes.c_longlong(state.stride(0))
+    decay, step, want, want_state = torch.empty(n, H, device="cuda"), torch.empty(n, H, device="cuda"), torch.empty(n, H * dv, device="cuda"), state.clone()
+    beta = raw[:, H:]
+    _call("mix", "fg_decay_gates", raw, 2 * H, beta if delta else None, 2 * H, A_log, bias, delta, decay, step, n, H)
+    _call("mix", "fg_decay_recurrence", q, Hq * d, k, Hq * d, v, H * dv, decay, step, None if delta else skip, want, H * dv, cu, slots, want_state, stride, n, H, Hq,
+          d, dv, delta)
+    torch.cuda.synchronize()
+    out = torch.empty(n, H * dv, device="cuda")
+    _call("mix", "fg_decay_recurrence_step", q, Hq * d, k, Hq * d, v, H * dv, raw, 2 * H, beta if delta else None, 2 * H, A_log, bias, None if delta else skip, out,
+          H * dv, cu, slots, state, stride, n, H, Hq, d, dv, delta, early)
+    assert torch.equal(out, want) and torch.equal(state, want_state)
+
+
+@pytest.mark.parametrize("rotated", [True, False])
+@pytest.mark.parametrize("dk,dv", [(64, 64), (64, 128), (128, 64), (128, 128), (48, 64)])        # the last: state in shared memory
+def test_retention_step(dk, dv, rotated):
+    """Sequences of one to three tokens against float64, the state included; fetching the state early changes nothing."""
+    n, H, lengths = 4, 3, [1, 3, 1, 2]
+    M = sum(lengths)
+    g = torch.Generator().manual_seed(dk + dv)
+    proj, start = torch.randn(M, H * (2 * dk + 2 * dv), generator=g).cuda(), torch.randn(n + 1, H, dk, dv, generator=g).cuda()
+    decay = torch.tensor([0.9, 0.97, 0.99]).cuda()
+    cos, sin = (f(torch.rand(50, dk // 2, generator=g) * 6.0).cuda() for f in (torch.cos, torch.sin))
+    cu = torch.tensor([0] + list(np.cumsum(lengths)), dtype=torch.int32).cuda()
+    slots, pos = torch.tensor([4, 0, 3, 1], dtype=torch.int32).cuda(), torch.arange(20, 20 + M, dtype=torch.int32).cuda()
+    outs = []
+    for early in (0, 1):
+        state, out = start.clone(), torch.empty(M, H * dv, device="cuda")
+        torch.cuda.synchronize()
+        _call("mix", "fg_retention_step", proj, proj.shape[1], out, 0, H * dv, pos, cu, slots, cos if rotated else None, sin if rotated else None, decay, state, n, H,
+              dk, dv, 0.25, 1e-6, 0, early)
+        torch.cuda.synchronize()
+        outs.append((out, state))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+    S, rows, half = start.double(), proj.double(), dk // 2
+    c, s = (t.double()[pos.long()][:, None] if rotated else x for t, x in ((cos, 1.0), (sin, 0.0)))
+    turn = lambda x: torch.cat([x[..., :half] * c - x[..., half:] * s, x[..., half:] * c + x[..., :half] * s], -1)       # noqa: E731
+    q, k = turn(rows[:, :H * dk].view(M, H, dk)), turn(rows[:, H * dk:2 * H * dk].view(M, H, dk)) * 0.25
+    v, z = rows[:, 2 * H * dk:2 * H * dk + H * dv].view(M, H, dv), rows[:, 2 * H * dk + H * dv:].view(M, H, dv)
+    for i in range(n):
+        for t in range(int(cu[i]), int(cu[i + 1])):
+            S[slots[i]] = S[slots[i]] * decay.double()[:, None, None] + k[t][:, :, None] * v[t][:, None]
+            o = (q[t][:, :, None] * S[slots[i]]).sum(1)
+            want = o / (o.square().mean(-1, keepdim=True) + 1e-6).sqrt() * torch.nn.functional.silu(z[t])
+            assert (outs[0][0][t].view(H, dv).double() - want).abs().max() <= 1e-5 * want.abs().max()
+    assert (outs[0][1].double() - S).abs().max() <= 1e-6 * S.abs().max()
