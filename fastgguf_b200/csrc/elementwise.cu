@@ -697,6 +697,31 @@ extern "C" int fg_decode_advance(int *tokens, int *positions, const int *next_to
     return fg_launch(decode_advance_kernel, dim3((B + 127) / 128), dim3(128), 0, stream, tokens, positions, next_tokens, active, B);
 }
 
+// The same for at most 1,024 rows (one block), the tokens also to the host: region *turn of a ring of `regions` in pinned memory that the device
+// can write.  The host finds them when the step's event has fired, and no copy stands between one step's graph and the next.  A copy of
+// 32 bytes behind each graph cost 8 to 9 us a step: tiny model of the tests 53 -> 45 us, Llama 1B at batch 8 683 -> 675.
+__global__ void decode_advance_host_kernel(int *__restrict__ tokens, int *__restrict__ positions, const int *__restrict__ next_tokens,
+                                           const int *__restrict__ active, int B, int *__restrict__ host_tokens, int *turn, int regions) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int b = threadIdx.x, at = *turn;
+    __syncthreads();
+    if (b == 0) *turn = at + 1 < regions ? at + 1 : 0;
+    if (b >= B) return;
+    const int token = next_tokens[b];
+    host_tokens[(size_t)at * B + b] = token;
+    tokens[b] = token;
+    if (active[b]) positions[b] += 1;
+}
+
+extern "C" int fg_decode_advance_host(int *tokens, int *positions, const int *next_tokens, const int *active, int B, int *host_tokens, int *turn,
+                                      int regions, cudaStream_t stream) {
+    if (B <= 0) return 0;
+    if (B > 1024 || regions <= 0) return FG_ERR_BAD_SIZE;
+    return fg_launch(decode_advance_host_kernel, dim3(1), dim3((B + 31) / 32 * 32), 0, stream, tokens, positions, next_tokens, active, B, host_tokens, turn,
+                     regions);
+}
+
 // ------------------------------------------------------------------ two float32 matrices side by side
 // out[m, 0 .. E) = a[m, :], out[m, E .. 2 E) = b[m, :], in the contraction's input dtype
 template <typename T>

@@ -68,6 +68,9 @@ int fg_cast_rows(const float *x, int ldx, void *out, int out_dtype, int ldo, int
 int fg_gelu_mul_gather(const float *z, int ldz, const void *table, int table_dtype, int ldt, int col0, const int *tokens, void *out,
                        int out_dtype, int ldo, int M, int D, cudaStream_t stream);
 int fg_decode_advance(int *tokens, int *positions, const int *next_tokens, const int *active, int B, cudaStream_t stream);
+/* the same (B <= 1,024), the tokens also to region *turn of host_tokens [regions, B] in pinned host memory; *turn moves on by one */
+int fg_decode_advance_host(int *tokens, int *positions, const int *next_tokens, const int *active, int B, int *host_tokens, int *turn,
+                           int regions, cudaStream_t stream);
 int fg_gemm_generic_step(const void *A, int a_dtype, int lda, const void *W, int w_dtype, int ldw, void *C, int out_dtype,
                          int ldc, int accumulate, int M, int N, int K, int early, cudaStream_t stream);
 int fg_gemm_generic(const void *A, int a_dtype, int lda, const void *W, int w_dtype, int ldw, void *C, int out_dtype,

@@ -167,7 +167,7 @@ DecodeGraph::DecodeGraph(Engine &e, Sampler &sampler, int width_) : width(width_
     table_width = (cache.max_seq_len + cache.page_size - 1) / cache.page_size;
     const int B = width, n_groups = (int)cache.groups.size();
     auto pad = [](size_t n) { return (n + 3) / 4 * 4; };
-    std::vector<size_t> sizes = {(size_t)B, (size_t)B, (size_t)B, (size_t)B + 1, (size_t)B, (size_t)B, (size_t)B, (size_t)B, 4};
+    std::vector<size_t> sizes = {(size_t)B, (size_t)B, (size_t)B, (size_t)B + 1, (size_t)B, (size_t)B, (size_t)B, (size_t)B, 4, 4};
     for (int g = 0; g < n_groups; g++) sizes.push_back((size_t)B * table_width);
     std::vector<size_t> offs;
     size_t total = 0;
@@ -177,8 +177,8 @@ DecodeGraph::DecodeGraph(Engine &e, Sampler &sampler, int width_) : width(width_
     int *base = (int *)ints_.get();
     tokens = base + offs[0]; positions = base + offs[1]; row_seq = base + offs[2]; cu_rows = base + offs[3];
     rows = base + offs[4]; want = base + offs[5]; active = base + offs[6]; next_tokens = base + offs[7];
-    spare_cell = base + offs[8];
-    for (int g = 0; g < n_groups; g++) tables.push_back(base + offs[9 + (size_t)g]);
+    spare_cell = base + offs[8]; turn = base + offs[9];
+    for (int g = 0; g < n_groups; g++) tables.push_back(base + offs[10 + (size_t)g]);
     std::vector<int> ar((size_t)B + 1), spare((size_t)B, sampler.spare_row);
     for (int i = 0; i <= B; i++) ar[(size_t)i] = i;
     FG_CUDA(cudaMemcpy(row_seq, ar.data(), (size_t)B * 4, cudaMemcpyHostToDevice));
@@ -188,8 +188,10 @@ DecodeGraph::DecodeGraph(Engine &e, Sampler &sampler, int width_) : width(width_
     FG_CUDA(cudaMemcpy(spare_cell, spare.data(), 4, cudaMemcpyHostToDevice));
     upload_cap = std::max<size_t>(16, (size_t)B * table_width * (size_t)std::max(1, n_groups));
     regions.resize(4);
-    for (auto &r : regions) {
-        FG_CUDA(cudaMallocHost((void **)&r.tokens, (size_t)B * 4));
+    FG_CUDA(cudaMallocHost((void **)&host_tokens_, regions.size() * B * 4));
+    for (size_t i = 0; i < regions.size(); i++) {
+        Region &r = regions[i];
+        r.tokens = host_tokens_ + i * B;
         FG_CUDA(cudaMallocHost((void **)&r.upload, upload_cap * 4));
         FG_CUDA(cudaEventCreateWithFlags(&r.done, cudaEventDisableTiming));
     }
@@ -209,6 +211,7 @@ DecodeGraph::DecodeGraph(Engine &e, Sampler &sampler, int width_) : width(width_
     FG_CUDA(cudaStreamSynchronize(e.stream));
     FG_CUDA(cudaMemset(tokens, 0, (size_t)B * 4));
     FG_CUDA(cudaMemset(positions, 0, (size_t)B * 4));
+    FG_CUDA(cudaMemset(turn, 0, 4));
     arena_.reset();                                  // one block for what the warm-up needed
     arena_.forbid_growth(true);
     FG_CUDA(cudaStreamBeginCapture(e.capture_stream, cudaStreamCaptureModeRelaxed));
@@ -228,9 +231,9 @@ DecodeGraph::DecodeGraph(Engine &e, Sampler &sampler, int width_) : width(width_
 DecodeGraph::~DecodeGraph() {
     for (auto &r : regions) {
         if (r.done) { cudaEventSynchronize(r.done); cudaEventDestroy(r.done); }
-        if (r.tokens) cudaFreeHost(r.tokens);
         if (r.upload) cudaFreeHost(r.upload);
     }
+    if (host_tokens_) cudaFreeHost(host_tokens_);
     if (exec_) cudaGraphExecDestroy(exec_);
     if (graph_) cudaGraphDestroy(graph_);
 }
@@ -246,7 +249,7 @@ void DecodeGraph::run(cudaStream_t s, bool recording) {
     arena_.reset();
     Tensor logits = engine_.model->forward(rt, batch_);
     sampler_.sample(logits.ptr<float>(), width, (int)logits.cols, (int)logits.ld, rows, next_tokens, s);
-    FG_LAUNCH("core", fg_decode_advance, tokens, positions, next_tokens, active, width, s);
+    FG_LAUNCH("core", fg_decode_advance_host, tokens, positions, next_tokens, active, width, host_tokens_, turn, (int)regions.size(), s);
 }
 
 void DecodeGraph::replay() { FG_CUDA(cudaGraphLaunch(exec_, engine_.stream)); }
@@ -384,9 +387,8 @@ int DecodeSession::advance(const std::vector<int> &live) {
         }
     }
     const int idx = g.next_region;
-    g.next_region = (g.next_region + 1) % (int)g.regions.size();
     DecodeGraph::Region &region = g.regions[(size_t)idx];
-    FG_CUDA(cudaEventSynchronize(region.done));                      // its copies of four steps ago have left it
+    FG_CUDA(cudaEventSynchronize(region.done));                      // its step, four steps ago, is done
     size_t used = 0;
     std::vector<int> row((size_t)g.table_width);
     for (int i : live) {                                             // upload page-table entries the step will touch
@@ -408,9 +410,9 @@ int DecodeSession::advance(const std::vector<int> &live) {
         }
     }
     g.replay();
+    g.next_region = (idx + 1) % (int)g.regions.size();               // (the device's count moves on with the replay)
     cache.commit(steps);
     eng.stats.steps++;
-    FG_CUDA(cudaMemcpyAsync(region.tokens, g.next_tokens, (size_t)g.width * 4, cudaMemcpyDeviceToHost, s));
     FG_CUDA(cudaEventRecord(region.done, s));
     eng.stats.d2h_bytes += 4LL * g.width;
     return idx;

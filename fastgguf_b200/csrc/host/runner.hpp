@@ -114,11 +114,11 @@ public:
     int width, table_width;
     long long launches_per_step = 0;
     // device views
-    int *tokens, *positions, *row_seq, *cu_rows, *rows, *want, *active, *next_tokens, *spare_cell;
+    int *tokens, *positions, *row_seq, *cu_rows, *rows, *want, *active, *next_tokens, *spare_cell, *turn;
     std::vector<int *> tables;
-    // pinned host memory, a few regions in turn, each guarded by an event: the sampled tokens of a step on their
-    // way to the host, and the page-table entries of a step on their way to the device (copies from pageable
-    // memory would make the host wait for the stream at every step)
+    // pinned host memory, a few regions in turn, each guarded by an event: the sampled tokens of a step, which its last kernel writes
+    // there (*turn on the device is the region the next replay writes, next_region here), and the page-table entries of a step on
+    // their way to the device (copies from pageable memory would make the host wait for the stream at every step)
     struct Region { int *tokens = nullptr; int *upload = nullptr; cudaEvent_t done = nullptr; };
     std::vector<Region> regions;
     int next_region = 0;
@@ -130,6 +130,7 @@ private:
     Sampler &sampler_;
     Arena arena_;
     DeviceBuffer ints_;
+    int *host_tokens_ = nullptr;                     // the regions' tokens, one behind the other
     Batch batch_;
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t exec_ = nullptr;

@@ -237,6 +237,20 @@ def test_decode_advance():
     assert tokens.cpu().tolist() == [7, 8, 9] and pos.cpu().tolist() == [11, 21, 0]
 
 
+@pytest.mark.parametrize("B", [1, 33, 256])
+def test_decode_advance_host(B):
+    """The same with the tokens also in a ring of pinned host memory, region after region."""
+    g = torch.Generator().manual_seed(B)
+    tokens, active = torch.zeros(B, dtype=torch.int32).cuda(), (torch.arange(B) % 3 != 1).int().cuda()
+    pos, turn, ring = torch.arange(B, dtype=torch.int32).cuda(), torch.zeros(1, dtype=torch.int32).cuda(), torch.full((3, B), -1, dtype=torch.int32).pin_memory()
+    want = [torch.randint(0, 1000, (B,), generator=g, dtype=torch.int32) for _ in range(5)]
+    for i, new in enumerate(want):
+        _call("core", "fg_decode_advance_host", tokens, pos, new.cuda(), active, B, ring, turn, 3)
+        torch.cuda.synchronize()
+        assert torch.equal(ring[i % 3], new) and torch.equal(tokens.cpu(), new) and turn.item() == (i + 1) % 3
+    assert torch.equal(pos.cpu(), torch.arange(B, dtype=torch.int32) + 5 * active.cpu())
+
+
 def _call(module, name, *args):
     """A launcher that has no Python wrapper: tensors by pointer, Python floats as C floats."""
     import ctypes
