@@ -28,7 +28,7 @@ CSRC_DIR = os.path.dirname(os.path.abspath(__file__))
 
 #: module name -> source files.  Headers every module depends on are listed in HEADERS.
 MODULES = {
-    "core": ["elementwise.cu", "gemm_generic.cu", "attention_generic.cu", "attention_prefill_f32.cu", "sampling.cu"],
+    "core": ["elementwise.cu", "gemm_generic.cu", "attention_generic.cu", "attention_decode_f32.cu", "attention_prefill_f32.cu", "sampling.cu"],
     "tc": ["gemm_tc.cu"],
     "attn": ["attention_decode.cu", "attention_prefill.cu", "attention_prefill_tc.cu"],
     # mixers beyond plain attention: retention and gated linear attention (a state per sequence), what stands between an

@@ -145,12 +145,62 @@ __global__ void rmsnorm_kernel(const float *__restrict__ x, const float *__restr
     }
 }
 
+// The same with a row's numbers in registers, N vectors of four a thread, and the weights fetched before the wait: the row is read once.  The
+// additions are those above.  (What it gives in a step: see attention_decode_f32.cu.)
+template <typename TO, int N>
+__global__ void __launch_bounds__(256)
+rmsnorm_regs_kernel(const float *__restrict__ x, const float *__restrict__ w, const int *__restrict__ rows, TO *__restrict__ out, int E, float eps) {
+    __shared__ float scratch[32];
+    pdl_launch_dependents();
+    const int r = blockIdx.x, n = E / 4;
+    float4 g[N], v[N];
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        const int i = threadIdx.x + j * blockDim.x;
+        g[j] = i < n ? ((const float4 *)w)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    pdl_wait();
+    const float4 *x4 = (const float4 *)(x + (size_t)(rows ? rows[r] : r) * E);
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        const int i = threadIdx.x + j * blockDim.x;
+        v[j] = i < n ? x4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int j = 0; j < N; j++) { ss += v[j].x * v[j].x; ss += v[j].y * v[j].y; ss += v[j].z * v[j].z; ss += v[j].w * v[j].w; }
+    ss = block_sum(ss, scratch);
+    const float inv = 1.0f / sqrtf(ss / (float)E + eps);
+    TO *o = out + (size_t)r * E;
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        const int i = threadIdx.x + j * blockDim.x;
+        if (i < n) store4<TO>(o + 4 * i, v[j].x * inv * g[j].x, v[j].y * inv * g[j].y, v[j].z * inv * g[j].z, v[j].w * inv * g[j].w);
+    }
+}
+
+template <typename TO>
+static int launch_rmsnorm_regs(const float *x, const float *w, const int *rows, TO *out, int R, int E, float eps, int threads, cudaStream_t stream) {
+    const int per = (E / 4 + threads - 1) / threads;
+#define RMS_RUN(N) return fg_launch(rmsnorm_regs_kernel<TO, N>, dim3(R), dim3(threads), 0, stream, x, w, rows, out, E, eps)
+    if (per <= 1) RMS_RUN(1);
+    if (per <= 2) RMS_RUN(2);
+    if (per <= 4) RMS_RUN(4);
+    RMS_RUN(8);
+#undef RMS_RUN
+}
+
 extern "C" int fg_rmsnorm(const float *x, const float *w, const int *rows, void *out, int out_dtype,
                           int R, int E, float eps, cudaStream_t stream) {
     if (R <= 0) return 0;
     bool vec = E % 4 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)w & 15) == 0 && ((uintptr_t)out & 15) == 0;
     int per = vec ? E / 4 : E;
     int threads = per >= 1024 ? 256 : (per >= 256 ? 128 : 64);
+    if (vec && per <= 8 * threads) {
+        if (out_dtype == FG_F32) return launch_rmsnorm_regs<float>(x, w, rows, (float *)out, R, E, eps, threads, stream);
+        if (out_dtype == FG_BF16) return launch_rmsnorm_regs<bf16>(x, w, rows, (bf16 *)out, R, E, eps, threads, stream);
+        return FG_ERR_BAD_DTYPE;
+    }
     if (out_dtype == FG_F32) {
         if (vec) return fg_launch(rmsnorm_kernel<float, true>, dim3(R), dim3(threads), 0, stream, x, w, rows, (float *)out, E, eps);
         return fg_launch(rmsnorm_kernel<float, false>, dim3(R), dim3(threads), 0, stream, x, w, rows, (float *)out, E, eps);

@@ -418,6 +418,23 @@ Tensor rope_attention(Runtime &rt, const Tensor &qkv, const Batch &b, const Laye
             return out;
         }
     }
+    // The same in float32 (attention_decode_f32.cu).
+    if (io.write_cache && b.single_token && a.rotate && !rt.plain_kernels && qkv.dtype == FG_F32 && io.cache_dtype == FG_F32 && a.v_head_dim == hd &&
+        (hd == 16 || hd == 32 || hd == 64 || hd == 128) && io.page_size == 64 && !(a.window > 0 && a.keep_first > 0)) {
+        Tensor out = rt.arena->matrix(qkv.rows, (int64_t)H * hd, FG_F32);
+        const int n_splits = FG_KERNEL("core", fg_attention_decode_f32_splits)(b.n_seq, H, KV, b.table_width, rt.n_sm);
+        count_launch();
+        int code;
+        {
+            ProfileScope scope("fg_attention_decode_f32");
+            code = FG_KERNEL("core", fg_attention_decode_f32)(qkv.data, (int)qkv.ld, out.data, (int)out.ld, b.positions, table, b.table_width, io.k_pool,
+                                                              io.v_pool, cos_t, sin_t, b.n_seq, H, KV, hd, io.page_size, a.scale, a.window, n_splits, rt.stream);
+        }
+        if (code != KERNEL_BAD_SIZE) {
+            check_kernel(code, "fg_attention_decode_f32");
+            return out;
+        }
+    }
     if (!a.rotate) {
         // nothing to rotate: keys and values go to the cache as they are
         if (io.write_cache)

@@ -289,6 +289,52 @@ def test_attention_decode_fused_with_rope_and_append(H, KV, hd, window, n_splits
     assert torch.equal(k2, k1) and torch.equal(v2, v1)          # the cache received the same rows
 
 
+@pytest.mark.parametrize("n_splits", [1, 2, 4, 8])
+@pytest.mark.parametrize("H,KV,hd,window", [(8, 2, 64, 0), (6, 2, 128, 0), (20, 1, 64, 0), (4, 4, 16, 0), (9, 3, 32, 0), (4, 4, 64, 100), (4, 2, 16, 64), (6, 2, 128, 65),
+                                            (8, 1, 64, -200)])
+def test_attention_decode_f32(H, KV, hd, window, n_splits):
+    """One kernel for rotation, cache append and attention of a float32 decode step, against the separate kernels; places of a page that no
+    token has reached hold what is no number."""
+    import ctypes
+    from fastgguf_b200 import ops
+    from fastgguf_b200.ops.lib import lib, ptr, stream
+    lens = [0, 63, 64, 700, 2047, 129]
+    case = make_case(lens, [1] * 6, H, KV, hd, torch.float32, 15)
+    for s, n in enumerate(lens):
+        last = int(case["table"][s, n // PAGE])
+        case["v_pool"][last, :, n % PAGE:] = float("nan")
+        case["k_pool"][last, :, n % PAGE:] = float("inf")
+    g = torch.Generator().manual_seed(16)
+    qkv = torch.randn(6, (H + 2 * KV) * hd, generator=g).cuda()
+    ang = torch.arange(2100, dtype=torch.float64)[:, None] * torch.pow(torch.tensor(10000.0, dtype=torch.float64), -2.0 * torch.arange(hd // 2) / hd)
+    cos, sin = torch.cos(ang).float().cuda(), torch.sin(ang).float().cuda()
+    scale = 1.0 / math.sqrt(hd)
+
+    def both():
+        k1, v1, q1 = case["k_pool"].clone(), case["v_pool"].clone(), qkv.clone()
+        rows = torch.arange(6, dtype=torch.int32).cuda()
+        ops.rope_append(q1, case["positions"], rows, case["table"], k1, v1, cos, sin, H, KV, hd)
+        want = ops.attention_generic(q1, case["positions"], rows, case["table"], k1, v1, H, KV, hd, scale, window)
+        torch.cuda.synchronize()
+        k2, v2, out, f = case["k_pool"].clone(), case["v_pool"].clone(), torch.empty(6, H * hd, device="cuda"), ctypes.c_float
+        torch.cuda.synchronize()
+        assert lib("core").fg_attention_decode_f32(ptr(qkv), qkv.stride(0), ptr(out), out.stride(0), ptr(case["positions"]), ptr(case["table"]),
+                                                   case["table"].shape[1], ptr(k2), ptr(v2), ptr(cos), ptr(sin), 6, H, KV, hd, 64,
+                                                   f(scale), window, n_splits, stream()) == 0
+        assert (k2 - k1).nan_to_num().abs().max() <= 2e-6 and torch.equal(v2.nan_to_num(7.0), v1.nan_to_num(7.0))
+        return out, want
+
+    out, want = both()
+    assert _err(out, want.double().cpu()) < 5e-6
+    # numbers that are none, or infinite, at places that tokens see
+    case["k_pool"][int(case["table"][3, 10]), 0, 5, 1] = float("nan")
+    case["k_pool"][int(case["table"][4, 30]), 0, 60, 1] = float("inf")
+    case["v_pool"][int(case["table"][5, 1]), 0, 60, 1] = float("inf")
+    bad, bad_want = both()
+    assert torch.equal(bad.isfinite(), bad_want.isfinite()) and torch.equal(bad.isnan(), bad_want.isnan())
+    assert torch.equal(bad[:3], out[:3])
+
+
 @pytest.mark.parametrize("H,KV,hd", [(8, 2, 64), (4, 1, 128)])
 def test_attention_prefill_tcgen05_growing_maximum(H, KV, hd):
     """Scores that grow by tens of binary orders every 128 keys: every iteration moves the running base, and
