@@ -108,7 +108,7 @@ __device__ __forceinline__ bool elect_one() {
 // only memory that nothing launched since the last full barrier of the stream writes - a full barrier
 // being a memory copy, or the boundary of a graph launch.  Weights qualify always.  Positions, page
 // tables and an entry's own cache pool qualify for the fused decode attention because the engine writes
-// positions and tables only by the copy that opens a step or by `decode_advance_kernel`, the LAST
+// positions and tables only by the copy that opens a step or by `decode_advance_host_kernel`, the LAST
 // node of the decode graph, and because an entry's pool is appended to by that entry's kernel alone.
 // FASTGGUF_PDL=0 turns the attribute off; the two instructions are then no-ops.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
