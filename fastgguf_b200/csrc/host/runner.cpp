@@ -119,23 +119,25 @@ Sampler::Sampler(const SamplingParams &p, int n_slots, const std::vector<int> &s
       stream_(stream) {
     p.validate();
     std::vector<uint64_t> init((size_t)n_rows_, 0x9E3779B97F4A7C15ull);
+    // (everything on the engine's own stream: it does not wait for the default stream, so what is set up there could land late)
     rng_ = DeviceBuffer((size_t)n_rows_ * 8, "sampler state");
-    FG_CUDA(cudaMemcpy(rng_.get(), init.data(), init.size() * 8, cudaMemcpyHostToDevice));
+    FG_CUDA(cudaMemcpyAsync(rng_.get(), init.data(), init.size() * 8, cudaMemcpyHostToDevice, stream));
     if (use_hist_) {
         hist_ = DeviceBuffer((size_t)n_rows_ * hist_cap_ * 4, "sampler history");
         hist_count_ = DeviceBuffer((size_t)n_rows_ * 4, "sampler history");
-        FG_CUDA(cudaMemset(hist_.get(), 0, hist_.bytes()));
-        FG_CUDA(cudaMemset(hist_count_.get(), 0, hist_count_.bytes()));
+        FG_CUDA(cudaMemsetAsync(hist_.get(), 0, hist_.bytes(), stream));
+        FG_CUDA(cudaMemsetAsync(hist_count_.get(), 0, hist_count_.bytes(), stream));
     }
     n_stop_ = (int)stop_ids.size();
     if (n_stop_) {
         stop_ = DeviceBuffer((size_t)n_stop_ * 4, "stop ids");
-        FG_CUDA(cudaMemcpy(stop_.get(), stop_ids.data(), (size_t)n_stop_ * 4, cudaMemcpyHostToDevice));
+        FG_CUDA(cudaMemcpyAsync(stop_.get(), stop_ids.data(), (size_t)n_stop_ * 4, cudaMemcpyHostToDevice, stream));
     }
     // 4096 words a batch row: the candidates of the two-stage top-k, or (greedy) the two words in which the blocks
     // of a row meet.  Owned by this sampler, so samplers of other engines or streams share nothing with it.
     scratch_ = DeviceBuffer((size_t)bucket_for(std::max(1, n_slots)) * 4096 * 8, "sampler scratch");
-    FG_CUDA(cudaMemset(scratch_.get(), 0, scratch_.bytes()));
+    FG_CUDA(cudaMemsetAsync(scratch_.get(), 0, scratch_.bytes(), stream));
+    FG_CUDA(cudaStreamSynchronize(stream));
 }
 
 void Sampler::begin(int row, uint64_t state, const int *prompt, int prompt_len) {
@@ -172,8 +174,10 @@ DecodeGraph::DecodeGraph(Engine &e, Sampler &sampler, int width_) : width(width_
     std::vector<size_t> offs;
     size_t total = 0;
     for (size_t sz : sizes) { offs.push_back(total); total += pad(sz); }
+    // Set up on the stream that replays: it does not wait for the default stream, and a `turn` zeroed there after the first replay
+    // would leave host and device at different regions for good.
     ints_ = DeviceBuffer(total * 4, "decode graph buffers");
-    FG_CUDA(cudaMemset(ints_.get(), 0, total * 4));
+    FG_CUDA(cudaMemsetAsync(ints_.get(), 0, total * 4, e.stream));
     int *base = (int *)ints_.get();
     tokens = base + offs[0]; positions = base + offs[1]; row_seq = base + offs[2]; cu_rows = base + offs[3];
     rows = base + offs[4]; want = base + offs[5]; active = base + offs[6]; next_tokens = base + offs[7];
@@ -181,11 +185,11 @@ DecodeGraph::DecodeGraph(Engine &e, Sampler &sampler, int width_) : width(width_
     for (int g = 0; g < n_groups; g++) tables.push_back(base + offs[10 + (size_t)g]);
     std::vector<int> ar((size_t)B + 1), spare((size_t)B, sampler.spare_row);
     for (int i = 0; i <= B; i++) ar[(size_t)i] = i;
-    FG_CUDA(cudaMemcpy(row_seq, ar.data(), (size_t)B * 4, cudaMemcpyHostToDevice));
-    FG_CUDA(cudaMemcpy(cu_rows, ar.data(), ((size_t)B + 1) * 4, cudaMemcpyHostToDevice));
-    FG_CUDA(cudaMemcpy(want, ar.data(), (size_t)B * 4, cudaMemcpyHostToDevice));
-    FG_CUDA(cudaMemcpy(rows, spare.data(), (size_t)B * 4, cudaMemcpyHostToDevice));
-    FG_CUDA(cudaMemcpy(spare_cell, spare.data(), 4, cudaMemcpyHostToDevice));
+    FG_CUDA(cudaMemcpyAsync(row_seq, ar.data(), (size_t)B * 4, cudaMemcpyHostToDevice, e.stream));
+    FG_CUDA(cudaMemcpyAsync(cu_rows, ar.data(), ((size_t)B + 1) * 4, cudaMemcpyHostToDevice, e.stream));
+    FG_CUDA(cudaMemcpyAsync(want, ar.data(), (size_t)B * 4, cudaMemcpyHostToDevice, e.stream));
+    FG_CUDA(cudaMemcpyAsync(rows, spare.data(), (size_t)B * 4, cudaMemcpyHostToDevice, e.stream));
+    FG_CUDA(cudaMemcpyAsync(spare_cell, spare.data(), 4, cudaMemcpyHostToDevice, e.stream));
     upload_cap = std::max<size_t>(16, (size_t)B * table_width * (size_t)std::max(1, n_groups));
     regions.resize(4);
     FG_CUDA(cudaMallocHost((void **)&host_tokens_, regions.size() * B * 4));
@@ -208,10 +212,10 @@ DecodeGraph::DecodeGraph(Engine &e, Sampler &sampler, int width_) : width(width_
     long long before = launch_count();
     run(e.stream, false);
     launches_per_step = launch_count() - before;
+    FG_CUDA(cudaMemsetAsync(tokens, 0, (size_t)B * 4, e.stream));
+    FG_CUDA(cudaMemsetAsync(positions, 0, (size_t)B * 4, e.stream));
+    FG_CUDA(cudaMemsetAsync(turn, 0, 4, e.stream));
     FG_CUDA(cudaStreamSynchronize(e.stream));
-    FG_CUDA(cudaMemset(tokens, 0, (size_t)B * 4));
-    FG_CUDA(cudaMemset(positions, 0, (size_t)B * 4));
-    FG_CUDA(cudaMemset(turn, 0, 4));
     arena_.reset();                                  // one block for what the warm-up needed
     arena_.forbid_growth(true);
     FG_CUDA(cudaStreamBeginCapture(e.capture_stream, cudaStreamCaptureModeRelaxed));
@@ -443,6 +447,7 @@ Engine::Engine(const ModelSpec &spec, const EngineOptions &o, const TensorSource
     model = std::make_unique<DecoderModel>(spec, o.dtype, o.device, stream);
     model->load_weights(source, seed_random, seed);
     model->make_cache(o.max_tokens, o.max_batch, o.max_seq_len, 64, o.verbose);
+    FG_CUDA(cudaStreamSynchronize(cudaStreamLegacy));      // caches and states are zeroed on the default stream, for which this engine's does not wait
 }
 
 Engine::~Engine() {

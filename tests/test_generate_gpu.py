@@ -254,3 +254,36 @@ def test_float32_steps_where_device_memory_is_short():
     assert planes and np.array_equal(portions, want)
     plain, planes = logits(gib - (100 << 20))
     assert not planes and 0 < np.abs(plain - want).max() <= 1e-5 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_a_busy_default_stream_changes_nothing(models, dtype):
+    """The engine's stream does not wait for the default stream.  Whatever an engine, a sampler and a recorded step set up before their first
+    use is therefore queued on the engine's own stream: a thread that keeps the default stream milliseconds behind must not delay it."""
+    import threading
+    from fastgguf_b200.engine.api import Engine
+    d, cfg, _ = models["b"]
+    prompts = [random_tokens(n, cfg["vocab_size"], 70 + i) for i, n in enumerate([9, 30, 2])]
+
+    def outputs():
+        engine = Engine.from_dir(d, dtype=dtype, max_tokens=1024, max_batch=4)
+        return [[c.tokens for c in engine.generate(prompts, temp=t, top_k=20, top_p=0.9, repeat_penalty=1.2, seed=3, max_tokens=12, ignore_eos=True)]
+                for t in (0, 0.7)]
+
+    want, stop, idle = outputs(), threading.Event(), torch.cuda.Event()
+
+    def keep_busy():
+        while not stop.is_set():
+            for _ in range(8):
+                torch.cuda._sleep(2_000_000)                  # about a millisecond each
+            idle.record()
+            idle.synchronize()
+
+    t = threading.Thread(target=keep_busy)
+    t.start()
+    try:
+        got = [outputs() for _ in range(3)]
+    finally:
+        stop.set()
+        t.join()
+    assert all(g == want for g in got)
