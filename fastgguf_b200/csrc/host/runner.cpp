@@ -376,7 +376,9 @@ int DecodeSession::advance(const std::vector<int> &live) {
     std::vector<std::pair<int, int>> steps;
     std::vector<char> is_live((size_t)n_, 0);
     for (int i : live) {
+        // (before anything is queued: a call that fails halfway would leave copies in flight from an upload region that the next call fills)
         if (i < 0 || i >= n_) fail(FG_E_USAGE, format("sequence %d is not in this batch of %d", i, n_));
+        if (widths_[(size_t)i] < 0) fail(FG_E_USAGE, format("sequence %d has left this batch", i));
         steps.emplace_back(slots[(size_t)i], 1);
         is_live[(size_t)i] = 1;
     }
@@ -396,7 +398,6 @@ int DecodeSession::advance(const std::vector<int> &live) {
     size_t used = 0;
     std::vector<int> row((size_t)g.table_width);
     for (int i : live) {                                             // upload page-table entries the step will touch
-        if (widths_[(size_t)i] < 0) fail(FG_E_USAGE, format("sequence %d has left this batch", i));
         int need = (cache.length(slots[(size_t)i]) + 1 + cache.page_size - 1) / cache.page_size;
         if (need > widths_[(size_t)i]) {
             int have = widths_[(size_t)i];
@@ -415,9 +416,9 @@ int DecodeSession::advance(const std::vector<int> &live) {
     }
     g.replay();
     g.next_region = (idx + 1) % (int)g.regions.size();               // (the device's count moves on with the replay)
+    FG_CUDA(cudaEventRecord(region.done, s));
     cache.commit(steps);
     eng.stats.steps++;
-    FG_CUDA(cudaEventRecord(region.done, s));
     eng.stats.d2h_bytes += 4LL * g.width;
     return idx;
 }

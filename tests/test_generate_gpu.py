@@ -287,3 +287,29 @@ def test_a_busy_default_stream_changes_nothing(models, dtype):
         stop.set()
         t.join()
     assert all(g == want for g in got)
+
+
+def test_a_session_step_that_is_refused_queues_nothing(models):
+    """A step that names a sequence which has left its batch is refused before page-table entries are on their way to the device, and the
+    steps behind it find what they would have found without it."""
+    from fastgguf_b200.engine.api import Engine
+    from fastgguf_b200.engine.batch import StepEntry
+    from fastgguf_b200 import SamplingParams
+    d, cfg, _ = models["b"]
+    prompts = [random_tokens(n, cfg["vocab_size"], 80 + i) for i, n in enumerate([61, 5, 62])]
+
+    def run(with_refused_calls):
+        engine = Engine.from_dir(d, dtype="float32", max_tokens=2048, max_batch=4)
+        session = engine.session(prompts, SamplingParams(temp=0.0))
+        session.advance([0, 1, 2])
+        for step in range(70):                               # sequences 0 and 2 come to new pages one step after the other
+            session.advance([0, 2])
+            if with_refused_calls:
+                before = engine.stats()
+                with pytest.raises(Exception, match="left this batch"):
+                    session.advance([0, 2, 1])
+                assert engine.stats() == before
+        slots = [session.slots[0], session.slots[2]]
+        return engine.step_host([StepEntry(s, [7, 8], [0, 1]) for s in slots])
+
+    assert np.array_equal(run(True), run(False))
