@@ -118,7 +118,8 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // first weights meanwhile.  In a larger step they are the persistent tensor-memory kernels: a short kernel that released its
 // successor at its start and then sat resident, waiting, let the second contraction start beside the first, and now and then
 // a prompt step never finished (a hardware wait: every wait of these kernels' own is bounded).  There the successor is
-// released when the row-wise kernel ends.
+// released when the row-wise kernel ends.  The kernels that walk a recurrence token by token stand there too; they take the rows
+// from the end of the step's row offsets, and a prompt's chunk kernels in front of an output projection release at their end.
 // Kernels that stand next to ATTENTION cannot go by the rows: a prompt of 16 tokens already runs the tensor-memory attention kernel
 // (64 rows of token x query head).  They, and others that such a step may run between two tensor-memory kernels, take `early`
 // from the host, which sets it at up to 64 rows of one token a sequence (attention without tensor memory) and in float32 engines

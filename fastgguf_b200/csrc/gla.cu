@@ -37,7 +37,7 @@ gla_seq_kernel(const float *__restrict__ proj, int ld, const float *__restrict__
                float eps) {
     extern __shared__ float sm[];
     __shared__ float scratch[32];
-    pdl_launch_dependents();
+    pdl_launch_dependents_small_step(cu_rows[gridDim.x]);          // (all rows of the step: sequences may bring several)
     pdl_wait();
     const int seq = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
     const int row0 = cu_rows[seq], row1 = cu_rows[seq + 1];
@@ -203,8 +203,7 @@ gla_chunk_out_kernel(const float *__restrict__ proj, int ld, const float *__rest
                      const int *__restrict__ chunk_len, const float *__restrict__ P, const float *__restrict__ Bg, int H, int dk, int dv,
                      float inv_tau, float q_scale, float eps) {
     extern __shared__ __align__(16) float sm[];
-    pdl_launch_dependents();
-    pdl_wait();
+    pdl_wait();                                  // (no early release: the output projection must not start beside the projection in front)
     const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
     const int r0 = chunk_row[c], n = chunk_len[c];
     // b, qs, ks: [GC][dk]; qd: [dk][GC] = q_t * exp(b_t), zero beyond n; AT: [GC (u)][GC (t)] = A[t][u], zero where u > t

@@ -101,7 +101,7 @@ retention_seq_kernel(const float *__restrict__ proj, int ld, TO *__restrict__ ou
                      int dv_all, float k_scale, float eps, int opts, int slab) {
     extern __shared__ float sm[];
     __shared__ float scratch[32];
-    pdl_launch_dependents();
+    pdl_launch_dependents_small_step(cu_rows[gridDim.x]);          // (all rows of the step: sequences may bring several)
     pdl_wait();
     const int seq = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
     const int row0 = cu_rows[seq], row1 = cu_rows[seq + 1];
@@ -164,7 +164,7 @@ retention_regs_kernel(const float *__restrict__ proj, int ld, TO *__restrict__ o
                       const float *__restrict__ sin_t, const float *__restrict__ decay, float *state, int H, float k_scale, float eps, int opts) {
     constexpr int G = RET_THREADS / DV, RPT = DK / G, half = DK / 2;
     __shared__ float qs[DK], ks[DK], vs[DV], part[RET_THREADS], scratch[32];
-    pdl_launch_dependents();
+    pdl_launch_dependents_small_step(cu_rows[gridDim.x]);
     if (!AHEAD) pdl_wait();
     const int seq = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, j = tid % DV, g = tid / DV;
     float *Sg = state + ((size_t)slots[seq] * H + h) * DK * DV + (size_t)g * DV + j;
@@ -318,8 +318,7 @@ retention_chunk_out_kernel(const float *__restrict__ proj, int ld, TO *__restric
                            const float *__restrict__ sin_t, const float *__restrict__ decay, const float *__restrict__ U, int H,
                            int dk, int dv, float k_scale, float eps, int opts) {
     extern __shared__ float sm[];
-    pdl_launch_dependents();
-    pdl_wait();
+    pdl_wait();                                  // (no early release: the output projection must not start beside the projection in front)
     const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
     const int r0 = chunk_row[c], n = chunk_len[c];
     const int dkp = dk + 1;                      // padded rows: threads of a warp read different rows of Q / K
@@ -446,8 +445,7 @@ retention_chunk_out_fast(const float *__restrict__ proj, int ld, TO *__restrict_
     constexpr int NJ = DV / 4, NI = RET_THREADS / NJ, TT = RC / NI, DKP = DK + 4;
     extern __shared__ __align__(16) float sm[];
     float *Q = sm, *K = Q + RC * DKP, *V = K + RC * DKP, *A = V + RC * DV;       // Q, K: [RC][DKP]; V: [RC][DV]; A: [RC][RC]
-    pdl_launch_dependents();
-    pdl_wait();
+    pdl_wait();                                  // (no early release: the output projection must not start beside the projection in front)
     const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
     const int r0 = chunk_row[c], n = chunk_len[c];
     const float l2 = log2f(decay[h]);

@@ -22,6 +22,21 @@ def test_kernels_beside_attention_do_not_go_by_the_number_of_rows():
             assert re.sub(r"if \(early\) pdl_launch_dependents\(\);", "", body).count("pdl_launch_dependents") == 0, k
 
 
+def test_recurrences_release_the_output_projection_early_in_small_steps_alone():
+    """The last kernel of a recurrence stands between two contractions.  In a step of more than 64 rows both hold tensor memory, and one that
+    released its successor at its start would let the second start beside the first.  How many rows a step has is not its number of
+    sequences, which is the grid of the token-by-token kernels."""
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "fastgguf_b200", "csrc")
+    for name, by_rows, at_the_end in (("retention.cu", ("retention_seq_kernel", "retention_regs_kernel"), ("retention_chunk_out_kernel", "retention_chunk_out_fast")),
+                                      ("gla.cu", ("gla_seq_kernel",), ("gla_chunk_out_kernel",))):
+        with open(os.path.join(csrc, name)) as f:
+            text = f.read()
+        for k in by_rows + at_the_end:
+            body = text[text.index(k + "(const"):]
+            body = body[:body.index("row0 = " if k in by_rows else "const int c =")]
+            assert re.findall(r"pdl_launch_dependents\w*\([^;]*;", body) == ["pdl_launch_dependents_small_step(cu_rows[gridDim.x]);"] * (k in by_rows), k
+
+
 def _saluzen():
     from saluzen_cases import attn, config, delta, dense, latent, parallel, parallel_2, ssm
     left = dict(heads=16, kv_heads=4, dim=64, vdim=64, scale=0.125)
@@ -68,6 +83,46 @@ def test_many_short_prompt_steps_back_to_back(case):
         if i % 4 == 0:
             first = got if first is None else first
             assert np.array_equal(got, first)
+        if i % 10 == 0:
+            assert np.isfinite(eng.step_host([StepEntry(s, draw(1), [0]) for s in slots])).all()
+        for s in slots:
+            eng.release(s)
+    eng.cache.check()
+
+
+def _zirivik():
+    from zirivik_cases import config, dense, retention
+    decay = [1.0 - 2.0 ** (-5 - h / 2) for h in range(8)]
+    return config(1024, 4096, [(retention(8, 128, 128, decay, (10000.0, 64)), dense(4096)), (retention(8, 64, 64, decay), dense(4096))] * 2)
+
+
+def _salulorn():
+    from salulorn_cases import config, dense, gla
+    return config(512, 2048, [(gla(8, 64, 64, 16.0, 16), dense(1024))] * 4)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", [_zirivik, _salulorn])
+def test_many_steps_of_many_short_portions(case, tmp_path):
+    """One hundred and fifty steps of 8 to 80 sequences with 2 to 15 tokens each, more than 64 rows in all, which the token-by-token kernels
+    walk between two tensor-memory contractions, every tenth followed by a step of one token for each: all end with finite logits."""
+    from fastgguf_b200.engine.api import Engine
+    from fastgguf_b200.engine.batch import StepEntry
+    from fastgguf_b200.registry import config_from_dict
+    room = dict(dtype="bfloat16", max_tokens=16384, max_batch=80, max_seq_len=256)
+    if case is _salulorn:                                    # (the rank of a decay is a shape of its weights)
+        import salulorn_cases
+        eng = Engine.from_dir(salulorn_cases.make_model(tmp_path, case(), 3)[0], **room)
+    else:
+        eng = Engine.from_random(config_from_dict(case()), 3, **room)
+    rng = np.random.default_rng(6)
+    draw = lambda n: [int(t) for t in rng.integers(0, 2048, size=n)]  # noqa: E731
+    for i in range(150):
+        lengths = rng.integers(2, 16, size=int(rng.integers(8, 81)))
+        lengths[0] += max(0, 65 - int(lengths.sum())) if i % 2 else 0
+        toks = [draw(int(n)) for n in lengths]
+        slots = [eng.acquire() for _ in toks]
+        assert np.isfinite(eng.step_host([StepEntry(s, t, [len(t) - 1]) for s, t in zip(slots, toks)])).all()
         if i % 10 == 0:
             assert np.isfinite(eng.step_host([StepEntry(s, draw(1), [0]) for s in slots])).all()
         for s in slots:
