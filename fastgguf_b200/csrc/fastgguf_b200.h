@@ -80,11 +80,15 @@ int fg_attention_generic(const void *q, int ldq, void *out, int ldo, int dtype, 
                          const void *v_pool, int M, int H, int KV, int hd, int page_size, float scale, int window,
                          cudaStream_t stream);
 /* decode in float32, one new token a sequence: rotation, cache append and attention in one kernel (head sizes 16, 32, 64, 128, pages of 64);
-   n_splits 1, 2, 4 or 8, fg_attention_decode_f32_splits names the one that fills the GPU */
+   n_splits 1, 2, 4 or 8, fg_attention_decode_f32_splits names the one that fills the GPU; warps a CTA (0: by the step's shape).  A row's bits
+   depend on neither */
 int fg_attention_decode_f32_splits(int B, int H, int KV, int table_width, int n_sm);
 int fg_attention_decode_f32(const void *qkv, int ldq, void *out, int ldo, const int *positions, const int *block_table, int table_width,
                             void *k_pool, void *v_pool, const float *cos_t, const float *sin_t, int B, int H, int KV, int hd, int page_size,
                             float scale, int window, int n_splits, cudaStream_t stream);
+int fg_attention_decode_f32_ext(const void *qkv, int ldq, void *out, int ldo, const int *positions, const int *block_table, int table_width,
+                                void *k_pool, void *v_pool, const float *cos_t, const float *sin_t, int B, int H, int KV, int hd, int page_size,
+                                float scale, int window, int n_splits, int warps, cudaStream_t stream);
 /* prefill in float32 on the tensor cores, by bfloat16 planes: head sizes 64 and 128, pages of 64 (arguments as fg_attention_prefill) */
 int fg_attention_prefill_f32(const void *q, int ldq, void *out, int ldo, const int *cu_rows, const int *seq_start,
                              const int *block_table, int table_width, const void *k_pool, const void *v_pool, int n_seq,

@@ -347,3 +347,82 @@ def test_attention_prefill_tcgen05_growing_maximum(H, KV, hd):
     assert fast_attention.prefill_tc_error() == 0
     want = plain(case, H, KV, hd, scale, 0)
     assert (got.double().cpu() - want).abs().max().item() <= 2e-2 * want.abs().max().item()
+
+
+def _decode_f32(case, qkv, cos, sin, H, KV, hd, window, n_splits, warps, rows=None, width=None):
+    """fg_attention_decode_f32_ext over copies of the pools, for the sequences `rows` with a page table of `width` entries."""
+    import ctypes
+    from fastgguf_b200.ops.lib import lib, ptr, stream
+    rows = list(range(qkv.shape[0])) if rows is None else rows
+    table, pos, x = case["table"][rows], case["positions"][rows].contiguous(), qkv[rows].contiguous()
+    table = torch.cat([table, torch.zeros(len(rows), (width or table.shape[1]) - table.shape[1], dtype=torch.int32, device="cuda")], 1).contiguous()
+    k, v, out, f = case["k_pool"].clone(), case["v_pool"].clone(), torch.empty(len(rows), H * hd, device="cuda"), ctypes.c_float
+    torch.cuda.synchronize()
+    assert lib("core").fg_attention_decode_f32_ext(ptr(x), x.stride(0), ptr(out), out.stride(0), ptr(pos), ptr(table), table.shape[1], ptr(k), ptr(v), ptr(cos),
+                                                   ptr(sin), len(rows), H, KV, hd, 64, f(1.0 / math.sqrt(hd)), window, n_splits, warps, stream()) == 0
+    torch.cuda.synchronize()
+    return out, k, v
+
+
+def _decode_f32_case(lens, H, KV, hd, seed, turned=True):
+    case = make_case(lens, [1] * len(lens), H, KV, hd, torch.float32, seed)
+    qkv = torch.randn(len(lens), (H + 2 * KV) * hd, generator=torch.Generator().manual_seed(seed + 1)).cuda()
+    ang = torch.arange(max(lens) + 1, dtype=torch.float64)[:, None] * torch.pow(torch.tensor(10000.0, dtype=torch.float64), -2.0 * torch.arange(hd // 2) / hd)
+    return case, qkv, torch.cos(ang * turned).float().cuda(), torch.sin(ang * turned).float().cuda()
+
+
+@pytest.mark.parametrize("H,KV,hd,window", [(8, 2, 64, 0), (4, 2, 64, 0), (2, 2, 64, 100), (6, 1, 128, 0), (2, 1, 128, 65), (1, 1, 128, 0), (8, 2, 32, 0), (3, 3, 32, -200),
+                                            (4, 2, 16, 0), (6, 2, 16, 33), (5, 5, 16, 0)])
+def test_attention_decode_f32_does_not_depend_on_the_step(H, KV, hd, window):
+    """A row's bits follow from its own sequence: alone or beside others, with any number of CTAs and warps and any width of the page table.
+    Lengths around the edges of units, of runs of one and two units, and of more than 64 runs."""
+    lens = [0, 31, 32, 63, 64, 97, 129, 1023, 1024, 1055, 2047, 2048, 2100, 4200]
+    case, qkv, cos, sin = _decode_f32_case(lens, H, KV, hd, 21)
+    want, want_k, want_v = _decode_f32(case, qkv, cos, sin, H, KV, hd, window, 1, 2)
+    assert want.isfinite().all()
+    for n_splits in (1, 2, 4, 8):
+        for warps in (0, 2, 4) + ((8,) if hd < 128 else ()):
+            got, k, v = _decode_f32(case, qkv, cos, sin, H, KV, hd, window, n_splits, warps)
+            assert torch.equal(got, want) and torch.equal(k, want_k) and torch.equal(v, want_v), (n_splits, warps)
+    for i in (0, 2, 5, 8, 13):
+        assert torch.equal(_decode_f32(case, qkv, cos, sin, H, KV, hd, window, 8, 0, rows=[i], width=90)[0][0], want[i])
+
+
+@pytest.mark.parametrize("H,KV,hd", [(8, 2, 64), (4, 4, 64), (8, 2, 128), (4, 2, 32), (4, 2, 16)])
+def test_attention_decode_f32_is_as_near_to_float64_as_the_any_size_kernel(H, KV, hd):
+    """Without rotation (cosines of one), so that both kernels and float64 have the same queries, keys and scores.  The 2-norm of the error over
+    sequences of three length classes: sums of 16 values added up in a tree against eight runs of up to 128 in a chain."""
+    from fastgguf_b200 import ops
+    errors, size = [0.0, 0.0], 0.0
+    for seed in range(23, 35, 2):
+        for lens in ([20 + 3 * i for i in range(48)], [150 + 9 * i for i in range(48)], [1100 + 20 * i for i in range(48)]):
+            case, qkv, cos, sin = _decode_f32_case(lens, H, KV, hd, seed, turned=False)
+            got, k, v = _decode_f32(case, qkv, cos, sin, H, KV, hd, 0, 1, 0)
+            any_size = ops.attention_generic(qkv[:, :H * hd].contiguous(), case["positions"], torch.arange(48, dtype=torch.int32).cuda(), case["table"], k, v, H, KV,
+                                             hd, 1.0 / math.sqrt(hd), 0)
+            for b, n in enumerate(lens):
+                pages = case["table"][b, :n // PAGE + 1].long()
+                K, V = (x[pages].double().transpose(1, 2).reshape(-1, KV, hd)[:n + 1].repeat_interleave(H // KV, 1) for x in (k, v))
+                p = torch.softmax(torch.einsum("hd,khd->hk", qkv[b, :H * hd].double().view(H, hd), K) / math.sqrt(hd), -1)
+                want = torch.einsum("hk,khd->hd", p, V).flatten()
+                errors = [e + (x[b].double() - want).square().sum() for e, x in zip(errors, (got, any_size))]
+                size = size + want.square().sum()
+    ours, other = (math.sqrt(float(e / size)) for e in errors)
+    assert ours <= other, (ours, other)
+
+
+@pytest.mark.parametrize("hd", [16, 128])
+@pytest.mark.parametrize("power", [-140, -30, 12, 17, 18, 19, 30, 100])
+def test_attention_decode_f32_over_the_range_of_scores(power, hd):
+    """Scores of 2^-140 to 2^100, around 2^20 with both kinds of bases in one row, against the any-size kernel, which has the same scores: every
+    weight is off by a few units in the last place (expf, its argument), so the output by less than 16 * 2^-24 of the largest value."""
+    from fastgguf_b200 import ops
+    H, KV, lens = 8, 2, [3, 40, 100, 500, 2200]
+    case, qkv, cos, sin = _decode_f32_case(lens, H, KV, hd, 29, turned=False)
+    qkv[:, :H * hd] *= 2.0 ** power
+    got, k, v = _decode_f32(case, qkv, cos, sin, H, KV, hd, 0, 1, 0)
+    want = ops.attention_generic(qkv[:, :H * hd].contiguous(), case["positions"], torch.arange(5, dtype=torch.int32).cuda(), case["table"], k, v, H, KV, hd,
+                                 1.0 / math.sqrt(hd), 0)
+    assert got.isfinite().all() and (got - want).abs().max() <= 16 * 2.0 ** -24 * v.abs().max()
+    for n_splits, warps in ((8, 4), (2, 2)):
+        assert torch.equal(_decode_f32(case, qkv, cos, sin, H, KV, hd, 0, n_splits, warps)[0], got)
