@@ -695,8 +695,7 @@ static int launch_prefill_f32(const float *q, int ldq, float *out, int ldo, cons
 
 // q: [rows, ldq] float32 rows of all sequences one after another (cu_rows[b] = first row of sequence b, seq_start[b] = its length
 // before the step); pools [pages, KV, 64, hd] float32; out [rows, ldo] float32.  max_new: most rows any sequence brings.
-// skip_few > 0: sequences that f32_few_rows names with pairs = skip_few are left out (the any-size kernel has them); 1 stands for 2,048 (1,536 at
-// head size 128).
+// skip_few > 0: sequences that f32_few_rows names with pairs = skip_few are left out (the any-size kernel has them).
 // Refuses (FG_ERR_BAD_SIZE) other head sizes and pages and rows that are not 16-byte aligned; the any-size kernel takes those.
 extern "C" int fg_attention_prefill_f32_ext(const void *q, int ldq, void *out, int ldo, const int *cu_rows, const int *seq_start,
                                             const int *block_table, int table_width, const void *k_pool, const void *v_pool, int n_seq,
@@ -708,7 +707,7 @@ extern "C" int fg_attention_prefill_f32_ext(const void *q, int ldq, void *out, i
         return FG_ERR_BAD_SIZE;
 #define PF32_RUN(HD) launch_prefill_f32<HD>((const float *)q, ldq, (float *)out, ldo, cu_rows, seq_start, block_table, table_width, \
                                             (const float *)k_pool, (const float *)v_pool, n_seq, max_new, H, KV, scale, window, \
-                                            skip_few == 1 ? (HD == 64 ? 2048 : 1536) : skip_few, stream)
+                                            skip_few, stream)
     if (hd == 64) return PF32_RUN(64);
     if (hd == 128) return PF32_RUN(128);
 #undef PF32_RUN
@@ -722,10 +721,7 @@ extern "C" int fg_attention_prefill_f32(const void *q, int ldq, void *out, int l
                                         page_size, scale, window, 0, stream);
 }
 
-extern "C" int fg_attention_f32_few_rows(int tokens, int past, int heads, int hd, int window) {
-    return f32_few_rows(tokens, past, heads, window, hd == 64 ? 2048 : 1536);
-}
-// the same by the times of this kernel: skip_few for fg_attention_prefill_f32_ext, and whether it leaves a sequence out
+// skip_few for fg_attention_prefill_f32_ext by the times of both kernels, and whether it leaves a sequence out
 extern "C" int fg_attention_f32_skip_few(int hd) { return f32_pairs(hd); }
 extern "C" int fg_attention_f32_left_out(int tokens, int past, int heads, int hd, int window) { return f32_few_rows(tokens, past, heads, window, f32_pairs(hd)); }
 

@@ -93,8 +93,8 @@ int fg_attention_decode_f32_ext(const void *qkv, int ldq, void *out, int ldo, co
 int fg_attention_prefill_f32(const void *q, int ldq, void *out, int ldo, const int *cu_rows, const int *seq_start,
                              const int *block_table, int table_width, const void *k_pool, const void *v_pool, int n_seq,
                              int max_new, int H, int KV, int hd, int page_size, float scale, int window, cudaStream_t stream);
-/* the same with skip_few: without the sequences of few new tokens, where `pairs` in f32_few_rows (attention_prefill_f32.cu) is skip_few, 1: those that
-   fg_attention_f32_few_rows names, fg_attention_f32_skip_few(hd): those that fg_attention_f32_left_out names; and what each kernel takes */
+/* the same with skip_few (0: all sequences): without the sequences of few new tokens, `pairs` in f32_few_rows (attention_prefill_f32.cu) being skip_few;
+   fg_attention_f32_skip_few(hd): those that fg_attention_f32_left_out names; and what each kernel takes */
 int fg_attention_prefill_f32_ext(const void *q, int ldq, void *out, int ldo, const int *cu_rows, const int *seq_start,
                                  const int *block_table, int table_width, const void *k_pool, const void *v_pool, int n_seq,
                                  int max_new, int H, int KV, int hd, int page_size, float scale, int window, int skip_few, cudaStream_t stream);
@@ -102,7 +102,6 @@ int fg_attention_prefill_f32_ext(const void *q, int ldq, void *out, int ldo, con
    ordinary one; skip_scores: a kernel's first scores are never computed) */
 int fg_attention_prefill_f32_error(void);
 int fg_attention_prefill_f32_test_hook(long long wait_limit_cycles, int skip_scores);
-int fg_attention_f32_few_rows(int tokens, int past, int heads, int hd, int window);
 int fg_attention_f32_skip_few(int hd);
 int fg_attention_f32_left_out(int tokens, int past, int heads, int hd, int window);
 int fg_attention_f32_cost(int tokens, int past, int H, int KV, int hd, int window, int n_sm, double *any_size, double *tiles, double *walk);

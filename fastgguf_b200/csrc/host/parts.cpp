@@ -308,7 +308,7 @@ struct F32AttentionSplit {
 static F32AttentionSplit split_f32_attention(const Batch &b, int H, int KV, int hd, int window, int n_sm) {
     F32AttentionSplit s;
     if ((int)b.host_cu_rows.size() <= b.n_seq || (int)b.host_seq_start.size() < b.n_seq) {      // the host does not know the lengths
-        s.tiles = (long long)b.max_new * H >= 4096;
+        s.tiles = !FG_KERNEL("core", fg_attention_f32_left_out)(b.max_new, std::max(0, b.max_len - b.max_new), H, hd, window);
         return s;
     }
     const auto cost = FG_KERNEL("core", fg_attention_f32_cost);            // (looked up once: a step of many sequences asks often)

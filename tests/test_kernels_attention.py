@@ -175,26 +175,28 @@ def test_attention_prefill_f32_outside_the_range_of_the_planes(what, hd):
         assert y > 0 and abs(x - y) <= 2 * hd * 84 * 2.0 ** -24 * y
 
 
-def test_attention_prefill_f32_leaves_out_sequences_of_few_rows():
-    """With skip_few the rows of every sequence that the rule names keep what the output held, all others have their values."""
+@pytest.mark.parametrize("hd,window,few", [(64, 0, "-x-x-xxx"), (64, 100, "-x-x-xxx"), (64, -256, "-x-x-xxx"), (128, 0, "-x-----x"), (128, 300, "-x-----x")])
+def test_attention_prefill_f32_leaves_out_sequences_of_few_rows(hd, window, few):
+    """With the engine's skip_few the rows of every sequence that the host's rule names keep what the output held, all others have their values:
+    host and kernel agree on both sides of the line, behind a past of any length, under windows and chunks."""
     import ctypes
     from fastgguf_b200.ops import fast_attention
     from fastgguf_b200.ops.lib import lib, ptr, stream
-    H, KV, hd = 32, 8, 64
-    before, new = [0, 300, 2000, 0, 700, 64], [200, 1, 70, 40, 130, 63]
+    H, KV = 32, 8
+    before, new = [0, 300, 2000, 0, 700, 64, 2000, 100], [200, 1, 70, 40, 130, 20, 20, 14]
     case = make_case(before, new, H, KV, hd, torch.float32, 14)
-    few = [bool(lib("core").fg_attention_f32_few_rows(n, p, H, hd, 0)) for n, p in zip(new, before)]
-    assert few == [False, True, False, True, False, True]
+    left = [bool(lib("core").fg_attention_f32_left_out(n, p, H, hd, window)) for n, p in zip(new, before)]
+    assert "".join("x" if x else "-" for x in left) == few
     q, scale = case["q"], 1.0 / math.sqrt(hd)
     want = fast_attention.attention_prefill_f32(q, case["cu_rows"], case["seq_start"], case["table"], case["k_pool"], case["v_pool"], len(new), max(new),
-                                                H, KV, hd, scale, 0)
+                                                H, KV, hd, scale, window)
     out = torch.full_like(want, 9.0)
     f = ctypes.c_float
     assert lib("core").fg_attention_prefill_f32_ext(ptr(q), q.stride(0), ptr(out), out.stride(0), ptr(case["cu_rows"]), ptr(case["seq_start"]),
                                                     ptr(case["table"]), case["table"].shape[1], ptr(case["k_pool"]), ptr(case["v_pool"]), len(new),
-                                                    max(new), H, KV, hd, 64, f(scale), 0, 1, stream()) == 0
+                                                    max(new), H, KV, hd, 64, f(scale), window, lib("core").fg_attention_f32_skip_few(hd), stream()) == 0
     at = 0
-    for n, left_out in zip(new, few):
+    for n, left_out in zip(new, left):
         rows = out[at:at + n]
         assert (rows == 9.0).all() if left_out else torch.equal(rows, want[at:at + n])
         at += n
