@@ -732,7 +732,7 @@ extern "C" int fg_attention_f32_cost(int tokens, int past, int H, int KV, int hd
     const int G = H / KV, Gc = G < 16 ? G : 16, TQ = ROWS / Gc;
     const double ctas = (double)((tokens + TQ - 1) / TQ) * KV * ((G + Gc - 1) / Gc);
     *walk = (keys + tokens) / PAGE + 1.0;
-    *any_size = (double)tokens * H * seen / PAGE / f32_pairs(hd);
+    *any_size = (double)tokens * H * (seen / PAGE + 1.0) / f32_pairs(hd);           // (a pair's block takes a page's time beside its pages')
     *tiles = ctas * (seen / PAGE + 1.0) / ((hd == 64 ? 1.23 : 0.86) * n_sm);        // (2,048 tokens: an SM walks a page in 2.8 us, 5.8 at 128)
     return 0;
 }

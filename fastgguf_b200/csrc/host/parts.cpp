@@ -331,7 +331,10 @@ static F32AttentionSplit split_f32_attention(const Batch &b, int H, int KV, int 
         }
     }
     const double many = std::max(many_walk, many_tiles), all = std::max(std::max(many_walk, few_walk), many_tiles + few_tiles);
-    if (all - many <= few_any + 3.5 * (double)s.any_size.size()) s.any_size.clear();     // (3.5: a launch of the any-size kernel, at least 12 us)
+    // (1.2: what a launch of either kernel takes beside its walks, 4 us; the tiles' is there anyway where other sequences need them.  One sequence of
+    // 17 tokens, 32 heads of 64: 6.1 us, as a tile 8.9; 33 tokens 10.8 : 9.9; four of 17 tokens 18.1 : 8.9; four heads, 128 tokens 10.1 : 13.0)
+    const double launch = 1.2;
+    if (all - many + (many > 0.0 ? 0.0 : launch) <= few_any + launch * (double)s.any_size.size()) s.any_size.clear();
     s.tiles = many_walk > 0.0 || (s.any_size.empty() && few_walk > 0.0);
     return s;
 }

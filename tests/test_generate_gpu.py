@@ -313,3 +313,19 @@ def test_a_session_step_that_is_refused_queues_nothing(models):
         return engine.step_host([StepEntry(s, [7, 8], [0, 1]) for s in slots])
 
     assert np.array_equal(run(True), run(False))
+
+
+@pytest.mark.parametrize("heads,kv_heads,lengths,tiles", [(8, 8, [17], False), (8, 8, [33], False), (8, 8, [33] * 4, True), (8, 8, [200], True),
+                                                          (4, 1, [64], False), (4, 1, [17] * 4, False), (32, 8, [17], False), (32, 8, [17] * 4, True)])
+def test_float32_prompts_take_the_kernel_that_is_done_first(heads, kv_heads, lengths, tiles):
+    """A few new tokens are the any-size kernel's, unless there are so many such sequences that their tiles, side by side, are done first."""
+    from helpers import TINY_B
+    from fastgguf_b200.engine.api import Engine
+    from fastgguf_b200.registry import config_from_dict
+    cfg = dict(TINY_B, hidden_size=512, num_attention_heads=heads, num_key_value_heads=kv_heads, head_dim=64, intermediate_size=512, vocab_size=256)
+    engine = Engine.from_random(config_from_dict(cfg), 3, dtype="float32", max_tokens=2048, max_batch=4)
+    engine.profile(True)
+    engine.generate([random_tokens(n, 256, 90 + i) for i, n in enumerate(lengths)], temp=0, max_tokens=1, ignore_eos=True)
+    names = {r["name"].split(" ")[0] for r in engine.profile_report()}
+    engine.profile(False)
+    assert ("fg_attention_prefill_f32" in names) == tiles and any(n.startswith("fg_attention_generic") for n in names) == (not tiles), names
