@@ -115,9 +115,9 @@ template <> __device__ __forceinline__ void store4<bf16>(bf16 *dst, float a, flo
 // VEC: rows are read and written four elements at a time (E % 4 == 0, 16-byte aligned rows)
 template <typename TO, bool VEC>
 __global__ void rmsnorm_kernel(const float *__restrict__ x, const float *__restrict__ w,
-                               const int *__restrict__ rows, TO *__restrict__ out, int E, float eps) {
+                               const int *__restrict__ rows, TO *__restrict__ out, int E, float eps, int early) {
     __shared__ float scratch[32];
-    pdl_launch_dependents();
+    if (early) pdl_launch_dependents();
     pdl_wait();
     int r = blockIdx.x;
     const float *xi = x + (size_t)(rows ? rows[r] : r) * E;
@@ -149,9 +149,9 @@ __global__ void rmsnorm_kernel(const float *__restrict__ x, const float *__restr
 // additions are those above.  (What it gives in a step: see attention_decode_f32.cu.)
 template <typename TO, int N>
 __global__ void __launch_bounds__(256)
-rmsnorm_regs_kernel(const float *__restrict__ x, const float *__restrict__ w, const int *__restrict__ rows, TO *__restrict__ out, int E, float eps) {
+rmsnorm_regs_kernel(const float *__restrict__ x, const float *__restrict__ w, const int *__restrict__ rows, TO *__restrict__ out, int E, float eps, int early) {
     __shared__ float scratch[32];
-    pdl_launch_dependents();
+    if (early) pdl_launch_dependents();
     const int r = blockIdx.x, n = E / 4;
     float4 g[N], v[N];
 #pragma unroll
@@ -180,9 +180,9 @@ rmsnorm_regs_kernel(const float *__restrict__ x, const float *__restrict__ w, co
 }
 
 template <typename TO>
-static int launch_rmsnorm_regs(const float *x, const float *w, const int *rows, TO *out, int R, int E, float eps, int threads, cudaStream_t stream) {
+static int launch_rmsnorm_regs(const float *x, const float *w, const int *rows, TO *out, int R, int E, float eps, int early, int threads, cudaStream_t stream) {
     const int per = (E / 4 + threads - 1) / threads;
-#define RMS_RUN(N) return fg_launch(rmsnorm_regs_kernel<TO, N>, dim3(R), dim3(threads), 0, stream, x, w, rows, out, E, eps)
+#define RMS_RUN(N) return fg_launch(rmsnorm_regs_kernel<TO, N>, dim3(R), dim3(threads), 0, stream, x, w, rows, out, E, eps, early)
     if (per <= 1) RMS_RUN(1);
     if (per <= 2) RMS_RUN(2);
     if (per <= 4) RMS_RUN(4);
@@ -190,25 +190,29 @@ static int launch_rmsnorm_regs(const float *x, const float *w, const int *rows, 
 #undef RMS_RUN
 }
 
-extern "C" int fg_rmsnorm(const float *x, const float *w, const int *rows, void *out, int out_dtype,
-                          int R, int E, float eps, cudaStream_t stream) {
+// early: the successor is released at the start (see common.cuh: not between two tensor-memory contractions, which a step's rows tell and not R)
+extern "C" int fg_rmsnorm_step(const float *x, const float *w, const int *rows, void *out, int out_dtype, int R, int E, float eps, int early,
+                               cudaStream_t stream) {
     if (R <= 0) return 0;
     bool vec = E % 4 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)w & 15) == 0 && ((uintptr_t)out & 15) == 0;
     int per = vec ? E / 4 : E;
     int threads = per >= 1024 ? 256 : (per >= 256 ? 128 : 64);
     if (vec && per <= 8 * threads) {
-        if (out_dtype == FG_F32) return launch_rmsnorm_regs<float>(x, w, rows, (float *)out, R, E, eps, threads, stream);
-        if (out_dtype == FG_BF16) return launch_rmsnorm_regs<bf16>(x, w, rows, (bf16 *)out, R, E, eps, threads, stream);
+        if (out_dtype == FG_F32) return launch_rmsnorm_regs<float>(x, w, rows, (float *)out, R, E, eps, early, threads, stream);
+        if (out_dtype == FG_BF16) return launch_rmsnorm_regs<bf16>(x, w, rows, (bf16 *)out, R, E, eps, early, threads, stream);
         return FG_ERR_BAD_DTYPE;
     }
     if (out_dtype == FG_F32) {
-        if (vec) return fg_launch(rmsnorm_kernel<float, true>, dim3(R), dim3(threads), 0, stream, x, w, rows, (float *)out, E, eps);
-        return fg_launch(rmsnorm_kernel<float, false>, dim3(R), dim3(threads), 0, stream, x, w, rows, (float *)out, E, eps);
+        if (vec) return fg_launch(rmsnorm_kernel<float, true>, dim3(R), dim3(threads), 0, stream, x, w, rows, (float *)out, E, eps, early);
+        return fg_launch(rmsnorm_kernel<float, false>, dim3(R), dim3(threads), 0, stream, x, w, rows, (float *)out, E, eps, early);
     } else if (out_dtype == FG_BF16) {
-        if (vec) return fg_launch(rmsnorm_kernel<bf16, true>, dim3(R), dim3(threads), 0, stream, x, w, rows, (bf16 *)out, E, eps);
-        return fg_launch(rmsnorm_kernel<bf16, false>, dim3(R), dim3(threads), 0, stream, x, w, rows, (bf16 *)out, E, eps);
+        if (vec) return fg_launch(rmsnorm_kernel<bf16, true>, dim3(R), dim3(threads), 0, stream, x, w, rows, (bf16 *)out, E, eps, early);
+        return fg_launch(rmsnorm_kernel<bf16, false>, dim3(R), dim3(threads), 0, stream, x, w, rows, (bf16 *)out, E, eps, early);
     }
     return FG_ERR_BAD_DTYPE;
+}
+extern "C" int fg_rmsnorm(const float *x, const float *w, const int *rows, void *out, int out_dtype, int R, int E, float eps, cudaStream_t stream) {
+    return fg_rmsnorm_step(x, w, rows, out, out_dtype, R, E, eps, 1, stream);
 }
 
 // ------------------------------------------------------------------ RoPE + cache append

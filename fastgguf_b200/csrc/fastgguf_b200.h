@@ -34,6 +34,8 @@ int fg_embed_gather_norm(const void *table, int table_dtype, const int *tokens, 
                          void *xw, float *ss, int M, int E, cudaStream_t stream);
 int fg_rmsnorm(const float *x, const float *w, const int *rows, void *out, int out_dtype, int R, int E, float eps,
                cudaStream_t stream);
+/* the same; early: releases its successor at its start (fg_rmsnorm: yes) */
+int fg_rmsnorm_step(const float *x, const float *w, const int *rows, void *out, int out_dtype, int R, int E, float eps, int early, cudaStream_t stream);
 int fg_rope_append(void *qkv, int dtype, int ld, const int *positions, const int *row_seq, const int *block_table,
                    int table_width, void *k_pool, void *v_pool, const float *cos_t, const float *sin_t, int M, int H,
                    int KV, int hd, int page_size, int write_kv, cudaStream_t stream);

@@ -112,7 +112,7 @@ const Weight &tensor_of(const std::map<std::string, Weight> &tensors, const char
 // ------------------------------------------------------------------------------------ deferred norm
 Tensor DeferredNorm::materialize(Runtime &rt) const {
     Tensor out = rt.arena->matrix(x.rows, x.cols, FG_BF16);
-    FG_LAUNCH("core", fg_rmsnorm, x.ptr<float>(), weight, nullptr, out.data, FG_BF16, (int)x.rows, (int)x.cols, eps, rt.stream);
+    FG_LAUNCH_STEP("core", fg_rmsnorm, x.ptr<float>(), weight, nullptr, out.data, FG_BF16, (int)x.rows, (int)x.cols, eps, rt.early_between(x.rows), rt.stream);
     return out;
 }
 
@@ -478,7 +478,7 @@ public:
         int R = rows ? n_rows : (int)x.rows;
         Tensor out = rt.arena->matrix(R, x.cols, rt.dtype);
         if (R > 0)
-            FG_LAUNCH("core", fg_rmsnorm, x.ptr<float>(), w_.t.ptr<float>(), rows, out.data, rt.dtype, R, (int)x.cols, eps_, rt.stream);
+            FG_LAUNCH_STEP("core", fg_rmsnorm, x.ptr<float>(), w_.t.ptr<float>(), rows, out.data, rt.dtype, R, (int)x.cols, eps_, rt.early_between(x.rows), rt.stream);
         return out;
     }
     bool deferrable() const override { return true; }

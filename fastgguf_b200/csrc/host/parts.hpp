@@ -33,6 +33,8 @@ struct Runtime {
     bool single_token = false;
     // what the launchers ..._step take: whether kernels beside attention may release their successor at their start (common.cuh)
     int early(int64_t rows) const { return rows <= 64 && (single_token || dtype == FG_F32); }
+    // the same for a kernel that stands between two contractions, by the rows of the step
+    int early_between(int64_t rows) const { return rows <= 64 || dtype == FG_F32; }
     // Set by a block around ONE call of a mixer or feed-forward whose can_overwrite() is true: the `residual` handed over
     // holds nothing yet, and the part writes its output there instead of adding it (no zeroing pass in front).
     bool overwrite = false;

@@ -37,6 +37,21 @@ def test_recurrences_release_the_output_projection_early_in_small_steps_alone():
             assert re.findall(r"pdl_launch_dependents\w*\([^;]*;", body) == ["pdl_launch_dependents_small_step(cu_rows[gridDim.x]);"] * (k in by_rows), k
 
 
+def test_the_norm_between_contractions_goes_by_the_rows_of_the_step():
+    """A final norm has as many blocks as rows are wanted, behind a contraction of all the step's rows: the host says whether it may release the
+    head's contraction at its start."""
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "fastgguf_b200", "csrc")
+    with open(os.path.join(csrc, "elementwise.cu")) as f:
+        text = f.read()
+    for k in ("void rmsnorm_kernel(", "rmsnorm_regs_kernel("):
+        body = text[text.index(k):]
+        assert re.findall(r".*pdl_launch_dependents.*", body[:body.index("pdl_wait();")]) == ["    if (early) pdl_launch_dependents();"], k
+    with open(os.path.join(csrc, "host", "parts.cpp")) as f:
+        text = f.read()
+    calls = [line for line in text.splitlines() if "fg_rmsnorm," in line and "FG_LAUNCH" in line]
+    assert calls and all("FG_LAUNCH_STEP" in line and "rt.early_between(x.rows)" in line for line in calls)
+
+
 def _saluzen():
     from saluzen_cases import attn, config, delta, dense, latent, parallel, parallel_2, ssm
     left = dict(heads=16, kv_heads=4, dim=64, vdim=64, scale=0.125)
