@@ -79,7 +79,7 @@ attn_decode_kernel(const bf16 *__restrict__ q, int ldq, const int *__restrict__ 
     if (!FUSE) pdl_wait();
     // Read before the wait (fused form): positions, the page table and this entry's own pages.  Allowed only
     // because nothing launched since the stream's last full barrier writes them (see common.cuh): positions
-    // and tables change by the step's opening copy or by decode_advance, the last kernel of a step, and this
+    // and tables change by the step's opening copy or by decode_advance_host_kernel, the last of a recorded step, and this
     // pool is appended to by this kernel alone.  A caller that reorders that must launch without the overlap.
     const int pos = positions[b];
     const int lo_key = first_visible_key(pos, window);        // (window < 0: a chunked mask, see common.cuh)

@@ -106,10 +106,17 @@ __device__ __forceinline__ bool elect_one() {
 // completion is transitive); BEFORE it, not only the predecessor but kernels further back may still
 // run, because a kernel releases its successor at its start.  So a kernel may read before its wait
 // only memory that nothing launched since the last full barrier of the stream writes - a full barrier
-// being a memory copy, or the boundary of a graph launch.  Weights qualify always.  Positions, page
-// tables and an entry's own cache pool qualify for the fused decode attention because the engine writes
-// positions and tables only by the copy that opens a step or by `decode_advance_host_kernel`, the LAST
-// node of the decode graph, and because an entry's pool is appended to by that entry's kernel alone.
+// being a memory copy or memset, or the boundary of a graph launch.  Weights qualify always.  Beside them:
+//   positions, page tables     written by the copy that opens a step and by `decode_advance_host_kernel`, the LAST node of
+//                              the decode graph (read early by the fused decode attention kernels)
+//   slots, row_seq, cu_rows    written by the copy that opens a step, or when a session or a recorded step is set up; a finished
+//                              sequence's slot by a device-to-device copy between two graph launches (conv1d_step, decay_step,
+//                              retention_regs; cu_rows also for the release by rows)
+//   an entry's cache pool      appended to by that entry's own attention kernel alone
+//   an entry's state rows      written by that entry's own recurrent kernels alone, each part of a row by one kernel, once a step;
+//                              zeroed by a memset when a slot is taken (conv1d_step, decay_step, retention_regs in steps of one token a
+//                              sequence).  A pass of a loop has states of its own.
+// A kernel that writes any of these elsewhere takes the early reads with it.
 // FASTGGUF_PDL=0 turns the attribute off; the two instructions are then no-ops.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -123,7 +130,7 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // Kernels that stand next to ATTENTION cannot go by the rows: a prompt of 16 tokens already runs the tensor-memory attention kernel
 // (64 rows of token x query head).  They, and others that such a step may run between two tensor-memory kernels, take `early`
 // from the host, which sets it at up to 64 rows of one token a sequence (attention without tensor memory) and in float32 engines
-// (whose tensor-memory contraction neither starts early nor releases its successor early).
+// (whose tensor-memory kernels, the contraction and prompt attention, are launched in plain stream order and release nobody early).
 __device__ __forceinline__ void pdl_launch_dependents_small_step(unsigned rows) {
     if (rows <= 64) pdl_launch_dependents();
 }

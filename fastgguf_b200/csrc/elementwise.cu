@@ -146,7 +146,8 @@ __global__ void rmsnorm_kernel(const float *__restrict__ x, const float *__restr
 }
 
 // The same with a row's numbers in registers, N vectors of four a thread, and the weights fetched before the wait: the row is read once.  The
-// additions are those above.  (What it gives in a step: see attention_decode_f32.cu.)
+// additions are those above.  Two passes : here (us, launches behind one another): 8 rows of 2,048 2.4 : 1.5, 512 of 2,048 3.9 : 2.5, 4,096 of 2,048 10.7 : 8.9,
+// 8 of 8,192 3.7 : 2.2, 16,384 of 8,192 163 : 168 (float32 out).
 template <typename TO, int N>
 __global__ void __launch_bounds__(256)
 rmsnorm_regs_kernel(const float *__restrict__ x, const float *__restrict__ w, const int *__restrict__ rows, TO *__restrict__ out, int E, float eps, int early) {

@@ -129,10 +129,7 @@ int fg_argmax(const float *logits, int B, int V, int ldl, int *out, cudaStream_t
 /* ---- libfg_mix: retention (linear attention with a fixed decay per head) and the mixture of experts */
 /* proj rows: q [H, dk] | k [H, dk] | v [H, dv] | g [H, dv] float32; state [slots, H, dk, dv] float32; out [M, H * dv].  cos_t null: no
    rotation; opts: 1 = silu on q, k and v, 2 = the sums o themselves, without unit norm and gate */
-int fg_retention(const float *proj, int ld, void *out, int out_dtype, int ldo, const int *positions, const int *cu_rows,
-                 const int *slots, const float *cos_t, const float *sin_t, const float *decay, float *state, int n_seq,
-                 int H, int dk, int dv, float k_scale, float eps, int opts, cudaStream_t stream);
-/* the same; early: the state is fetched before the wait on the kernel in front, which must not have written it */
+/* early: the state is fetched before the wait on the kernel in front, which must not have written it */
 int fg_retention_step(const float *proj, int ld, void *out, int out_dtype, int ldo, const int *positions, const int *cu_rows,
                       const int *slots, const float *cos_t, const float *sin_t, const float *decay, float *state, int n_seq,
                       int H, int dk, int dv, float k_scale, float eps, int opts, int early, cudaStream_t stream);

@@ -128,7 +128,7 @@ public:
                       b.slots, cos_t, sin_t, decay_dev_.t.ptr<float>(), (float *)io.state, plan, U, b.n_seq, n_chunks, H_, dk_, dv_,
                       k_scale_, eps_, opts, rt.stream);
         } else {
-            FG_LAUNCH("mix", fg_retention_step, proj.ptr<float>(), (int)proj.ld, o.data, o.dtype, (int)o.ld, b.positions, b.cu_rows, b.slots, cos_t,
+            FG_LAUNCH_STEP("mix", fg_retention, proj.ptr<float>(), (int)proj.ld, o.data, o.dtype, (int)o.ld, b.positions, b.cu_rows, b.slots, cos_t,
                       sin_t, decay_dev_.t.ptr<float>(), (float *)io.state, b.n_seq, H_, dk_, dv_, k_scale_, eps_, opts, b.single_token ? 1 : 0, rt.stream);
         }
         if (whole_norm_)

@@ -243,7 +243,7 @@ DecodeGraph::~DecodeGraph() {
 }
 
 // The recorded step: layers, sampler, and LAST the feedback of the sampled tokens into the next step's inputs.
-// decode_advance must stay the last launch: it is the only kernel of the step that writes positions and tokens,
+// fg_decode_advance_host must stay the last launch: it is the only kernel of the step that writes positions and tokens,
 // and the fused decode attention reads them before waiting for its predecessor (see common.cuh).
 void DecodeGraph::run(cudaStream_t s, bool recording) {
     Runtime rt = engine_.model->runtime;

@@ -97,7 +97,7 @@ conv1d_state_kernel(const float *__restrict__ in, int ld, int taps, float *__res
 
 // One token a sequence: the output and the state's shift by one, in one kernel - a thread owns a channel of a row, and nobody else reads or
 // writes that channel's inputs.  Weights, and with AHEAD the state, are fetched before the wait (see decay_step_kernel below).  8 rows of 4,352
-// channels inside a step: 7.1 + 2.2 us as two kernels (what it takes here: see decay_step_kernel).
+// channels, four taps, launches behind one another: 7.3 us as two kernels, 1.4 here; 256 rows 16.8 : 9.7.
 template <bool AHEAD>
 __global__ void __launch_bounds__(256)
 conv1d_step_kernel(const float *__restrict__ in, int ld, const float *__restrict__ w, const float *__restrict__ bias, int taps, float *state,
@@ -311,9 +311,9 @@ decay_recurrence_kernel(const float *__restrict__ q, int ldq, const float *__res
 // The same for one token a sequence (a decode step): nothing to stage, so a lane reads its rows of k and q from the caches, the gates are computed
 // where they are used, and the state is in flight before the wait on the kernel in front (AHEAD: state rows are written by this entry's kernels
 // alone, once a step, and slots by the copy that opens a step, see common.cuh).  Lanes, rows and order of additions are those of the kernel above.
-// Bound by memory: 2 x 1 MB of state a sequence, 2.6 us for 8.  Inside a step of 8 sequences 12.3 us at 32 heads of 128 x 64 and 12.8 for the
-// delta rule at 16 heads of 128 x 128, 2 more for the gates' kernel, before.  This kernel, conv1d_step_kernel and the norms of q and k in one launch take
-// a step with two layers of each from 712 to 644 us.
+// Bound by memory: 2 x 1 MB of state a sequence, 2.6 us for 8 and 21 for 64.  Gates and recurrence as two kernels : this one, launches behind one another
+// (us): 32 heads of 128 x 64, 8 sequences 12.1 : 4.9, 64 sequences 83 : 34, 1 sequence 4.6 : 2.3; the delta rule at 16 heads of 128 x 128, 8 sequences
+// 12.9 : 5.2, 256 sequences 351 : 140.  With conv1d_step_kernel and the norms of q and k in one launch a step with two layers of each went from 712 to 644 us.
 #define STEP_THREADS 128
 template <bool DELTA, int NJ, bool AHEAD>
 __global__ void __launch_bounds__(STEP_THREADS)

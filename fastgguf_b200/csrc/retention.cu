@@ -155,8 +155,9 @@ retention_seq_kernel(const float *__restrict__ proj, int ld, TO *__restrict__ ou
 // The same for head sizes 64 and 128 (keys and values each) with the state in registers: thread (g, j) holds column j of rows g, g + G, ...
 // With AHEAD the state is fetched before the wait on the kernel in front: state rows are written by this entry's kernels alone, once a step, and
 // slots by the copy that opens a step (see common.cuh).  The additions are those of retention_seq_kernel, in its order.  Bound by memory: 2 x
-// 1 MB of state a sequence at 16 heads of 128 x 128, 2.6 us for 8; inside a step of 8 sequences 15.0 us with the state in shared memory; a step
-// with four such layers 381 us before, 349 with this kernel.
+// 1 MB of state a sequence at 16 heads of 128 x 128, 2.6 us for 8.  State in shared memory : here, launches behind one another (us): 8 sequences 12.3 : 4.0,
+// 64 sequences 47.9 : 29.2, 1 sequence 8.9 : 3.3, 8 sequences of 8 tokens 49.9 : 17.5; heads of 64 x 64, 8 sequences 5.3 : 2.5.  A step with four such
+// layers of 128 x 128 went from 381 to 349 us.
 template <typename TO, int DK, int DV, bool AHEAD>
 __global__ void __launch_bounds__(RET_THREADS)
 retention_regs_kernel(const float *__restrict__ proj, int ld, TO *__restrict__ out, int ldo, const int *__restrict__ positions,
@@ -575,13 +576,6 @@ extern "C" int fg_retention_step(const float *proj, int ld, void *out, int out_d
     if (out_dtype == FG_F32) RET_SEQ(float, false);
     RET_SEQ(bf16, false);
 #undef RET_SEQ
-}
-
-extern "C" int fg_retention(const float *proj, int ld, void *out, int out_dtype, int ldo, const int *positions, const int *cu_rows,
-                            const int *slots, const float *cos_t, const float *sin_t, const float *decay, float *state, int n_seq,
-                            int H, int dk, int dv, float k_scale, float eps, int opts, cudaStream_t stream) {
-    return fg_retention_step(proj, ld, out, out_dtype, ldo, positions, cu_rows, slots, cos_t, sin_t, decay, state, n_seq, H, dk, dv, k_scale, eps, opts, 0,
-                             stream);
 }
 
 // The chunk table (decay_attention.cu asks for it too).  plan: ints
