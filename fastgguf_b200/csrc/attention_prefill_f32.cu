@@ -36,9 +36,9 @@
 //
 // A CTA walks its pages alone, 3.45 us a page at head size 64 and 5.0 at 128, whatever it has of rows; the any-size kernel spreads the
 // (row, head) pairs over the GPU, 83 ns and 165 ns for 1,000 keys of a pair.  So a sequence with few new tokens is the any-size
-// kernel's, however long its past is (us, this kernel : any-size, 32 heads of 64): 1 token behind 4,000 keys 221 : 82, 16 tokens 223 :
-// 204, 64 tokens 227 : 692; no past, 24 tokens 22 : 26, 64 tokens 23 : 25, 300 tokens 27 : 172.  24 heads of 128: 32 tokens behind 4,000
-// keys 315 : 578.
+// kernel's, however long its past is (us, launches behind one another, this kernel : any-size, 32 heads of 64): 2 tokens behind 2,000 keys 117 : 40,
+// 8 behind 500 33 : 24, 64 behind 4,000 230 : 702; no past, 17 tokens 9.3 : 6.3, 33 tokens 10.1 : 11.2, 64 tokens 10.1 : 20.6, 512 tokens 35 : 418.  24
+// heads of 128: 17 tokens 11.8 : 9.4, 33 tokens 13.4 : 14.7, 64 behind 4,000 keys 320 : 1,073.
 #include "common.cuh"
 #include <atomic>
 
